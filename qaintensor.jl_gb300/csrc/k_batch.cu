@@ -7,9 +7,11 @@
 //
 // One launch per circuit layer: a persistent kernel whose CTAs take
 // (circuit, site) tasks from an atomic counter and run a whole update each:
-//   theta' = G (A B)            FP32, gate folded per (a, b), kept in a per-CTA slab
-//   one-sided Jacobi on theta'  FP32 columns, warps on disjoint column pairs of a
-//                               round-robin round, rotation angles in FP64
+//   theta' = G (A B)            FP32, tiled product, gate folded per (a, b), kept in a
+//                               per-CTA slab
+//   one-sided Jacobi on theta'  FP32 columns in shared memory (in the slab, i.e. in L2,
+//                               where theta' does not fit), rotation angles as
+//                               FP64 gives them (qt_cta.cuh)
 //   sigma_j = ||x_j||           FP64, bitonic sort, tail rule (FP64, sequential) at
 //                               the caller's cutoff, cap; a decision below the FP32
 //                               resolution without a certificate (cap or exact rank
@@ -28,6 +30,7 @@
 #include <cstring>
 #include <vector>
 
+#include "qt_cta.cuh"
 #include "qt_internal.cuh"
 #include "qt_rank_model.h"
 
@@ -52,6 +55,7 @@ struct BatchArgs {
   int* counter;
   float2* slab;              // per CTA: 4 * slab_elems float2 (FP32 X, T; or the FP64 X, T of a fallback)
   int slab_elems;
+  int smem_elems;            // float2 entries of the CTA's dynamic shared memory
   double cutoff;
   double floor_rel;          // FP32 resolution relative to ||theta'||_F (<= 0: 4 sqrt(max(m, n)) u)
   float tol;                 // FP32 Jacobi tolerance (relative off-diagonal)
@@ -62,43 +66,31 @@ struct BatchArgs {
   int* task_cert;            // QT_CERT_* of the rank decision (QT_CERT_NONE: the FP64 split decided)
 };
 
-__device__ inline void tourney(int r, int q, int n, int& a, int& b) {
-  if (q == 0) { a = r % (n - 1); b = n - 1; }
-  else { a = (r + q) % (n - 1); b = (r - q + (n - 1)) % (n - 1); }
-}
-
-template <typename R>
-__device__ inline R warp_sum(R v) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-// theta' = G (A B) into X and T (m x n, ld m), one thread per (a, b) owning
-// the four physical values; C = float2 (FP32 products) or double2 (FP64).
-template <int NT, typename C>
-__device__ void form_theta(const float2* A, const float2* B, int chil, int chim, int chir, const C* g, C* X, C* T) {
-  const int m = 2 * chil;
+// theta' = G (A B) into T (m x n, ld m) and X (ld ldx): the product into T, then the
+// gate on the four physical values of each (a, b).  C = float2 (FP32 products)
+// or double2 (FP64, from double2 copies of the sites).
+template <int NT, int TMAX, typename C>
+__device__ void form_theta(const C* A, const C* B, int chil, int chim, int chir, const C* g, C* X, int ldx, C* T,
+                           void* sm) {
+  const int m = 2 * chil, n = 2 * chir;
+  cta_gemm<NT, TMAX, C>(false, false, m, n, chim, A, m, nullptr, B, chim, sm,
+                        [&](int r, int col, C v) { T[r + (size_t)m * col] = v; });
   for (int idx = threadIdx.x; idx < chil * chir; idx += NT) {
     const int a = idx % chil, b = idx / chil;
-    C acc[4] = {czero<C>(), czero<C>(), czero<C>(), czero<C>()};
-    for (int k = 0; k < chim; k++) {
-      const C a0 = ccast<C>(A[a + chil * (2 * k)]), a1 = ccast<C>(A[a + chil * (2 * k + 1)]);
-      const C b0 = ccast<C>(B[k + chim * (2 * b)]), b1 = ccast<C>(B[k + chim * (2 * b + 1)]);
-      cfma(acc[0], a0, b0);
-      cfma(acc[1], a1, b0);
-      cfma(acc[2], a0, b1);
-      cfma(acc[3], a1, b1);
-    }
+    C th[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) th[q] = T[a + chil * (q & 1) + (size_t)m * ((q >> 1) + 2 * b)];
 #pragma unroll
     for (int o = 0; o < 4; o++) {
       C v = czero<C>();
 #pragma unroll
-      for (int q = 0; q < 4; q++) cfma(v, g[o + 4 * q], acc[q]);
-      const int r = a + chil * (o & 1), col = (o >> 1) + 2 * b;
-      X[r + m * col] = v;
-      T[r + m * col] = v;
+      for (int q = 0; q < 4; q++) cfma(v, g[o + 4 * q], th[q]);
+      const int row = a + chil * (o & 1), col = (o >> 1) + 2 * b;
+      T[row + (size_t)m * col] = v;
+      X[row + (size_t)ldx * col] = v;
     }
   }
+  __syncthreads();
 }
 
 // ||X||_F^2 in FP64 over the CTA.
@@ -107,7 +99,7 @@ __device__ double fro2_of(const C* X, int cnt, double* s_red) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double part = 0;
   for (int i = threadIdx.x; i < cnt; i += NT) part += (double)X[i].x * X[i].x + (double)X[i].y * X[i].y;
-  part = warp_sum(part);
+  part = cta_warp_sum(part);
   __syncthreads();
   if (lane == 0) s_red[warp] = part;
   __syncthreads();
@@ -116,73 +108,18 @@ __device__ double fro2_of(const C* X, int cnt, double* s_red) {
   return fro2;
 }
 
-// One-sided Jacobi on the n columns of X (m rows): warps on disjoint column
-// pairs of a round-robin round, rotation angles in FP64.  Columns with
-// |x|^2 <= nu2 are frozen.  Returns the sweeps run.
-template <int NT, typename C>
-__device__ int jacobi_columns(C* X, int m, int n, double tol, double nu2, int max_sweeps, int* s_rot) {
-  typedef typename real_of<C>::type R;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int sweeps = 0;
-  if (n < 2) return 0;
-  for (int sweep = 0; sweep < max_sweeps; sweep++) {
-    __syncthreads();  // every thread has read s_rot of the previous sweep
-    if (threadIdx.x == 0) *s_rot = 0;
-    __syncthreads();
-    for (int r = 0; r < n - 1; r++) {
-      for (int q = warp; q < n / 2; q += NT / 32) {
-        int pc, qc;
-        tourney(r, q, n, pc, qc);
-        C* xp = X + (size_t)m * pc;
-        C* xq = X + (size_t)m * qc;
-        R aa = 0, bb = 0, gr = 0, gi = 0;
-        for (int i = lane; i < m; i += 32) {
-          const C u = xp[i], v = xq[i];
-          aa = fma(u.x, u.x, fma(u.y, u.y, aa));
-          bb = fma(v.x, v.x, fma(v.y, v.y, bb));
-          gr = fma(u.x, v.x, fma(u.y, v.y, gr));
-          gi = fma(u.x, v.y, fma(-u.y, v.x, gi));
-        }
-        aa = warp_sum(aa);
-        bb = warp_sum(bb);
-        gr = warp_sum(gr);
-        gi = warp_sum(gi);
-        const double ag = sqrt((double)gr * gr + (double)gi * gi);
-        if ((double)aa > nu2 && (double)bb > nu2 && ag > tol * sqrt((double)aa * bb)) {
-          const double zeta = ((double)bb - aa) / (2.0 * ag);
-          const double t = copysign(1.0, zeta) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-          const double cs = 1.0 / sqrt(1.0 + t * t);
-          const R c = (R)cs, s = (R)(cs * t);
-          const R er = (R)(gr / ag), ei = (R)(gi / ag);
-          for (int i = lane; i < m; i += 32) {
-            const C u = xp[i], v = xq[i];
-            // x_p' = c x_p - s e^{-i phi} x_q ;  x_q' = s e^{i phi} x_p + c x_q
-            xp[i] = mk(c * u.x - s * (er * v.x + ei * v.y), c * u.y - s * (er * v.y - ei * v.x));
-            xq[i] = mk(s * (er * u.x - ei * u.y) + c * v.x, s * (er * u.y + ei * u.x) + c * v.y);
-          }
-          if (lane == 0) *s_rot = 1;
-        }
-      }
-      __syncthreads();
-    }
-    sweeps = sweep + 1;
-    const int again = *s_rot;  // read after the round's closing barrier
-    if (!again) break;
-  }
-  return sweeps;
-}
-
 // Column norms of X in FP64, sorted descending into s_sig / s_perm (bitonic).
 template <int NT, typename C>
-__device__ void sorted_norms(const C* X, int m, int n, double* s_sig, int* s_perm) {
+__device__ void sorted_norms(const C* X, int ld, int m, int n, double* s_sig, int* s_perm) {
   int np2 = 1;
   while (np2 < n) np2 <<= 1;
   for (int j = threadIdx.x; j < np2; j += NT) {
     double s = -1.0;
     if (j < n) {
       s = 0;
+#pragma unroll 8
       for (int i = 0; i < m; i++) {
-        const C v = X[i + (size_t)m * j];
+        const C v = X[i + (size_t)ld * j];
         s += (double)v.x * v.x + (double)v.y * v.y;
       }
       s = sqrt(s);
@@ -211,27 +148,40 @@ __device__ void sorted_norms(const C* X, int m, int n, double* s_sig, int* s_per
 }
 
 // The tail rule of src/svd.jl:29-33 (sequential from the smallest value,
-// strict >, k >= 1) on the n sorted values.
+// strict >, k >= 1) on the n sorted values.  The square root, a dependent
+// FP64 chain per value, is taken only where the sum lies within rounding of
+// cutoff^2; elsewhere the comparison of the squares gives the same answer.
 __device__ int tail_rule(const double* s, int n, double cutoff) {
+  const double c2 = cutoff * cutoff;
+  const bool squares = c2 > 1e-290;
+  const double lo = squares ? c2 * (1.0 - 1e-14) : 0.0, hi = squares ? c2 * (1.0 + 1e-14) : INFINITY;
   double acc = 0;
   for (int i = n - 1; i >= 0; i--) {
     acc += s[i] * s[i];
-    if (sqrt(acc) > cutoff) return i + 1;
+    if (acc < lo) continue;
+    if (acc > hi || sqrt(acc) > cutoff) return i + 1;
   }
   return 1;
 }
 
-template <int NT>
+// RMAX: rows of theta' per lane at most (m <= 32 RMAX), by the bucket's cap.
+//
+// What bounds it: the Jacobi's FMAs and, where theta' exceeds the shared
+// memory, its column traffic to L2; one CTA works alone on a task, so the
+// tasks in flight are what fills the chip.
+template <int NT, int RMAX>
 __global__ void __launch_bounds__(NT) batch_layer_kernel(BatchArgs p) {
-  __shared__ int s_task, s_rot, s_k, s_fb;
+  extern __shared__ __align__(16) unsigned char dyn[];
+  __shared__ int s_task, s_k, s_fb;
   __shared__ float2 g[16];
   __shared__ double2 g64[16];
   __shared__ double s_sig[MAXN];
   __shared__ int s_perm[MAXN];
   __shared__ double s_red[NT / 32];
+  constexpr int TMAX = RMAX >= 2 ? 64 : 32;
   const int tid = threadIdx.x;
-  float2* X = p.slab + (size_t)blockIdx.x * 4 * p.slab_elems;
-  float2* T = X + p.slab_elems;
+  float2* slab = p.slab + (size_t)blockIdx.x * 4 * p.slab_elems;
+  float2* T = slab + p.slab_elems;
 
   for (;;) {
     if (tid == 0) s_task = p.task_begin + atomicAdd(p.counter, 1);
@@ -253,15 +203,19 @@ __global__ void __launch_bounds__(NT) batch_layer_kernel(BatchArgs p) {
     }
     __syncthreads();
 
-    // 1. theta' = G (A B) in FP32
-    form_theta<NT, float2>(A, B, chil, chim, chir, g, X, T);
-    __syncthreads();
-    const double fro2 = fro2_of<NT>(X, m * n, s_red);
+    // 1. theta' = G (A B) in FP32.  In shared memory the columns are an odd
+    // number of entries apart, so that threads on different columns meet
+    // different banks.
+    const bool in_smem = (m + 1) * n <= p.smem_elems;
+    float2* X = in_smem ? reinterpret_cast<float2*>(dyn) : slab;
+    const int ldx = in_smem ? m + 1 : m;
+    form_theta<NT, TMAX, float2>(A, B, chil, chim, chir, g, X, ldx, T, dyn);
+    const double fro2 = fro2_of<NT>(T, m * n, s_red);
     const double nu = 4.0 * sqrt((double)max(m, 16)) * 5.96e-8;
 
     // 2. one-sided Jacobi on the columns of X, 3. sorted FP64 norms
-    int sweeps = jacobi_columns<NT, float2>(X, m, n, (double)p.tol, nu * nu * fro2, p.max_sweeps, &s_rot);
-    sorted_norms<NT, float2>(X, m, n, s_sig, s_perm);
+    int sweeps = cta_jacobi_any<NT, RMAX>(X, ldx, m, n, (double)p.tol, nu * nu * fro2, p.max_sweeps);
+    sorted_norms<NT, float2>(X, ldx, m, n, s_sig, s_perm);
 
     // 4. the tail rule at the caller's cutoff, then the cap.  Below the FP32
     // resolution eta the decision needs a certificate: the cap binding with
@@ -307,35 +261,39 @@ __global__ void __launch_bounds__(NT) batch_layer_kernel(BatchArgs p) {
     if (!s_fb) {
       const int k = s_k;
       // 5. A' (chil, 2, k) = unit columns, into site slot w
-      for (int idx = tid; idx < m * k; idx += NT) {
-        const int r = idx % m, j = idx / m;
+      for (int j = tid >> 5; j < k; j += NT / 32) {
         const double s = s_sig[j];
         const float inv = s > 0 ? (float)(1.0 / s) : 0.f;
-        const float2 v = X[r + (size_t)m * s_perm[j]];
-        A[r + (size_t)m * j] = make_float2(v.x * inv, v.y * inv);
+        const float2* x = X + (size_t)ldx * s_perm[j];
+        for (int r = tid & 31; r < m; r += 32) A[r + (size_t)m * j] = make_float2(x[r].x * inv, x[r].y * inv);
       }
       __syncthreads();
       // 6. B' (k, 2, chir) = A'^H theta', into site slot w+1
-      for (int idx = tid; idx < k * n; idx += NT) {
-        const int j = idx % k, col = idx / k;
-        float2 acc = make_float2(0, 0);
-        for (int r = 0; r < m; r++) cfma_conj(acc, A[r + (size_t)m * j], T[r + (size_t)m * col]);
-        B[j + (size_t)k * col] = acc;
-      }
+      cta_gemm<NT, TMAX, float2>(true, false, k, n, m, A, m, nullptr, T, m, dyn,
+                                 [&](int r, int col, float2 v) { B[r + (size_t)k * col] = v; });
     } else {
       // The exact FP64 split: theta' from the complex64 sites in FP64, FP64
       // Jacobi (tolerance and freeze at FP64 rounding), the rule at the
-      // caller's cutoff; the FP64 X and T take the whole slab.
-      double2* X64 = reinterpret_cast<double2*>(X);
+      // caller's cutoff.  The FP64 X and T take the whole slab (X the shared
+      // memory where it fits); X holds the widened sites before that.
+      double2* X64 = reinterpret_cast<double2*>(slab);
       double2* T64 = X64 + p.slab_elems;
+      double2 *A64 = X64, *B64 = X64 + (size_t)m * chim;  // 2 chim (chil + chir) <= slab_elems
+      for (int i = tid; i < m * chim; i += NT) A64[i] = ccast<double2>(A[i]);
+      for (int i = tid; i < chim * n; i += NT) B64[i] = ccast<double2>(B[i]);
       __syncthreads();
-      form_theta<NT, double2>(A, B, chil, chim, chir, g64, X64, T64);
-      __syncthreads();
-      const double f64 = fro2_of<NT>(X64, m * n, s_red);
+      form_theta<NT, 32, double2>(A64, B64, chil, chim, chir, g64, T64, m, T64, dyn);
+      double* ws = reinterpret_cast<double*>(dyn);  // 4 n doubles, then X where it fits
+      const bool in_smem64 = 4 * n + 2 * (m + 1) * n <= p.smem_elems;
+      if (in_smem64) X64 = reinterpret_cast<double2*>(ws + 4 * n);
+      const int ld64 = in_smem64 ? m + 1 : m;
+      for (int j = tid >> 5; j < n; j += NT / 32)
+        for (int r = tid & 31; r < m; r += 32) X64[r + (size_t)ld64 * j] = T64[r + (size_t)m * j];
+      const double f64 = fro2_of<NT>(T64, m * n, s_red);
       const double nu64 = 4.0 * sqrt((double)max(m, 16)) * 1.11e-16;
-      sweeps += jacobi_columns<NT, double2>(X64, m, n, 16.0 * sqrt((double)max(m, 16)) * 1.11e-16,
-                                            nu64 * nu64 * f64, p.max_sweeps, &s_rot);
-      sorted_norms<NT, double2>(X64, m, n, s_sig, s_perm);
+      sweeps += cta_jacobi64<NT>(X64, ld64, m, n, 16.0 * sqrt((double)max(m, 16)) * 1.11e-16, nu64 * nu64 * f64,
+                                 p.max_sweeps, ws);
+      sorted_norms<NT, double2>(X64, ld64, m, n, s_sig, s_perm);
       if (tid == 0) {
         const int k = min(tail_rule(s_sig, n, p.cutoff), kcap);
         double disc = 0;
@@ -347,88 +305,109 @@ __global__ void __launch_bounds__(NT) batch_layer_kernel(BatchArgs p) {
       }
       __syncthreads();
       const int k = s_k;
-      // B' = A'^H theta' from the FP64 columns (before A is overwritten: B
-      // reads only X64 and T64), then A' = unit columns
-      for (int idx = tid; idx < k * n; idx += NT) {
-        const int j = idx % k, col = idx / k;
+      // A' = unit columns, then B' = A'^H theta', both from the FP64 columns.
+      // The product's tiles take the start of the shared memory: columns kept
+      // there move to the slab first.
+      if (in_smem64) {
+        double2* Xs = reinterpret_cast<double2*>(slab);
+        for (int j = tid >> 5; j < n; j += NT / 32)
+          for (int r = tid & 31; r < m; r += 32) Xs[r + (size_t)m * j] = X64[r + (size_t)ld64 * j];
+        X64 = Xs;
+        __syncthreads();
+      }
+      for (int j = tid >> 5; j < k; j += NT / 32) {
         const double s = s_sig[j];
         const double inv = s > 0 ? 1.0 / s : 0.0;
-        const double2* xj = X64 + (size_t)m * s_perm[j];
-        double2 acc = make_double2(0, 0);
-        for (int r = 0; r < m; r++) cfma_conj(acc, xj[r], T64[r + (size_t)m * col]);
-        B[j + (size_t)k * col] = make_float2((float)(acc.x * inv), (float)(acc.y * inv));
+        const double2* x = X64 + (size_t)m * s_perm[j];
+        for (int r = tid & 31; r < m; r += 32) A[r + (size_t)m * j] = make_float2((float)(x[r].x * inv), (float)(x[r].y * inv));
       }
-      for (int idx = tid; idx < m * k; idx += NT) {
-        const int r = idx % m, j = idx / m;
-        const double s = s_sig[j];
+      __syncthreads();
+      cta_gemm<NT, 32, double2>(true, false, k, n, m, X64, m, s_perm, T64, m, dyn, [&](int r, int col, double2 v) {
+        const double s = s_sig[r];
         const double inv = s > 0 ? 1.0 / s : 0.0;
-        const double2 v = X64[r + (size_t)m * s_perm[j]];
-        A[r + (size_t)m * j] = make_float2((float)(v.x * inv), (float)(v.y * inv));
-      }
+        B[r + (size_t)k * col] = make_float2((float)(v.x * inv), (float)(v.y * inv));
+      });
     }
     if (tid == 0) bond[w + 1] = s_k;
     __syncthreads();
   }
 }
 
-// <Z_site> per circuit: a left-to-right transfer sweep in FP32 with the
-// environment in a per-CTA slab; one CTA per circuit (grid-stride).
+// <Z_site> per circuit in FP32, one CTA per circuit (grid-stride): the
+// environment L of the sites left of the measured one (L <- sum_s A_s^H L
+// A_s), R of those right of it (R <- sum_s A_s R A_s^H), and
+// d_s = tr(A_s^H L A_s R) at the measured site, so <Z> = (d_0 - d_1) /
+// (d_0 + d_1).  Each site is passed once, by two tiled products over both
+// physical values at a time.
+constexpr int EXPECT_TILE = 64;
 __global__ void __launch_bounds__(BT)
 batch_expect_kernel(const float2* sites, const int64_t* site_off, const int* cap, const int* nsites, const int* bonds,
                     const int* bond_off, int ncirc, int site, float2* slab, int slab_elems, double* out) {
-  float2* E = slab + (size_t)blockIdx.x * 3 * slab_elems;
-  float2* E2 = E + slab_elems;
-  float2* Tm = E2 + slab_elems;
-  __shared__ double s_red[BWARPS];
+  extern __shared__ __align__(16) unsigned char dyn[];
+  __shared__ double s_red[2][BWARPS];
+  const int tid = threadIdx.x;
   for (int c = blockIdx.x; c < ncirc; c += gridDim.x) {
     const int n = nsites[c];
     const int* bd = bonds + bond_off[c];
-    const size_t slot = (size_t)cap[c] * 2 * cap[c];
-    double res[2];
-    for (int pass = 0; pass < 2; pass++) {  // pass 0: <psi|psi>, pass 1: <psi|Z|psi>
-      const int c0 = bd[0];
-      for (int i = threadIdx.x; i < c0 * c0; i += BT) E[i] = make_float2((i % c0) == (i / c0) ? 1.f : 0.f, 0.f);
-      __syncthreads();
-      for (int st = 0; st < n; st++) {
-        const float2* Aq = sites + site_off[c] + (size_t)st * slot;
-        const int cl = bd[st], cr = bd[st + 1];
-        for (int i = threadIdx.x; i < cr * cr; i += BT) E2[i] = make_float2(0, 0);
-        __syncthreads();
-        for (int s = 0; s < 2; s++) {
-          const float wgt = (pass == 1 && st == site && s == 1) ? -1.f : 1.f;
-          // Tm (cl x cr) = E (cl x cl) A_s
-          for (int idx = threadIdx.x; idx < cl * cr; idx += BT) {
-            const int i = idx % cl, j = idx / cl;
-            float2 acc = make_float2(0, 0);
-            for (int q = 0; q < cl; q++) cfma(acc, E[i + cl * q], Aq[q + cl * (s + 2 * j)]);
-            Tm[idx] = acc;
-          }
-          __syncthreads();
-          // E2 (cr x cr) += w A_s^H Tm
-          for (int idx = threadIdx.x; idx < cr * cr; idx += BT) {
-            const int i = idx % cr, j = idx / cr;
-            float2 acc = make_float2(0, 0);
-            for (int q = 0; q < cl; q++) cfma_conj(acc, Aq[q + cl * (s + 2 * i)], Tm[q + cl * j]);
-            E2[idx].x += wgt * acc.x;
-            E2[idx].y += wgt * acc.y;
-          }
-          __syncthreads();
-        }
-        for (int i = threadIdx.x; i < cr * cr; i += BT) E[i] = E2[i];
-        __syncthreads();
-      }
-      const int cn = bd[n];
-      double tr = 0;
-      for (int i = threadIdx.x; i < cn; i += BT) tr += E[i + cn * i].x;
-      for (int o = 16; o > 0; o >>= 1) tr += __shfl_xor_sync(0xffffffffu, tr, o);
-      if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = tr;
-      __syncthreads();
-      double tot = 0;
-      for (int i = 0; i < BWARPS; i++) tot += s_red[i];
-      res[pass] = tot;
-      __syncthreads();
+    const size_t e2 = (size_t)cap[c] * cap[c], slot = 2 * e2;
+    float2* L = slab + (size_t)blockIdx.x * 4 * slab_elems;
+    float2 *R = L + e2, *T = R + e2, *U = T + slot;
+    const float2* base = sites + site_off[c];
+    auto eye = [&](float2* E, int d) {
+      for (int i = tid; i < d * d; i += BT) E[i] = make_float2((i % d) == (i / d) ? 1.f : 0.f, 0.f);
+    };
+    eye(L, bd[0]);
+    eye(R, bd[n]);
+    __syncthreads();
+    // a site (cl, 2, cr) is its (cl x 2 cr) matrix with ld cl and its (2 cl x
+    // cr) matrix with ld 2 cl in the same memory
+    auto times_left = [&](const float2* A, int cl, int cr) {  // T = L A
+      cta_gemm<BT, EXPECT_TILE, float2>(false, false, cl, 2 * cr, cl, L, cl, nullptr, A, cl, dyn,
+                                [&](int r, int col, float2 v) { T[r + (size_t)cl * col] = v; });
+    };
+    auto times_right = [&](const float2* A, int cl, int cr) {  // U = A R
+      cta_gemm<BT, EXPECT_TILE, float2>(false, false, 2 * cl, cr, cr, A, 2 * cl, nullptr, R, cr, dyn,
+                                [&](int r, int col, float2 v) { U[r + (size_t)2 * cl * col] = v; });
+    };
+    for (int st = 0; st < site; st++) {
+      const float2* A = base + (size_t)st * slot;
+      const int cl = bd[st], cr = bd[st + 1];
+      times_left(A, cl, cr);
+      cta_gemm<BT, EXPECT_TILE, float2>(true, false, cr, cr, 2 * cl, A, 2 * cl, nullptr, T, 2 * cl, dyn,
+                                [&](int r, int col, float2 v) { L[r + (size_t)cr * col] = v; });
     }
-    if (threadIdx.x == 0) out[c] = res[1] / res[0];
+    for (int st = n - 1; st > site; st--) {
+      const float2* A = base + (size_t)st * slot;
+      const int cl = bd[st], cr = bd[st + 1];
+      times_right(A, cl, cr);
+      cta_gemm<BT, EXPECT_TILE, float2>(false, true, cl, cl, 2 * cr, U, cl, nullptr, A, cl, dyn,
+                                [&](int r, int col, float2 v) { R[r + (size_t)cl * col] = v; });
+    }
+    const float2* A = base + (size_t)site * slot;
+    const int cl = bd[site], cr = bd[site + 1];
+    times_left(A, cl, cr);
+    times_right(A, cl, cr);
+    // R is Hermitian: tr(A_s^H L A_s R) = sum T_s conj(U_s)
+    double d[2] = {0, 0};
+    for (int j = tid >> 5; j < cr; j += BWARPS) {
+      float f[2] = {0.f, 0.f};
+      for (int i = tid & 31; i < 2 * cl; i += 32) {
+        const float2 t = T[i + (size_t)2 * cl * j], u = U[i + (size_t)2 * cl * j];
+        f[i >= cl] = fmaf(t.x, u.x, fmaf(t.y, u.y, f[i >= cl]));
+      }
+      d[0] += f[0];
+      d[1] += f[1];
+    }
+    for (int s = 0; s < 2; s++) {
+      d[s] = cta_warp_sum(d[s]);
+      if ((tid & 31) == 0) s_red[s][tid >> 5] = d[s];
+    }
+    __syncthreads();
+    if (tid == 0) {
+      double t0 = 0, t1 = 0;
+      for (int i = 0; i < BWARPS; i++) { t0 += s_red[0][i]; t1 += s_red[1][i]; }
+      out[c] = (t0 - t1) / (t0 + t1);
+    }
     __syncthreads();
   }
 }
@@ -455,7 +434,8 @@ struct qt_batch {
   int64_t* d_site_off = nullptr;
   int *d_cap = nullptr, *d_nsites = nullptr, *d_bonds = nullptr, *d_bond_off = nullptr;
   float2* d_slab = nullptr;
-  int ctas = 0, slab_elems = 0;
+  int ctas = 0;
+  int bucket_elems[4] = {0, 0, 0, 0};  // entries of the largest theta' per bond-cap bucket (0: no circuit in it)
   int* d_counter = nullptr;  // one counter per layer
   int counter_cap = 0;
   // the last program (device copies) and its captured graph
@@ -472,14 +452,49 @@ struct qt_batch {
   cudaGraphExec_t graph = nullptr;
   // launch shape per bond-cap bucket (caps <= 16, 32, 64, 128): threads per
   // CTA and CTAs per SM of the persistent layer kernel (qt_batch_set_launch)
-  int threads[4] = {256, 256, 256, 256};
-  int cps[4] = {1, 1, 1, 1};
-  int slab_ctas = 0;         // CTAs the slab holds
+  int threads[4] = {128, 256, 256, 256};
+  int cps[4] = {4, 2, 1, 1};
+  size_t slab_count = 0;     // float2 entries of the slab
+  // float2 entries that the launches of every bucket need (4 theta' per CTA),
+  // and the observable kernel's one CTA per SM
+  size_t slab_need() const {
+    size_t need = 0;
+    for (int bk = 0; bk < 4; bk++) need = std::max(need, (size_t)ctas * cps[bk] * 4 * bucket_elems[bk]);
+    return need;
+  }
 };
 
 namespace {
 
 int bucket_of(int cap) { return cap <= 16 ? 0 : cap <= 32 ? 1 : cap <= 64 ? 2 : 3; }
+
+// Dynamic shared memory of the layer kernel: the whole theta' of a bucket
+// (caps 16, 32 and 64: 8, 33 and 132 KB) and the product tiles; 200 KB for
+// caps up to 128, whose theta' (512 KB) fits up to bonds of 80 and is kept in
+// the slab above.
+size_t batch_smem(int bk) {
+  static const size_t theta[4] = {33 * 32, 65 * 64, 129 * 128, 25600};
+  return std::max(theta[bk] * sizeof(float2),
+                  std::max(cta_gemm_smem<double2>(32), cta_gemm_smem<float2>(bk == 0 ? 32 : 64)));
+}
+
+typedef void (*layer_fn)(BatchArgs);
+
+template <int NT>
+layer_fn layer_kernel_rows(int bk) {
+  static const layer_fn fn[4] = {batch_layer_kernel<NT, 1>, batch_layer_kernel<NT, 2>, batch_layer_kernel<NT, 4>,
+                                 batch_layer_kernel<NT, 8>};
+  return fn[bk];
+}
+
+layer_fn layer_kernel(int threads, int bk) {
+  switch (threads) {
+    case 128: return layer_kernel_rows<128>(bk);
+    case 512: return layer_kernel_rows<512>(bk);
+    case 1024: return layer_kernel_rows<1024>(bk);
+    default: return layer_kernel_rows<256>(bk);
+  }
+}
 
 }  // namespace
 
@@ -513,11 +528,13 @@ extern "C" int qt_batch_create(qt_handle* h, int ncirc, const int* nqubits, cons
     off += (int64_t)nqubits[c] * chi_max[c] * 2 * chi_max[c];
     boff += nqubits[c] + 1;
     b->capmax = std::max(b->capmax, chi_max[c]);
+    int& be = b->bucket_elems[bucket_of(chi_max[c])];
+    be = std::max(be, 4 * chi_max[c] * chi_max[c]);
   }
   int dev_sms = 152;
   cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, h->device);
   b->ctas = dev_sms;
-  b->slab_elems = (2 * b->capmax) * (2 * b->capmax);
+  b->slab_count = b->slab_need();
   std::vector<int> bonds(boff, 1);
   bool ok = cudaMalloc(&b->d_sites, sizeof(float2) * off) == cudaSuccess &&
             cudaMalloc(&b->d_site_off, sizeof(int64_t) * ncirc) == cudaSuccess &&
@@ -525,8 +542,7 @@ extern "C" int qt_batch_create(qt_handle* h, int ncirc, const int* nqubits, cons
             cudaMalloc(&b->d_nsites, sizeof(int) * ncirc) == cudaSuccess &&
             cudaMalloc(&b->d_bonds, sizeof(int) * boff) == cudaSuccess &&
             cudaMalloc(&b->d_bond_off, sizeof(int) * ncirc) == cudaSuccess &&
-            cudaMalloc(&b->d_slab, sizeof(float2) * 4 * (size_t)b->slab_elems * b->ctas) == cudaSuccess;
-  b->slab_ctas = b->ctas;
+            cudaMalloc(&b->d_slab, sizeof(float2) * b->slab_count) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();
     qt_batch_free(h, b);
@@ -598,19 +614,17 @@ extern "C" int qt_batch_run(qt_handle* h, qt_batch* b, int nlayers, const int* l
     std::memcpy(&og[(size_t)32 * i], gates + (size_t)32 * order[i], sizeof(double) * 32);
   }
   b->order = order;
-  // the slab holds one 4-unit block per CTA of the widest launch
   const int dev_sms = b->ctas;
-  int need = 0;
-  for (int bk = 0; bk < 4; bk++) need = std::max(need, dev_sms * b->cps[bk]);
-  if (need > b->slab_ctas) {
+  if (b->slab_need() > b->slab_count) {  // launch shapes set since
     cudaFree(b->d_slab);
     b->d_slab = nullptr;
-    if (cudaMalloc(&b->d_slab, sizeof(float2) * 4 * (size_t)b->slab_elems * need) != cudaSuccess) {
+    b->slab_count = 0;
+    const size_t need = b->slab_need();
+    if (cudaMalloc(&b->d_slab, sizeof(float2) * need) != cudaSuccess) {
       cudaGetLastError();
-      b->slab_ctas = 0;
       return qt_fail(h, QT_ENOMEM, "batch_run: slab allocation failed");
     }
-    b->slab_ctas = need;
+    b->slab_count = need;
   }
   if (ntask > 0) {
     bool ok = cudaMalloc(&b->d_tc, sizeof(int) * ntask) == cudaSuccess &&
@@ -646,7 +660,7 @@ extern "C" int qt_batch_run(qt_handle* h, qt_batch* b, int nlayers, const int* l
   a.sites = b->d_sites; a.site_off = b->d_site_off; a.cap = b->d_cap; a.nsites = b->d_nsites; a.bonds = b->d_bonds;
   a.task_grank = b->d_grank; a.task_cert = b->d_cert;
   a.bond_off = b->d_bond_off; a.task_circ = b->d_tc; a.task_site = b->d_ts; a.task_gate = b->d_tg;
-  a.slab = b->d_slab; a.slab_elems = b->slab_elems; a.cutoff = cutoff;
+  a.slab = b->d_slab; a.slab_elems = 0; a.smem_elems = 0; a.cutoff = cutoff;
   a.floor_rel = h->cfg.noise_floor;  // <= 0: the default resolution of each task's shape
   // FP32 Jacobi tolerance: a pair is rotated while its relative
   // off-diagonal exceeds 16 u (u = 2^-24).  The FP32 Gram of a converged pair
@@ -658,6 +672,10 @@ extern "C" int qt_batch_run(qt_handle* h, qt_batch* b, int nlayers, const int* l
   a.tol = (float)(h->cfg.jacobi_tol > 0 ? h->cfg.jacobi_tol : 16.0 * 5.96e-8);
   a.max_sweeps = std::max(4, h->cfg.max_sweeps);
   a.task_rank = b->d_rank; a.task_sweeps = b->d_sweeps; a.task_discarded = b->d_disc;
+  for (int bk = 0; bk < 4; bk++)  // before a capture begins
+    if (b->bucket_elems[bk])
+      QT_CHECK_CUDA(h, cudaFuncSetAttribute((const void*)layer_kernel(b->threads[bk], bk),
+                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)batch_smem(bk)));
   auto launch_all = [&]() -> int {
     QT_CHECK_CUDA(h, cudaMemsetAsync(b->d_counter, 0, sizeof(int) * std::max(nseg, 1), h->stream));
     for (int sg = 0; sg < nseg; sg++) {
@@ -667,12 +685,10 @@ extern "C" int qt_batch_run(qt_handle* h, qt_batch* b, int nlayers, const int* l
       al.task_end = seg_end[sg];
       al.counter = b->d_counter + sg;
       const int grid = std::min(dev_sms * b->cps[bk], seg_end[sg] - seg_begin[sg]);
-      switch (b->threads[bk]) {
-        case 128: QT_LAUNCH(h, batch_layer_kernel<128>, grid, 128, 0, al); break;
-        case 512: QT_LAUNCH(h, batch_layer_kernel<512>, grid, 512, 0, al); break;
-        case 1024: QT_LAUNCH(h, batch_layer_kernel<1024>, grid, 1024, 0, al); break;
-        default: QT_LAUNCH(h, batch_layer_kernel<256>, grid, 256, 0, al); break;
-      }
+      al.slab_elems = b->bucket_elems[bk];
+      al.smem_elems = (int)(batch_smem(bk) / sizeof(float2));
+      const layer_fn batch_layer_kernel_fn = layer_kernel(b->threads[bk], bk);
+      QT_LAUNCH(h, batch_layer_kernel_fn, grid, b->threads[bk], batch_smem(bk), al);
     }
     return QT_OK;
   };
@@ -794,10 +810,10 @@ extern "C" int qt_batch_expect_z(qt_handle* h, qt_batch* b, int site, double* ou
   double* d_out;
   QT_CHECK_CUDA(h, cudaMalloc(&d_out, sizeof(double) * b->ncirc));
   const int grid = std::min(b->ncirc, b->ctas);
-  // the slab holds 4 * slab_elems per CTA for the update; the sweep needs 3 (cap^2 each fits in one)
-  batch_expect_kernel<<<grid, BT, 0, h->stream>>>(b->d_sites, b->d_site_off, b->d_cap, b->d_nsites, b->d_bonds,
-                                                   b->d_bond_off, b->ncirc, site, b->d_slab, b->slab_elems / 4 + 1,
-                                                   d_out);
+  // the slab holds 16 cap^2 entries per CTA of the widest bucket; the sweep needs 6 cap^2
+  batch_expect_kernel<<<grid, BT, cta_gemm_smem<float2>(EXPECT_TILE), h->stream>>>(
+      b->d_sites, b->d_site_off, b->d_cap, b->d_nsites, b->d_bonds, b->d_bond_off, b->ncirc, site, b->d_slab,
+      b->bucket_elems[bucket_of(b->capmax)], d_out);
   h->launches++;
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(out, d_out, sizeof(double) * b->ncirc, cudaMemcpyDeviceToHost, h->stream);
