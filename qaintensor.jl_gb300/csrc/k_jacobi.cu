@@ -17,12 +17,14 @@
 //     unitaries (see the comment above that kernel);
 //   FP32 storage, two launches per round: pair_eig32_kernel (Gram + test +
 //     pair solver) and pair_apply32_kernel (rotation);
-//   FP64 storage, default: pair_round_kernel -- one launch per round, a
-//     thread-block cluster holding the pair's rows in shared memory;
+//   FP64 storage, default: pair_round64_kernel -- one launch per round, a
+//     thread-block cluster holding the pair's rows in shared memory, the
+//     rotation angles found in FP32 (see the comment above that kernel);
+//   FP32 storage on request: pair_round_kernel, the same shape of round;
 //   any storage: gram_kernel + eig_kernel + apply_kernel (partial Grams
 //     over row chunks, FP64 pair solver, rotation).
-// The FP64-storage solvers work on the FP64 Gram; the FP32-storage solvers
-// on the scaled FP32 Gram (cosines), see pair_eig_scaled below.
+// eig_kernel works on the FP64 Gram; the others on the scaled Gram (cosines) in
+// FP32, see pair_eig_scaled below.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -67,6 +69,16 @@ __device__ inline void pair_columns(int round, int pair, int nb, int nn, int* co
     const int gc = (c < JW) ? bi * JW + c : bj * JW + (c - JW);
     col[c] = (gc < nn) ? gc : -1;
   }
+}
+
+// partner of index y in inner round ir of the circle tournament over the 16
+// columns of a pair (the pairing of tournament(ir, ., 16)): 15 meets ir, the
+// others meet 2 ir - y (mod 15).  (Pairing the two blocks' columns first and
+// each block's own after converged in more outer sweeps.)
+__device__ inline int inner_partner(int ir, int y) {
+  if (y == JC - 1) return ir;
+  if (y == ir) return JC - 1;
+  return (2 * ir - y + (JC - 1)) % (JC - 1);
 }
 
 template <typename T> struct acc_of;
@@ -596,17 +608,15 @@ __device__ void stage_rows(const TS* __restrict__ M, int64_t ld, int nrows, int 
 // order, CTA 0 of the cluster tests the pair and diagonalises the Gram, the
 // other CTAs copy its unitary through distributed shared memory, and every
 // CTA rotates its own rows of X and its share of the rows of V.
-template <typename TS>
 __global__ void __launch_bounds__(NT)
-pair_round_kernel(TS* __restrict__ X, int64_t ldx, int mm, TS* __restrict__ V, int64_t ldv, int nn, int nb, int round,
+pair_round_kernel(float2* __restrict__ X, int64_t ldx, int mm, float2* __restrict__ V, int64_t ldv, int nn, int nb, int round,
                   int csize, int xrows_c, int vrows_c, int lds, double tol, double tol_inner, double nu_rel2,
                   const double* __restrict__ xnorm2, int* __restrict__ flags, int max_inner,
                   unsigned long long* __restrict__ phase_ns) {
-  typedef typename real_of<TS>::type RE;
+  typedef float2 TS;
   extern __shared__ __align__(16) unsigned char dyn_smem[];
   TS* Xs = reinterpret_cast<TS*>(dyn_smem);
-  constexpr bool F32 = sizeof(RE) == 4;
-  __shared__ typename std::conditional<F32, pair_eig_scaled, pair_eig_shared<double>>::type sh;
+  __shared__ pair_eig_scaled sh;
   __shared__ TS gpart[NGRAM];
   __shared__ int col[JC];
   __shared__ int any_rot, bad, offmax_blk, offbig_blk;
@@ -692,26 +702,21 @@ pair_round_kernel(TS* __restrict__ X, int64_t ldx, int mm, TS* __restrict__ V, i
         if (q < csize) sum_e = cadd(sum_e, ccast<double2>(v[q]));
       if (!isfinite(sum_e.x) || !isfinite(sum_e.y)) bad = 1;
     }
-    if constexpr (F32) {
-      __shared__ double dd[JC];
-      const int i = t / JC, j = t % JC;
-      if (i == j) {
-        dd[i] = sum_e.x;
-        sh.d[i] = (float)sum_e.x;
-        sh.d0[i] = (float)sum_e.x;
-      }
-      __syncthreads();
-      float2 v = make_float2(0.f, 0.f);
-      if (i != j && dd[i] > nu2 && dd[j] > nu2) {
-        const double sc = 1.0 / sqrt(dd[i] * dd[j]);
-        v = make_float2((float)(sum_e.x * sc), (float)(sum_e.y * sc));
-      }
-      sh.G[i][j] = v;
-      sh.W[i][j] = make_float2(i == j ? 1.f : 0.f, 0.f);
-    } else {
-      sh.G[t / JC][t % JC] = sum_e;
-      sh.W[t / JC][t % JC] = mk((RE)((t / JC) == (t % JC) ? 1 : 0), (RE)0);
+    __shared__ double dd[JC];
+    const int i = t / JC, j = t % JC;
+    if (i == j) {
+      dd[i] = sum_e.x;
+      sh.d[i] = (float)sum_e.x;
+      sh.d0[i] = (float)sum_e.x;
     }
+    __syncthreads();
+    float2 v = make_float2(0.f, 0.f);
+    if (i != j && dd[i] > nu2 && dd[j] > nu2) {
+      const double sc = 1.0 / sqrt(dd[i] * dd[j]);
+      v = make_float2((float)(sum_e.x * sc), (float)(sum_e.y * sc));
+    }
+    sh.G[i][j] = v;
+    sh.W[i][j] = make_float2(i == j ? 1.f : 0.f, 0.f);
   }
   cluster.sync();  // the partials have been read: CTAs 1.. may leave or move on
   phase(4);  // 3: partial sums + second barrier
@@ -729,13 +734,8 @@ pair_round_kernel(TS* __restrict__ X, int64_t ldx, int mm, TS* __restrict__ V, i
         if (i < j && col[i] >= 0 && col[j] >= 0) {
           double rel = 0, a, b;
           bool live;
-          if constexpr (F32) {
-            a = sh.d[i]; b = sh.d[j];
-            rel = sqrt((double)cabs2(sh.G[i][j]));
-          } else {
-            a = sh.G[i][i].x; b = sh.G[j][j].x;
-            if (a > nu2 && b > nu2) rel = sqrt(cabs2(sh.G[i][j])) / sqrt(a * b);
-          }
+          a = sh.d[i]; b = sh.d[j];
+          rel = sqrt((double)cabs2(sh.G[i][j]));
           live = a > nu2 && b > nu2;
           if (live && rel > tol) {
             any_rot = 1;
@@ -759,14 +759,9 @@ pair_round_kernel(TS* __restrict__ X, int64_t ldx, int mm, TS* __restrict__ V, i
     __syncthreads();
     if (any_rot) {
       if (t == 0) atomicAdd(&flags[QT_FLAG_ROTATED], 1);
-      int inner;
-      if constexpr (F32) {
-        inner = 0;
-        if (t < 32) inner = diagonalise_scaled_warp(sh, col, (float)tol_inner, (float)nu2, max_inner);
-        __syncthreads();
-      } else {
-        inner = diagonalise_pair<RE>(sh, col, tol_inner, nu2);
-      }
+      int inner = 0;
+      if (t < 32) inner = diagonalise_scaled_warp(sh, col, (float)tol_inner, (float)nu2, max_inner);
+      __syncthreads();
       if (t == 0) atomicAdd(&flags[QT_FLAG_INNER], inner);
     }
   }
@@ -790,6 +785,359 @@ pair_round_kernel(TS* __restrict__ X, int64_t ldx, int mm, TS* __restrict__ V, i
   stage_rows<TS>(V + vb, ldv, vr, vrows_c, col, Xs, lds);
   __syncthreads();
   rotate_rows<TS>(Xs, lds, vr, V + vb, ldv, col, sh.W);
+}
+
+// ---------------------------------------------------------------------------
+// FP64 storage: one launch per round, a cluster per pair
+// ---------------------------------------------------------------------------
+//
+// An SM has two FP64 lanes, so a warp instruction in FP64 occupies it for 16
+// cycles; what the round costs is FP64 instructions per SM and the latency of
+// the pair solver.
+//  - The pair's rows are spread over as many CTAs as the chip holds at once
+//    (clusters of up to 8, at least 8 rows each): Gram products and rotation
+//    are FP64 and shrink with the rows.
+//  - The rotation angles come from an FP32 two-sided Jacobi on the scaled Gram
+//    (cosines, each accurate relative to its own pair) with the diagonal kept
+//    as an FP32 pair (2^-48: the difference of nearly equal norms decides the
+//    angle).  Any angle gives a unitary rotation; one that is 1e-7 off leaves
+//    1e-7 of the pair's off-diagonal, which the next sweep measures from the
+//    FP64 columns again, so the iteration ends as with FP64 angles, at the
+//    same tolerance.  Each rotation (c, s e^{i phi}) is brought to unit length
+//    in FP64 and accumulated into the FP64 unitary by four further warps, one
+//    inner round behind the solver, while the solver's FP32 chain runs.
+//  - Every CTA of the cluster sums the partial Grams in rank order and runs the
+//    same solver on the same numbers, so the unitary needs no broadcast: one
+//    cluster barrier before the sums, one (split) before a CTA may leave.
+// Measured at 128 x 128 with V (8 pairs, clusters of 8; us per round): stage
+// 1.3, Gram 2.9, barrier 0.5, sums and test 4.6, solver 16, rotation 7.0 --
+// against 310 for one CTA per pair with an FP64 solver (Gram 42, solver 183,
+// rotation 25, unspread), and 46.5 -> 9.9 ms for the update of a bond of 64.
+
+constexpr int R64_SOLVE = 256;             // solver threads (warps 0-7)
+constexpr int R64_ACC = 128;               // unitary accumulation (warps 8-11)
+constexpr int NT64 = R64_SOLVE + R64_ACC;
+
+struct pair_solver64 {
+  float dh[2][JC], dl[2][JC];  // squared column norms, unevaluated pairs
+  float2 G[2][JC][JC + 1];     // scaled Gram (diagonal implicit 1)
+  float4 rot[2][JC];           // posted rotations (c, Re s e, Im s e, on) at the pair's lower index
+  int round[2];                // inner round of each post; -1: no more
+  double2 W[JC][JC + 1];       // the pair's unitary
+};
+
+template <int ID>
+__device__ inline void bar_sync(int n) { asm volatile("bar.sync %0, %1;" ::"n"(ID), "r"(n) : "memory"); }
+template <int ID>
+__device__ inline void bar_arrive(int n) { asm volatile("bar.arrive %0, %1;" ::"n"(ID), "r"(n) : "memory"); }
+// barriers 2, 3: post b is full; 4, 5: post b is free again
+__device__ inline void post_full_arrive(int b) { if (b) bar_arrive<3>(NT64); else bar_arrive<2>(NT64); }
+__device__ inline void post_full_wait(int b) { if (b) bar_sync<3>(NT64); else bar_sync<2>(NT64); }
+__device__ inline void post_free_arrive(int b) { if (b) bar_arrive<5>(NT64); else bar_arrive<4>(NT64); }
+__device__ inline void post_free_wait(int b) { if (b) bar_sync<5>(NT64); else bar_sync<4>(NT64); }
+__device__ inline void solver64_sync() { bar_sync<1>(R64_SOLVE); }
+
+// Warps 0-7: thread (x, y) computes the rotation of y's pair, takes x's from
+// lane x and updates Ghat[x][y] into the other buffer.  Posts every inner
+// round that rotates; the last post says so.
+__device__ int solve_pair64(pair_solver64& sh, const int* col, float tol_inner, float nu2, int max_inner) {
+  const int t = threadIdx.x, x = (t >> 4) & 15, y = t & 15;
+  const float tol2 = tol_inner * tol_inner;
+  int cur = 0, sweep = 0, posts = 0;
+  for (; sweep < max_inner; sweep++) {
+    bool rotated_any = false;
+    for (int ir = 0; ir < JC - 1; ir++) {
+      const int yp = inner_partner(ir, y), xp = inner_partner(ir, x);
+      const int p = min(y, yp), q = max(y, yp);
+      const float a = sh.dh[cur][p], b = sh.dh[cur][q], al = sh.dl[cur][p], bl = sh.dl[cur][q];
+      const float2 gs = sh.G[cur][p][q];
+      const float ags2 = gs.x * gs.x + gs.y * gs.y;
+      const bool rotp = col[p] >= 0 && col[q] >= 0 && a > nu2 && b > nu2 && ags2 > tol2;
+      if (!__any_sync(0xffffffffu, rotp)) continue;  // the same vote in every solver warp
+      rotated_any = true;
+      float2 jpp = make_float2(1.f, 0.f), jqp = make_float2(0.f, 0.f), jpq = jqp, jqq = jpp;
+      float a2 = a, b2 = b, a2l = al, b2l = bl;
+      float4 post = make_float4(1.f, 0.f, 0.f, 0.f);
+      if (rotp) {
+        const float ria = rsqrtf(a), rib = rsqrtf(b), rags = rsqrtf(ags2);
+        const float sqa = a * ria, sqb = b * rib;
+        const float ag = ags2 * rags * sqa * sqb;  // |gamma|
+        // the leading parts subtract exactly where they are close, and the
+        // trailing ones matter only there
+        const float diff = __fadd_rn(__fsub_rn(b, a), __fsub_rn(bl, al));
+        const float zeta = 0.5f * (diff * ria * rib) * rags;
+        const float az = fabsf(zeta);
+        // (az^2 would overflow where norms 1e14 apart meet cosines of 1e-13)
+        const float tt = copysignf(__fdividef(1.f, az > 1e6f ? 2.f * az : az + sqrtf(fmaf(az, az, 1.f))), zeta);
+        const float c = rsqrtf(fmaf(tt, tt, 1.f)), sn = c * tt;
+        const float2 e = make_float2(gs.x * rags, gs.y * rags);
+        const float d = tt * ag;
+        // a - d and b + d as pairs
+        {
+          const float s = __fsub_rn(a, d), bb = __fsub_rn(s, a);
+          const float er = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(-d, bb));
+          a2 = __fadd_rn(s, __fadd_rn(er, al));
+          a2l = __fsub_rn(__fadd_rn(er, al), __fsub_rn(a2, s));
+          if (!(a2 > nu2)) { a2 = nu2; a2l = 0.f; }  // a column driven to the noise level is frozen
+        }
+        {
+          const float s = __fadd_rn(b, d), bb = __fsub_rn(s, b);
+          const float er = __fadd_rn(__fsub_rn(b, __fsub_rn(s, bb)), __fsub_rn(d, bb));
+          b2 = __fadd_rn(s, __fadd_rn(er, bl));
+          b2l = __fsub_rn(__fadd_rn(er, bl), __fsub_rn(b2, s));
+        }
+        const float ia2 = rsqrtf(a2), ib2 = rsqrtf(b2);
+        const float fa = sqa * ia2, fb = sqb * ib2, fab = sqb * ia2, fba = sqa * ib2;
+        jpp = make_float2(c * fa, 0.f);
+        jqp = make_float2(-sn * e.x * fab, sn * e.y * fab);  // -s conj(e) sqrt(b/a')
+        jpq = make_float2(sn * e.x * fba, sn * e.y * fba);   //  s e sqrt(a/b')
+        jqq = make_float2(c * fb, 0.f);
+        post = make_float4(c, sn * e.x, sn * e.y, 1.f);
+      }
+      const bool low = y == p;
+      // post the round's rotations for the accumulation
+      const int pb = posts & 1;
+      if (posts >= 2) post_free_wait(pb);
+      if (x == 0 && low) sh.rot[pb][p] = post;
+      if (t == 0) sh.round[pb] = ir;
+      post_full_arrive(pb);
+      posts++;
+      const float2 jyy = low ? jpp : jqq, jpy = low ? jqp : jpq;
+      float2 jxx, jpx;
+      jxx.x = __shfl_sync(0xffffffffu, jyy.x, x);
+      jxx.y = __shfl_sync(0xffffffffu, jyy.y, x);
+      jpx.x = __shfl_sync(0xffffffffu, jpy.x, x);
+      jpx.y = __shfl_sync(0xffffffffu, jpy.y, x);
+      if (x == y) {
+        sh.dh[cur ^ 1][y] = low ? a2 : b2;
+        sh.dl[cur ^ 1][y] = low ? a2l : b2l;
+      }
+      float2 gnew = make_float2(0.f, 0.f);
+      if (xp == y && x != y) {
+        if (!rotp) gnew = sh.G[cur][x][y];
+      } else if (x != y) {
+        const float2 g_xy = sh.G[cur][x][y], g_xq = sh.G[cur][x][yp];
+        const float2 g_py = sh.G[cur][xp][y], g_pq = sh.G[cur][xp][yp];
+        const float2 hx = cadd(cmul(g_xy, jyy), cmul(g_xq, jpy));
+        const float2 hp = cadd(cmul(g_py, jyy), cmul(g_pq, jpy));
+        gnew = cadd(cmul(cconj(jxx), hx), cmul(cconj(jpx), hp));
+      }
+      sh.G[cur ^ 1][x][y] = gnew;
+      cur ^= 1;
+      solver64_sync();
+    }
+    if (!rotated_any) break;  // every solver warp took the same votes
+  }
+  const int pb = posts & 1;
+  if (posts >= 2) post_free_wait(pb);
+  if (t == 0) sh.round[pb] = -1;
+  post_full_arrive(pb);
+  if (posts >= 1) post_free_wait(pb ^ 1);  // every post was taken: the barriers end even
+  return sweep + (sweep < max_inner ? 1 : 0);
+}
+
+// Warps 8-11: W <- W J for every posted round.  Warp w holds rows 4 w .. 4 w + 3,
+// lane (row, pair); a row stays with its warp.
+__device__ void accumulate_pair64(pair_solver64& sh) {
+  const int t = threadIdx.x - R64_SOLVE, r = t >> 3, k = t & 7;
+  for (int i = 0;; i++) {
+    const int pb = i & 1;
+    post_full_wait(pb);
+    const int ir = sh.round[pb];
+    if (ir < 0) return;
+    int p, q;
+    tournament(ir, k, JC, p, q);
+    const float4 v = sh.rot[pb][p];
+    if (v.w != 0.f) {
+      // |(c, sr, si)|^2 = 1 - d with d ~ 1e-7: times 1 + d/2 + 3 d^2/8, to 1e-21
+      double c = v.x, sr = v.y, si = v.z;
+      const double d = fma(-si, si, fma(-sr, sr, fma(-c, c, 1.0)));
+      const double h = d * fma(0.375, d, 0.5);
+      c = fma(h, c, c);
+      sr = fma(h, sr, sr);
+      si = fma(h, si, si);
+      // w_p' = c w_p - conj(se) w_q ;  w_q' = se w_p + c w_q
+      const double2 u = sh.W[r][p], w = sh.W[r][q];
+      sh.W[r][p] = make_double2(fma(c, u.x, -fma(sr, w.x, si * w.y)), fma(c, u.y, -fma(sr, w.y, -(si * w.x))));
+      sh.W[r][q] = make_double2(fma(c, w.x, fma(sr, u.x, -(si * u.y))), fma(c, w.y, fma(sr, u.y, si * u.x)));
+    }
+    __syncwarp();
+    post_free_arrive(pb);
+  }
+}
+
+// rows [0, nrows) of the pair's columns of M -> Xs (column c at Xs + c * lds)
+__device__ inline void stage_rows64(const double2* __restrict__ M, int64_t ld, int nrows, const int* col,
+                                    double2* __restrict__ Xs, int lds) {
+  for (int idx = threadIdx.x; idx < nrows * JC; idx += NT64) {
+    const int r = idx % nrows, c = idx / nrows;
+    Xs[c * lds + r] = col[c] >= 0 ? M[r + ld * col[c]] : make_double2(0, 0);
+  }
+}
+
+// M[r, col[c]] = sum_k Xs[k][r] W[k][c]: one output per thread and turn, lanes
+// along the rows (FP64-bound: two shared loads per four FMAs of 16 cycles)
+__device__ inline void rotate_rows64(const double2* __restrict__ Xs, int lds, int nrows, double2* __restrict__ M,
+                                     int64_t ld, const int* col, const double2 (*W)[JC + 1]) {
+  for (int idx = threadIdx.x; idx < nrows * JC; idx += NT64) {
+    const int r = idx % nrows, c = idx / nrows;
+    if (col[c] < 0) continue;
+    double2 acc = make_double2(0, 0);
+#pragma unroll
+    for (int k = 0; k < JC; k++) cfma(acc, Xs[k * lds + r], W[k][c]);
+    M[r + ld * col[c]] = acc;
+  }
+}
+
+// grid: pairs x csize.  CTA q of a cluster holds rows [q xrows, (q + 1) xrows)
+// of the pair's columns of X, and (vboth: staged at the start, beside X) rows
+// [q vrows, ...) of V.
+__global__ void __launch_bounds__(NT64)
+pair_round64_kernel(double2* __restrict__ X, int64_t ldx, int mm, double2* __restrict__ V, int64_t ldv, int nn, int nb,
+                    int round, int csize, int xrows, int vrows, int lds, int vboth, double tol, double nu_rel2,
+                    const double* __restrict__ xnorm2, int* __restrict__ flags, int max_inner,
+                    unsigned long long* __restrict__ phase_ns) {
+  extern __shared__ __align__(16) unsigned char dyn_smem[];
+  double2* Xs = reinterpret_cast<double2*>(dyn_smem);
+  double2* Vs = vboth ? Xs + (size_t)JC * lds : Xs;
+  __shared__ pair_solver64 sh;
+  __shared__ double2 gpart[JC * (JC + 1)];
+  __shared__ int col[JC];
+  __shared__ int any_rot, bad, offmax_blk, offbig_blk;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int crank = (int)cluster.block_rank();
+  const int pair = blockIdx.x / csize;
+  const int t = threadIdx.x;
+  unsigned long long tp = 0;
+  auto phase = [&](int ph) {  // optional diagnostics: thread 0's time per phase
+    if (phase_ns && t == 0) {
+      unsigned long long tn;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(tn));
+      if (ph > 0) atomicAdd(&phase_ns[8 * (crank != 0) + ph - 1], tn - tp);
+      tp = tn;
+    }
+  };
+  phase(0);
+  pair_columns(round, pair, nb, nn, col);
+  if (t == 0) { any_rot = 0; bad = 0; offmax_blk = 0; offbig_blk = 0; }
+  // powers-of-two multiples bring ||X||_F^2 into [1, 2) for the solver
+  __shared__ double unit_sh;
+  __shared__ float nu2_sh, big2_sh;
+  if (t == NT64 - 1) {
+    const double xn2 = *xnorm2;
+    const double unit = xn2 > 0 && isfinite(xn2) ? ldexp(1.0, -ilogb(xn2)) : 1.0;
+    unit_sh = unit;
+    nu2_sh = (float)(nu_rel2 * xn2 * unit);
+    big2_sh = (float)(1e-6 * xn2 * unit);
+  }
+  for (int e = t; e < NGRAM; e += NT64) sh.W[e / JC][e % JC] = make_double2(e / JC == e % JC ? 1.0 : 0.0, 0.0);
+  __syncthreads();
+  const int xb = crank * xrows, xr = max(0, min(mm, xb + xrows) - xb);
+  const int vb = crank * vrows, vr = V ? max(0, min(nn, vb + vrows) - vb) : 0;
+  stage_rows64(X + xb, ldx, xr, col, Xs, lds);
+  if (vboth && vr > 0) stage_rows64(V + vb, ldv, vr, col, Vs, lds);
+  __syncthreads();
+  phase(1);  // 0: stage
+  // partial Gram: one upper entry per thread over every row, two row groups
+  // from 32 rows on (FP64-bound: sharing operands between entries would save
+  // shared loads that cost nothing here, and its reductions would be FP64 adds)
+  constexpr int NU = JC * (JC + 1) / 2;
+  int gi = 0, gj = 0;
+  const int groups = xr >= 32 ? 2 : 1;
+  double2 g_e = make_double2(0, 0);
+  if (t < NU * groups) {
+    int rem = t % NU;
+    while (rem >= JC - gi) { rem -= JC - gi; gi++; }
+    gj = gi + rem;
+    const double2 *xi = Xs + gi * lds, *xj = Xs + gj * lds;
+#pragma unroll 4
+    for (int rr = t / NU; rr < xr; rr += groups) cfma_conj(g_e, xi[rr], xj[rr]);
+    if (t >= NU) gpart[NU + (t - NU)] = g_e;
+  }
+  if (groups == 2) __syncthreads();
+  if (t < NU) {
+    if (groups == 2) g_e = cadd(g_e, gpart[NU + t]);
+    gpart[t] = g_e;
+  }
+  phase(2);  // 1: Gram
+  cluster.sync();
+  phase(3);  // 2: cluster barrier
+  // the upper entries, partials added in rank order
+  const double unit = unit_sh;
+  const float nu2 = nu2_sh, big2 = big2_sh;
+  const bool upper = t < NU;
+  if (upper) {
+    // all remote loads in flight before the first sum
+    double2 v[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+      if (q < csize) v[q] = cluster.map_shared_rank(gpart, q)[t];
+    g_e = v[0];
+#pragma unroll
+    for (int q = 1; q < 8; q++)
+      if (q < csize) g_e = cadd(g_e, v[q]);
+    if (!isfinite(g_e.x) || !isfinite(g_e.y)) bad = 1;
+    if (gi == gj) {
+      const double d = fmax(g_e.x * unit, 0.0);
+      sh.dh[0][gi] = (float)d;
+      sh.dl[0][gi] = (float)(d - (double)(float)d);
+    }
+  }
+  // this CTA has read the partials; it may leave once all have
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  __syncthreads();
+  if (upper) {
+    float2 v = make_float2(0.f, 0.f);
+    const float di = sh.dh[0][gi], dj = sh.dh[0][gj];
+    if (gi != gj && di > nu2 && dj > nu2) {
+      const double ri = rsqrtf(di), rj = rsqrtf(dj) * unit;
+      v = make_float2((float)(g_e.x * ri * rj), (float)(g_e.y * ri * rj));
+    }
+    sh.G[0][gi][gj] = v;
+    sh.G[0][gj][gi] = cconj(v);
+    // is this pair already orthogonal to tol?
+    if (!bad && gi != gj && col[gi] >= 0 && col[gj] >= 0 && di > nu2 && dj > nu2) {
+      const float rel = fminf(sqrtf(cabs2(v)), 1.f);
+      if (rel > (float)tol) {
+        any_rot = 1;
+        atomicMax(&offmax_blk, __float_as_int(rel));
+        if (di > big2 && dj > big2) atomicMax(&offbig_blk, __float_as_int(rel));
+      }
+    }
+  }
+  __syncthreads();
+  phase(4);  // 3: sums, cosines, test
+  if (t == 0 && crank == 0) {
+    if (bad) atomicOr(&flags[QT_FLAG_NONFINITE], 1);
+    if (any_rot) atomicAdd(&flags[QT_FLAG_ROTATED], 1);
+    if (offmax_blk > 0) atomicMax(&flags[QT_FLAG_OFFMAX], offmax_blk);
+    if (offbig_blk > 0) atomicMax(&flags[QT_FLAG_OFFBIG], offbig_blk);
+  }
+  if (any_rot) {
+    // down to 1e-6 of the pair's largest cosine: FP32 angles reach no further
+    const float tol_inner = fmaxf(1e-14f, 1e-6f * __int_as_float(offmax_blk));
+    if (t < R64_SOLVE) {
+      const int inner = solve_pair64(sh, col, fminf(tol_inner, (float)tol), nu2, max_inner);
+      if (t == 0 && crank == 0) atomicAdd(&flags[QT_FLAG_INNER], inner);
+    } else {
+      accumulate_pair64(sh);
+    }
+    __syncthreads();
+    phase(5);  // 4: pair solver
+    rotate_rows64(Xs, lds, xr, X + xb, ldx, col, sh.W);
+    if (vr > 0) {
+      if (!vboth) {
+        __syncthreads();  // Xs is reused for V
+        stage_rows64(V + vb, ldv, vr, col, Vs, lds);
+        __syncthreads();
+      }
+      rotate_rows64(Vs, lds, vr, V + vb, ldv, col, sh.W);
+    }
+    phase(6);  // 5: rotation
+  }
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // grid (pair, row chunk): apply the pair's unitary to this chunk's rows of X and V.
@@ -1094,16 +1442,6 @@ struct sweep_solver {
   float2 G[2][JC][JC + 1];
   float2 W[2][JC][JC + 1];
 };
-
-// partner of index y in inner round ir of the circle tournament over the 16
-// columns of a pair (the pairing of tournament(ir, ., 16)): 15 meets ir, the
-// others meet 2 ir - y (mod 15).  (Pairing the two blocks' columns first and
-// each block's own after converged in more outer sweeps.)
-__device__ inline int inner_partner(int ir, int y) {
-  if (y == JC - 1) return ir;
-  if (y == ir) return JC - 1;
-  return (2 * ir - y + (JC - 1)) % (JC - 1);
-}
 
 // named barrier of the 256 solver threads (warps 0-7)
 __device__ inline void solver_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
@@ -1582,11 +1920,12 @@ int qt_jacobi_layout(int64_t mm, int64_t nn, int* nb_out, int* chunks_out) {
   return pairs * chunks * NGRAM + 1 + pairs * NGRAM + pairs;
 }
 
-// Cluster shape of the one-launch round: the smallest cluster (<= 8 CTAs)
+// Cluster shape of the one-launch FP32 round: the smallest cluster (<= 8 CTAs)
 // whose row slice of the 16 pair columns fits in FUSED_SMEM bytes of shared
 // memory, widened while the grid would leave SMs idle.  0 = does not fit.
 constexpr size_t FUSED_SMEM = 100 * 1024;
-static int fused_shape(int64_t mm, int pairs, size_t elem, int* rows_c, int* lds, size_t* smem) {
+static int fused_shape(int64_t mm, int pairs, int* rows_c, int* lds, size_t* smem) {
+  const size_t elem = sizeof(float2);
   int csize = 0;
   for (int c = 1; c <= 8; c *= 2) {
     const int64_t rc = (mm + c - 1) / c;
@@ -1608,8 +1947,7 @@ static int fused_shape(int64_t mm, int pairs, size_t elem, int* rows_c, int* lds
   return csize;
 }
 
-template <typename TS>
-static int launch_pair_round(qt_handle* h, int csize, int pairs, size_t smem, TS* X, int64_t ldx, int mm, TS* V,
+static int launch_pair_round(qt_handle* h, int csize, int pairs, size_t smem, float2* X, int64_t ldx, int mm, float2* V,
                              int64_t ldv, int nn, int nb, int round, int xrows_c, int vrows_c, int lds, double tol,
                              double tol_inner, double nu_rel2, const double* xnorm2, int max_inner,
                              unsigned long long* phase_ns) {
@@ -1625,13 +1963,77 @@ static int launch_pair_round(qt_handle* h, int csize, int pairs, size_t smem, TS
   attr[0].val.clusterDim.z = 1;
   lc.attrs = attr;
   lc.numAttrs = 1;
-  if (h->prof) qt_prof_before(h, "pair_round_kernel<TS>");
-  const cudaError_t e = cudaLaunchKernelEx(&lc, pair_round_kernel<TS>, X, ldx, mm, V, ldv, nn, nb, round, csize,
+  if (h->prof) qt_prof_before(h, "pair_round_kernel");
+  const cudaError_t e = cudaLaunchKernelEx(&lc, pair_round_kernel, X, ldx, mm, V, ldv, nn, nb, round, csize,
                                            xrows_c, vrows_c, lds, tol, tol_inner, nu_rel2, xnorm2, h->d_flags, max_inner,
                                            phase_ns);
   if (h->prof) qt_prof_after(h);
   h->launches++;
   if (e != cudaSuccess) return qt_fail(h, QT_ECUDA, std::string("launch pair_round_kernel: ") + cudaGetErrorString(e));
+  return QT_OK;
+}
+
+// Shape of the FP64 round: the widest cluster (<= 8 CTAs) that keeps the grid
+// on the chip at once (152 SMs) with at least 8 rows of X per CTA, wider still
+// while the row slices do not fit.  Rows and not columns are spread because
+// the FP64 work of a CTA is its rows times the pair's 16 x 16 entries.
+// 128 x 128 with V (8 pairs), 10 sweeps: clusters of 8 9.9 ms an update, of 16
+// (8 rows each) 11.3 ms -- what the rotation gains, the launch of the wider
+// clusters loses.
+struct round64_shape {
+  int csize = 0, xrows = 0, vrows = 0, lds = 0, vboth = 0;
+  size_t smem = 0;
+};
+constexpr size_t R64_SMEM = 200 * 1024;
+static bool round64_fill(int64_t mm, int64_t vn, int c, round64_shape* s) {
+  s->csize = c;
+  s->xrows = (int)((mm + c - 1) / c);
+  s->vrows = (int)((vn + c - 1) / c);
+  s->lds = std::max(s->xrows, s->vrows) | 1;  // odd: columns start in different banks
+  const size_t slice = (size_t)s->lds * JC * sizeof(double2);
+  s->vboth = vn > 0 && 2 * slice <= R64_SMEM;
+  s->smem = slice * (s->vboth ? 2 : 1);
+  return s->smem <= R64_SMEM;
+}
+static round64_shape shape_round64(int64_t mm, int64_t vn, int pairs) {
+  round64_shape s, best;
+  for (int c = 1; c <= 8; c *= 2) {
+    if (!round64_fill(mm, vn, c, &s)) continue;
+    const bool wider = c > 1 && pairs * c <= 152 && s.xrows >= 8;
+    if (best.csize && !wider) break;
+    best = s;
+  }
+  // QT_JACOBI_CLUSTER=c (1, 2, 4 or 8) overrides the cluster size where the slice fits
+  if (const char* env = std::getenv("QT_JACOBI_CLUSTER")) {
+    const int c = std::atoi(env);
+    if ((c == 1 || c == 2 || c == 4 || c == 8) && round64_fill(mm, vn, c, &s)) best = s;
+  }
+  return best;
+}
+
+static int launch_pair_round64(qt_handle* h, const round64_shape& sh, int pairs, double2* X, int64_t ldx, int mm,
+                               double2* V, int64_t ldv, int nn, int nb, int round, double tol, double nu_rel2,
+                               const double* xnorm2, int max_inner, unsigned long long* phase_ns) {
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3((unsigned)(pairs * sh.csize));
+  lc.blockDim = dim3(NT64);
+  lc.dynamicSmemBytes = sh.smem;
+  lc.stream = h->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)sh.csize;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  lc.attrs = attr;
+  lc.numAttrs = 1;
+  if (h->prof) qt_prof_before(h, "pair_round64_kernel");
+  const cudaError_t e = cudaLaunchKernelEx(&lc, pair_round64_kernel, X, ldx, mm, V, ldv, nn, nb, round, sh.csize,
+                                           sh.xrows, sh.vrows, sh.lds, sh.vboth, tol, nu_rel2, xnorm2, h->d_flags,
+                                           max_inner, phase_ns);
+  if (h->prof) qt_prof_after(h);
+  h->launches++;
+  if (e != cudaSuccess)
+    return qt_fail(h, QT_ECUDA, std::string("launch pair_round64_kernel: ") + cudaGetErrorString(e));
   return QT_OK;
 }
 
@@ -1738,7 +2140,9 @@ int qt_jacobi_svd_ws(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, T
   const bool two_launch = fp32 && (jk == 3 || (jk == 0 && !sweep_kernel));
   int xrows_c = 0, lds = 0;
   size_t smem = 0;
-  const int csize = (jk == 1 || two_launch || sweep_kernel) ? 0 : fused_shape(mm, pairs, sizeof(TS), &xrows_c, &lds, &smem);
+  const bool one_launch = jk != 1 && !two_launch && !sweep_kernel;
+  const round64_shape r64 = one_launch && !fp32 ? shape_round64(mm, V ? nn : 0, pairs) : round64_shape();
+  const int csize = !one_launch ? 0 : fp32 ? fused_shape(mm, pairs, &xrows_c, &lds, &smem) : r64.csize;
   // two-launch shape: one row per rotation thread, about eight CTAs per SM
   int achunks = std::max(1, std::min<int>((8 * 152 + pairs - 1) / pairs, (int)((mm + NT - 1) / NT)));
   const int axrows = (int)(((mm + achunks - 1) / achunks + 31) / 32 * 32);
@@ -1747,9 +2151,11 @@ int qt_jacobi_svd_ws(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, T
   // the inner eigen-solve is driven well below the outer threshold so that the
   // rounding of the applied rotation cannot leave the pair just above `tol`
   const double tol_inner = fp32 ? tol / 16.0 : std::min(tol, 1e-14);
-  if (csize)
-    QT_CHECK_CUDA(h, cudaFuncSetAttribute(pair_round_kernel<TS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem));
+  if (csize && fp32)
+    QT_CHECK_CUDA(h, cudaFuncSetAttribute(pair_round_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (csize && !fp32)
+    QT_CHECK_CUDA(h, cudaFuncSetAttribute(pair_round64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)r64.smem));
   // QT_JACOBI_TRACE=1 in the environment prints one line per sweep to stderr;
   // QT_JACOBI_PHASES=1 adds the average time per phase of the one-launch
   // rounds at the end (CTA 0 of each cluster / the others); a handle without
@@ -1814,14 +2220,15 @@ int qt_jacobi_svd_ws(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, T
   }
   int sweep = 0;
   for (; sweep < max_sweeps; sweep++) {
-    // the pair solver runs up to 12 inner sweeps in the first two outer
-    // sweeps (FP32 storage: 2, which measured fastest overall); once the
-    // pairs are close to orthogonal one inner sweep of rotations reduces
-    // them quadratically and the outer test decides convergence
-    // (QT_JACOBI_INNER0 / QT_JACOBI_INNER override the two caps)
+    // FP32 storage: up to 2 inner sweeps of the pair solver in the first two
+    // outer sweeps (measured fastest); once the pairs are close to orthogonal
+    // one inner sweep of rotations reduces them quadratically and the outer
+    // test decides convergence.  FP64 storage: one throughout (1, 2, 4 and 12
+    // in the first two took 10.9, 11.3, 13.6 and 14.0 ms at 128 x 128).
+    // QT_JACOBI_INNER0 / QT_JACOBI_INNER override the two caps.
     static const int inner_cap = std::getenv("QT_JACOBI_INNER") ? std::atoi(std::getenv("QT_JACOBI_INNER")) : 1;
     static const int inner_cap0 =
-        std::getenv("QT_JACOBI_INNER0") ? std::atoi(std::getenv("QT_JACOBI_INNER0")) : (fp32 ? 2 : MAX_INNER);
+        std::getenv("QT_JACOBI_INNER0") ? std::atoi(std::getenv("QT_JACOBI_INNER0")) : (fp32 ? 2 : 1);
     const int max_inner = std::max(1, std::min(sweep < 2 ? inner_cap0 : inner_cap, MAX_INNER));
     QT_CHECK_CUDA(h, cudaMemsetAsync(h->d_flags, 0, sizeof(int) * QT_FLAG_COUNT, h->stream));
     if (sweep_kernel) {
@@ -1845,8 +2252,12 @@ int qt_jacobi_svd_ws(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, T
         continue;
       }
       if (csize) {
-        QT_TRY(launch_pair_round<TS>(h, csize, pairs, smem, X, ldx, (int)mm, V, ldv, (int)nn, nb, r, xrows_c, vrows_c,
-                                     lds, tol, tol_inner, nu_rel2, xnorm2, max_inner, phase_ns));
+        if constexpr (sizeof(typename real_of<TS>::type) == 4)
+          QT_TRY(launch_pair_round(h, csize, pairs, smem, X, ldx, (int)mm, V, ldv, (int)nn, nb, r, xrows_c, vrows_c,
+                                   lds, tol, tol_inner, nu_rel2, xnorm2, max_inner, phase_ns));
+        else
+          QT_TRY(launch_pair_round64(h, r64, pairs, X, ldx, (int)mm, V, ldv, (int)nn, nb, r, tol, nu_rel2, xnorm2,
+                                     max_inner, phase_ns));
         continue;
       }
       QT_LAUNCH(h, (gram_kernel<TS, TG>), grid, NT, 0, X, ldx, (int)mm, (int)nn, nb, r, xrows, parts);
@@ -1951,7 +2362,9 @@ int qt_jacobi_svd_ws(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, T
     unsigned long long hp[16];
     QT_CHECK_CUDA(h, cudaMemcpy(hp, phase_ns, sizeof(hp), cudaMemcpyDeviceToHost));
     const double launches = (double)(*sweeps_out) * rounds;
-    const char* nm[7] = {"stage", "gram", "barrier1", "sums+barrier2", "test+solver", "barriers+copy", "rotate"};
+    const char* nm32[7] = {"stage", "gram", "barrier1", "sums+barrier2", "test+solver", "barriers+copy", "rotate"};
+    const char* nm64[7] = {"stage", "gram", "barrier", "sums+test", "solver", "rotate", "-"};
+    const char** nm = fp32 ? nm32 : nm64;
     for (int g = 0; g < 2; g++) {
       const double ctas = launches * pairs * (g == 0 ? 1 : csize - 1);
       std::fprintf(stderr, "jacobi phases (%s), us per CTA per round:", g == 0 ? "CTA 0" : "other CTAs");

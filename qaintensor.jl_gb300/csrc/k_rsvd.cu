@@ -5,8 +5,8 @@
 // Gram-Schmidt with one re-orthogonalisation pass (BCGS2), each 32-column
 // block orthonormalised by CholeskyQR passes -- the first one shifted
 // (Fukaya, Kannan, Nakatsukasa, Zhang, Yamamoto 2020) so that numerically
-// rank-deficient blocks still factor, and a third one for an FP32 basis.  The
-// basis is stored in the element type of Y.  Three implementations:
+// rank-deficient blocks still factor, and a third one.  The basis is stored in
+// the element type of Y.  Three implementations:
 //   - FP32 bases of up to 2368 rows (whose rows fit the shared memory of one
 //     CTA per 16 rows): the whole orthonormalisation in one cooperative
 //     launch (orth_one_launch_kernel), grid barriers between its phases.
@@ -1373,9 +1373,11 @@ int qt_orthonormalize(qt_handle* h, C* Y, int64_t m, int64_t l, int use) {
       if (j0 > 0) QT_TRY(block_project<C>(h, Y, m, (int)j0, Yb, b, part, coef));
       QT_TRY(block_cholqr<C>(h, Yb, m, b, pass == 0, dG));
     }
-    // one more CholeskyQR (shifted CholeskyQR3): after a shifted pass with
-    // the FP32 shift the block is only well conditioned, not orthonormal
-    if (sizeof(typename real_of<C>::type) == 4) QT_TRY(block_cholqr<C>(h, Yb, m, b, false, dG));
+    // one more CholeskyQR (shifted CholeskyQR3): after a shifted pass the
+    // block is only well conditioned, not orthonormal, and the next pass
+    // leaves cond^2 u of that -- with the FP64 shift 5e-7 to 6e-3 for blocks
+    // of 7 to 31 columns whose norms fall over 14 decades
+    QT_TRY(block_cholqr<C>(h, Yb, m, b, false, dG));
   }
   if (phase_ns && cq_launches > 0) {
     unsigned long long hp[8];
