@@ -17,17 +17,19 @@ struct GateParam {
 
 // Each CTA owns a block of TA values of a and TB values of b and computes all
 // four (s1, s2) combinations for them, so the 4x4 gate mixes values that sit
-// in one thread's registers.  Thread (tx, ty) owns a = a0 + tx + 16 i,
-// b = b0 + ty + 16 j.  Accumulation in R (double or float).
-template <typename TI, typename R, typename TO, int RA, int RB>
-__global__ void __launch_bounds__(256)
+// in one thread's registers.  Thread (tx, ty) owns a = a0 + tx + TX i,
+// b = b0 + ty + TX j.  Accumulation in R (double or float).
+// TX: threads along each side.  FP64 is bound by the two FP64 lanes of an SM,
+// so it takes 8 x 8 threads, four times the CTAs (bond of 64: 82 -> 52 us).
+template <typename TI, typename R, typename TO, int RA, int RB, int TX>
+__global__ void __launch_bounds__(TX * TX)
 theta_gate_kernel(const TI* __restrict__ A, const TI* __restrict__ B, int chil, int chim, int chir,
                   GateParam gp, TO* __restrict__ out) {
   typedef typename cplx_of<R>::type CR;
-  constexpr int TA = 16 * RA, TB = 16 * RB, KC = 16;
+  constexpr int TA = TX * RA, TB = TX * RB, KC = 16, NT = TX * TX;
   __shared__ CR As[2][KC][TA];
   __shared__ CR Bs[2][KC][TB + 1];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
   const int a0 = blockIdx.x * TA, b0 = blockIdx.y * TB;
   CR acc[RA][RB][2][2];
 #pragma unroll
@@ -38,14 +40,14 @@ theta_gate_kernel(const TI* __restrict__ A, const TI* __restrict__ B, int chil, 
       for (int s = 0; s < 4; s++) acc[i][j][s >> 1][s & 1] = czero<CR>();
 
   for (int k0 = 0; k0 < chim; k0 += KC) {
-    for (int idx = threadIdx.x; idx < 2 * KC * TA; idx += 256) {
+    for (int idx = threadIdx.x; idx < 2 * KC * TA; idx += NT) {
       const int a = idx % TA, k = (idx / TA) % KC, s = idx / (TA * KC);
       const int ga = a0 + a, gk = k0 + k;
       CR v = czero<CR>();
       if (ga < chil && gk < chim) v = ccast<CR>(A[ga + (int64_t)chil * (s + 2 * (int64_t)gk)]);
       As[s][k][a] = v;
     }
-    for (int idx = threadIdx.x; idx < 2 * KC * TB; idx += 256) {
+    for (int idx = threadIdx.x; idx < 2 * KC * TB; idx += NT) {
       const int k = idx % KC, b = (idx / KC) % TB, s = idx / (KC * TB);
       const int gb = b0 + b, gk = k0 + k;
       CR v = czero<CR>();
@@ -58,13 +60,13 @@ theta_gate_kernel(const TI* __restrict__ A, const TI* __restrict__ B, int chil, 
       CR av[RA][2], bv[RB][2];
 #pragma unroll
       for (int i = 0; i < RA; i++) {
-        av[i][0] = As[0][k][tx + 16 * i];
-        av[i][1] = As[1][k][tx + 16 * i];
+        av[i][0] = As[0][k][tx + TX * i];
+        av[i][1] = As[1][k][tx + TX * i];
       }
 #pragma unroll
       for (int j = 0; j < RB; j++) {
-        bv[j][0] = Bs[0][k][ty + 16 * j];
-        bv[j][1] = Bs[1][k][ty + 16 * j];
+        bv[j][0] = Bs[0][k][ty + TX * j];
+        bv[j][1] = Bs[1][k][ty + TX * j];
       }
 #pragma unroll
       for (int i = 0; i < RA; i++)
@@ -82,11 +84,11 @@ theta_gate_kernel(const TI* __restrict__ A, const TI* __restrict__ B, int chil, 
   const int64_t ldo = 2 * (int64_t)chil;
 #pragma unroll
   for (int i = 0; i < RA; i++) {
-    const int a = a0 + tx + 16 * i;
+    const int a = a0 + tx + TX * i;
     if (a >= chil) continue;
 #pragma unroll
     for (int j = 0; j < RB; j++) {
-      const int b = b0 + ty + 16 * j;
+      const int b = b0 + ty + TX * j;
       if (b >= chir) continue;
 #pragma unroll
       for (int o = 0; o < 4; o++) {
@@ -100,25 +102,29 @@ theta_gate_kernel(const TI* __restrict__ A, const TI* __restrict__ B, int chil, 
   }
 }
 
-// Generic complex GEMM, 64x64 output tile, 16-deep K slices, 4x4 per thread.
-template <typename C>
+// Generic complex GEMM, T x T output tile (T = 16, 32, 64), 16-deep K slices,
+// T/16 x T/16 outputs per thread, each the same sequence of products whatever T.
+// The 64-wide tile reads its operands least often; a smaller one spreads a
+// small product over the SMs.  FP64 is bound by the two FP64 lanes of an SM at
+// every T, so only the spread counts there (see gemm_tile).
+template <typename C, int T>
 __global__ void __launch_bounds__(256)
 cgemm_kernel(int opA, int opB, int M, int N, int K, C alpha, const C* __restrict__ A, int64_t lda,
              const C* __restrict__ B, int64_t ldb, C beta, C* __restrict__ Cm, int64_t ldc) {
-  constexpr int BM = 64, BN = 64, BK = 16;
+  constexpr int BM = T, BN = T, BK = 16, RT = T / 16;
   __shared__ C As[BK][BM + 1];
   __shared__ C Bs[BK][BN + 1];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-  C acc[4][4];
+  C acc[RT][RT];
 #pragma unroll
-  for (int i = 0; i < 4; i++)
+  for (int i = 0; i < RT; i++)
 #pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j] = czero<C>();
+    for (int j = 0; j < RT; j++) acc[i][j] = czero<C>();
 
   for (int k0 = 0; k0 < K; k0 += BK) {
 #pragma unroll
-    for (int r = 0; r < 4; r++) {
+    for (int r = 0; r < RT; r++) {
       const int idx = threadIdx.x + 256 * r;
       int m, k;
       if (opA == QT_OP_N) { m = idx % BM; k = idx / BM; } else { k = idx % BK; m = idx / BK; }
@@ -131,7 +137,7 @@ cgemm_kernel(int opA, int opB, int M, int N, int K, C alpha, const C* __restrict
       As[k][m] = v;
     }
 #pragma unroll
-    for (int r = 0; r < 4; r++) {
+    for (int r = 0; r < RT; r++) {
       const int idx = threadIdx.x + 256 * r;
       int n, k;
       if (opB == QT_OP_N) { k = idx % BK; n = idx / BK; } else { n = idx % BN; k = idx / BN; }
@@ -146,25 +152,25 @@ cgemm_kernel(int opA, int opB, int M, int N, int K, C alpha, const C* __restrict
     __syncthreads();
 #pragma unroll 4
     for (int k = 0; k < BK; k++) {
-      C a[4], b[4];
+      C a[RT], b[RT];
 #pragma unroll
-      for (int i = 0; i < 4; i++) a[i] = As[k][tx + 16 * i];
+      for (int i = 0; i < RT; i++) a[i] = As[k][tx + 16 * i];
 #pragma unroll
-      for (int j = 0; j < 4; j++) b[j] = Bs[k][ty + 16 * j];
+      for (int j = 0; j < RT; j++) b[j] = Bs[k][ty + 16 * j];
 #pragma unroll
-      for (int i = 0; i < 4; i++)
+      for (int i = 0; i < RT; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) cfma(acc[i][j], a[i], b[j]);
+        for (int j = 0; j < RT; j++) cfma(acc[i][j], a[i], b[j]);
     }
     __syncthreads();
   }
   const bool use_beta = (beta.x != 0 || beta.y != 0);
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
+  for (int i = 0; i < RT; i++) {
     const int m = m0 + tx + 16 * i;
     if (m >= M) continue;
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
+    for (int j = 0; j < RT; j++) {
       const int n = n0 + ty + 16 * j;
       if (n >= N) continue;
       C v = cmul(alpha, acc[i][j]);
@@ -261,20 +267,20 @@ int qt_theta_gate(qt_handle* h, int dtype_in, const void* A, const void* B, int6
   for (int e = 0; e < 16; e++) gp.g[e] = make_double2(G[2 * e], G[2 * e + 1]);
   if (chil <= 0 || chim <= 0 || chir <= 0) return qt_fail(h, QT_EINVAL, "theta: empty bond");
   if (prec == 0) {
-    dim3 grid((unsigned)((chil + 15) / 16), (unsigned)((chir + 15) / 16));
+    dim3 grid((unsigned)((chil + 7) / 8), (unsigned)((chir + 7) / 8));
     if (dtype_in == QT_C128)
-      QT_LAUNCH(h, (theta_gate_kernel<double2, double, double2, 1, 1>), grid, 256, 0, (const double2*)A,
+      QT_LAUNCH(h, (theta_gate_kernel<double2, double, double2, 1, 1, 8>), grid, 64, 0, (const double2*)A,
                 (const double2*)B, (int)chil, (int)chim, (int)chir, gp, (double2*)theta_out);
     else
-      QT_LAUNCH(h, (theta_gate_kernel<float2, double, double2, 1, 1>), grid, 256, 0, (const float2*)A,
+      QT_LAUNCH(h, (theta_gate_kernel<float2, double, double2, 1, 1, 8>), grid, 64, 0, (const float2*)A,
                 (const float2*)B, (int)chil, (int)chim, (int)chir, gp, (double2*)theta_out);
   } else {
     dim3 grid((unsigned)((chil + 31) / 32), (unsigned)((chir + 31) / 32));
     if (dtype_in == QT_C128)
-      QT_LAUNCH(h, (theta_gate_kernel<double2, float, float2, 2, 2>), grid, 256, 0, (const double2*)A,
+      QT_LAUNCH(h, (theta_gate_kernel<double2, float, float2, 2, 2, 16>), grid, 256, 0, (const double2*)A,
                 (const double2*)B, (int)chil, (int)chim, (int)chir, gp, (float2*)theta_out);
     else
-      QT_LAUNCH(h, (theta_gate_kernel<float2, float, float2, 2, 2>), grid, 256, 0, (const float2*)A,
+      QT_LAUNCH(h, (theta_gate_kernel<float2, float, float2, 2, 2, 16>), grid, 256, 0, (const float2*)A,
                 (const float2*)B, (int)chil, (int)chim, (int)chir, gp, (float2*)theta_out);
   }
   return QT_OK;
@@ -287,13 +293,39 @@ int qt_apply_gate_inplace(qt_handle* h, float2* theta, int64_t chil, int64_t chi
   return QT_OK;
 }
 
+// Output tile of an M x N product.  FP64: the tile only sets how many CTAs
+// share the FP64 work, so 16 until 32 gives two CTAs per SM by itself
+// (128 x 128 x 128: 440 us on four CTAs of 64 x 64, 37 us on 64 of 16 x 16).
+// FP32: 64 where the grid covers half the SMs, else 32 where that does, else
+// 16 (the products of a 14-qubit circuit, up to 128 x 128: 7.8 -> 6.1 us on
+// average).
+template <typename C>
+static int gemm_tile(int64_t M, int64_t N) {
+  auto ctas = [&](int t) { return ((M + t - 1) / t) * ((N + t - 1) / t); };
+  if (N > 32 * (int64_t)65535) return 64;  // the grid's second dimension
+  if (sizeof(C) == 16) return ctas(32) >= 2 * 152 ? 32 : 16;
+  return ctas(64) >= 76 ? 64 : ctas(32) >= 76 ? 32 : 16;
+}
+
 template <typename C>
 int qt_cgemm(qt_handle* h, int opA, int opB, int64_t M, int64_t N, int64_t K, C alpha, const C* A, int64_t lda,
              const C* B, int64_t ldb, C beta, C* Cm, int64_t ldc) {
   if (M <= 0 || N <= 0) return QT_OK;
-  dim3 grid((unsigned)((M + 63) / 64), (unsigned)((N + 63) / 64));
-  QT_LAUNCH(h, cgemm_kernel<C>, grid, 256, 0, opA, opB, (int)M, (int)N, (int)K, alpha, A, lda, B, ldb, beta, Cm,
-            ldc);
+  const int t = gemm_tile<C>(M, N);
+  dim3 grid((unsigned)((M + t - 1) / t), (unsigned)((N + t - 1) / t));
+  switch (t) {
+    case 16:
+      QT_LAUNCH(h, (cgemm_kernel<C, 16>), grid, 256, 0, opA, opB, (int)M, (int)N, (int)K, alpha, A, lda, B, ldb, beta,
+                Cm, ldc);
+      break;
+    case 32:
+      QT_LAUNCH(h, (cgemm_kernel<C, 32>), grid, 256, 0, opA, opB, (int)M, (int)N, (int)K, alpha, A, lda, B, ldb, beta,
+                Cm, ldc);
+      break;
+    default:
+      QT_LAUNCH(h, (cgemm_kernel<C, 64>), grid, 256, 0, opA, opB, (int)M, (int)N, (int)K, alpha, A, lda, B, ldb, beta,
+                Cm, ldc);
+  }
   return QT_OK;
 }
 template int qt_cgemm<float2>(qt_handle*, int, int, int64_t, int64_t, int64_t, float2, const float2*, int64_t,

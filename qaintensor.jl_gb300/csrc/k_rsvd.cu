@@ -64,15 +64,30 @@ __global__ void gaussian_kernel(C* __restrict__ out, int64_t rows, int64_t cols,
 // triangle, FP64) with atomics.  Each CTA sums GR rows at a time over a grid-strided
 // set of row tiles; the per-tile partial sums run in the element precision of
 // Y (each entry then carries a relative error of a few u of its own column
-// norms) and are accumulated across tiles and CTAs in FP64.
-constexpr int GR = 16;
+// norms) and are accumulated across tiles and CTAs in FP64.  Thread t owns the
+// upper entries t, t + 256, t + 512 (column by column), so no lane works on
+// the lower triangle.  FP64: bound by the two FP64 lanes of an SM, so tiles of
+// 8 rows, twice the CTAs (128 rows: 23 -> 13 us).
 template <typename C>
-__global__ void __launch_bounds__(256) block_gram_kernel(const C* __restrict__ Y, int64_t m, int b, double2* __restrict__ G) {
+constexpr int gram_rows() { return sizeof(C) == 8 ? 16 : 8; }
+template <typename C>
+__global__ void __launch_bounds__(256) block_gram_kernel(const C* __restrict__ Y, int64_t m, int b, double2* __restrict__ G,
+                                                         const int* __restrict__ skip) {
+  if (skip && *skip) return;
+  constexpr int GR = gram_rows<C>(), NU = BW * (BW + 1) / 2, H = (NU + 255) / 256;
   __shared__ C Ys[GR][BW + 1];
-  // thread t owns entries e = t + 256 h (h = 0..3) of the 32 x 32 Gram: i = e % 32, j = e / 32
-  double2 acc[4];
+  double2 acc[H];
+  int ei[H], ej[H];
 #pragma unroll
-  for (int h = 0; h < 4; h++) acc[h] = make_double2(0, 0);
+  for (int h = 0; h < H; h++) {
+    acc[h] = make_double2(0, 0);
+    const int e = threadIdx.x + 256 * h;  // e = j (j + 1) / 2 + i
+    int j = (int)((sqrtf(8.f * e + 1.f) - 1.f) * 0.5f);
+    while (j * (j + 1) / 2 > e) j--;
+    while ((j + 1) * (j + 2) / 2 <= e) j++;
+    ej[h] = e < NU ? j : BW;
+    ei[h] = e - j * (j + 1) / 2;
+  }
   for (int64_t r0 = (int64_t)blockIdx.x * GR; r0 < m; r0 += (int64_t)gridDim.x * GR) {
     for (int idx = threadIdx.x; idx < GR * BW; idx += 256) {
       const int rr = idx % GR, c = idx / GR;
@@ -82,132 +97,22 @@ __global__ void __launch_bounds__(256) block_gram_kernel(const C* __restrict__ Y
     }
     __syncthreads();
 #pragma unroll
-    for (int h = 0; h < 4; h++) {
-      const int e = threadIdx.x + 256 * h;
-      const int i = e % BW, j = e / BW;
-      if (i <= j && j < b) {
+    for (int h = 0; h < H; h++) {
+      if (ej[h] < b) {
         C s = czero<C>();
 #pragma unroll
-        for (int rr = 0; rr < GR; rr++) cfma_conj(s, Ys[rr][i], Ys[rr][j]);
+        for (int rr = 0; rr < GR; rr++) cfma_conj(s, Ys[rr][ei[h]], Ys[rr][ej[h]]);
         acc[h] = cadd(acc[h], ccast<double2>(s));
       }
     }
     __syncthreads();
   }
 #pragma unroll
-  for (int h = 0; h < 4; h++) {
-    const int e = threadIdx.x + 256 * h;
-    const int i = e % BW, j = e / BW;
-    if (i <= j && j < b) {
-      atomicAdd(&G[i + BW * j].x, acc[h].x);
-      atomicAdd(&G[i + BW * j].y, acc[h].y);
+  for (int h = 0; h < H; h++) {
+    if (ej[h] < b) {
+      atomicAdd(&G[ei[h] + BW * ej[h]].x, acc[h].x);
+      atomicAdd(&G[ei[h] + BW * ej[h]].y, acc[h].y);
     }
-  }
-}
-
-// Cholesky G = R^H R (R upper); R replaces the upper triangle of G (the
-// Gram is accumulated in FP64 either way).  RT is the arithmetic: FP64 for
-// an FP64 basis; FP32 for an FP32 basis, whose shifted first pass adds
-// 11 (m b + b (b+1)) u_fp32 (about 4 % of the trace at m = 2048) and whose
-// later passes see a block orthonormal to a few percent, so FP32 pivots
-// lose nothing the stored basis could keep (GB300 runs FP32 at 64x the FP64
-// rate).  `shift` adds shift * trace(G) to the diagonal first.  A
-// non-positive pivot sets QT_FLAG_CHOL and is replaced by a tiny positive
-// value.  One thread per entry (32 x 32 threads), right-looking: at step k
-// one thread forms the pivot, the pivot row is scaled and the trailing upper
-// triangle updated, in barrier-separated phases.
-template <typename RT>
-__global__ void __launch_bounds__(BW * BW) chol_kernel(double2* __restrict__ G, int b, double shift,
-                                                       int* __restrict__ flags) {
-  typedef typename cplx_of<RT>::type CT;
-  __shared__ CT R[BW][BW + 1];
-  __shared__ CT X[BW][BW + 1];
-  __shared__ RT piv[2], rdiag[BW];
-  __shared__ double tr;
-  const int t = threadIdx.x, i = t / BW, j = t % BW;  // thread t owns entry (i, j)
-  const double2 g = (i < b && j < b && i <= j) ? G[i + BW * j] : make_double2(0, 0);
-  if (t < 32) {
-    double s = (t < b) ? G[t + BW * t].x : 0.0;
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (t == 0) tr = s;
-  }
-  __syncthreads();
-  R[i][j] = ccast<CT>(i == j && i < b ? make_double2(g.x + shift * tr, 0.0) : g);
-  __syncthreads();
-  for (int k = 0; k < b; k++) {
-    // row k: R[k][k] = sqrt(d), R[k][j] /= R[k][k] for j > k.  One thread
-    // forms the pivot.  FP64: 1/sqrt(d) from the single-precision estimate
-    // refined by two Newton steps y <- y (3 - d y^2) / 2 (quadratic
-    // convergence: ~2^-22 -> 2^-44 -> below 2^-52); sqrt(d) = d / sqrt(d).
-    if (t == 0) {
-      RT d = R[k][k].x;
-      if (!(d > (RT)0)) {
-        atomicOr(&flags[QT_FLAG_CHOL], 1);
-        d = (RT)(fabs(tr) * 1e-30 + (sizeof(RT) == 8 ? 1e-300 : 1e-37));
-      }
-      RT y = (RT)rsqrtf((float)d);
-      if (sizeof(RT) == 8) {
-        if (!(y > (RT)0) || isinf(y)) y = (RT)(1.0 / sqrt((double)d));  // d outside the FP32 range
-        y = y * ((RT)1.5 - (RT)0.5 * d * y * y);
-        y = y * ((RT)1.5 - (RT)0.5 * d * y * y);
-      }
-      piv[0] = d * y;
-      piv[1] = y;
-      rdiag[k] = y;
-    }
-    __syncthreads();
-    if (i == k && j == k) R[k][k] = mk(piv[0], (RT)0);
-    if (i == k && j > k && j < b) R[k][j] = cscale(R[k][j], piv[1]);
-    __syncthreads();
-    // trailing update: R[i][j] -= conj(R[k][i]) R[k][j], k < i <= j
-    if (i > k && j >= i && j < b) R[i][j] = csub(R[i][j], cmul(cconj(R[k][i]), R[k][j]));
-    __syncthreads();
-  }
-  // X = R^{-1} (upper) by column sweeps of R X = I, one entry per thread:
-  // for k = b-1 .. 0, row k of X is final once scaled by 1 / R[k][k], and
-  // its multiples R[r][k] X[k][:] are removed from the rows r < k.
-  X[i][j] = mk((RT)(i == j && i < b ? 1 : 0), (RT)0);
-  __syncthreads();
-  for (int k = b - 1; k >= 0; k--) {
-    if (i == k) X[k][j] = cscale(X[k][j], rdiag[k]);
-    __syncthreads();
-    if (i < k) X[i][j] = csub(X[i][j], cmul(R[i][k], X[k][j]));
-    __syncthreads();
-  }
-  G[i + BW * j] = (i <= j) ? ccast<double2>(R[i][j]) : make_double2(0, 0);
-  G[BW * BW + i + BW * j] = ccast<double2>(X[i][j]);
-}
-
-// Yb <- Yb R^{-1} with the explicit inverse X = R^{-1} (upper triangular,
-// formed by chol_kernel): 16 rows per CTA, thread (row t >> 4, columns
-// 2 (t & 15) and + 1), out_j = sum_{k <= j} y_k X[k][j] in the element
-// precision of Y.  The block's rows are read into shared memory before any
-// is written.
-template <typename C>
-__global__ void __launch_bounds__(256) apply_rinv_kernel(C* __restrict__ Y, int64_t m, int b,
-                                                         const double2* __restrict__ Xinv) {
-  __shared__ C Xs[BW][BW + 1];
-  __shared__ C Ys[16][BW + 1];
-  const int t = threadIdx.x, rl = t >> 4, jp = t & 15;
-  const int64_t r0 = (int64_t)blockIdx.x * 16;
-  for (int e = t; e < BW * BW; e += 256) Xs[e % BW][e / BW] = ccast<C>(Xinv[e]);
-  for (int e = t; e < 16 * BW; e += 256) {
-    const int rr = e % 16, c = e / 16;
-    Ys[rr][c] = (r0 + rr < m && c < b) ? Y[r0 + rr + m * (int64_t)c] : czero<C>();
-  }
-  __syncthreads();
-  const int j0 = 2 * jp, j1 = 2 * jp + 1;
-  C a0 = czero<C>(), a1 = czero<C>();
-#pragma unroll 8
-  for (int k = 0; k < BW; k++) {
-    const C y = Ys[rl][k];
-    if (k <= j0) cfma(a0, y, Xs[k][j0]);
-    if (k <= j1) cfma(a1, y, Xs[k][j1]);
-  }
-  const int64_t r = r0 + rl;
-  if (r < m) {
-    if (j0 < b) Y[r + m * (int64_t)j0] = a0;
-    if (j1 < b) Y[r + m * (int64_t)j1] = a1;
   }
 }
 
@@ -249,9 +154,22 @@ __host__ __device__ constexpr size_t cq_smem_bytes(int nrb) {
          BW * sizeof(double) + BW * sizeof(float) + 16;
 }
 
+// acc -= conj(a) * b and acc -= a * b, four fused products each
+template <typename C>
+__device__ inline void cfms_conj(C& acc, C a, C b) {
+  acc.x = fma(-a.x, b.x, acc.x); acc.x = fma(-a.y, b.y, acc.x);
+  acc.y = fma(-a.x, b.y, acc.y); acc.y = fma(a.y, b.x, acc.y);
+}
+template <typename C>
+__device__ inline void cfms(C& acc, C a, C b) {
+  acc.x = fma(-a.x, b.x, acc.x); acc.x = fma(a.y, b.y, acc.x);
+  acc.y = fma(-a.x, b.y, acc.y); acc.y = fma(-a.y, b.x, acc.y);
+}
+
 // Step (E) of a CholeskyQR pass, called by all 256 threads of the CTA.
-// From the FP32 Gram in the upper triangle of Gl (row stride CQ_RS) and its
-// FP64 diagonal Gd: R = chol(G + shift trace(G) I) in place of the Gram's
+// (FP32 in the cluster and one-launch kernels; chol_kernel runs it in either
+// precision).  From the Gram in the upper triangle of Gl (row stride CQ_RS) and
+// its FP64 diagonal Gd: R = chol(G + shift trace(G) I) in place of the Gram's
 // upper triangle, then X = R^{-1}, both blocked by 8 columns.  Cholesky: for
 // each diagonal block, warp 0 runs its 8 pivot steps on the block's rows
 // of every column to the right (lane l: column k0 + l, an 8-row register
@@ -264,51 +182,61 @@ __host__ __device__ constexpr size_t cq_smem_bytes(int nrb) {
 // Ry receives 1 / R[k][k] (and the tiny pivot at Ry[BW]), Xs = R^{-1}
 // (BW x BW, row-major), Tb is 256 entries of scratch.  `report` marks the
 // one CTA that raises QT_FLAG_CHOL for a non-positive pivot.
-__device__ void cq_factor(float2* __restrict__ Gl, const double* __restrict__ Gd, float* __restrict__ Ry,
-                          float2* __restrict__ Xs, float2* __restrict__ Tb, int b, double shift,
-                          int* __restrict__ flags, bool report) {
+template <typename C>
+__device__ void cq_factor(C* __restrict__ Gl, const double* __restrict__ Gd, typename real_of<C>::type* __restrict__ Ry,
+                          C* __restrict__ Xs, C* __restrict__ Tb, int b, double shift, int* __restrict__ flags,
+                          bool report) {
+  typedef typename real_of<C>::type R;
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-  float* trs = (float*)(Ry + BW);
+  R* trs = Ry + BW;
   if (w == 0) {
     double tr = lane < b ? Gd[lane] : 0.0;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) tr += __shfl_xor_sync(0xffffffffu, tr, o);
-    if (lane < b) Gl[lane * CQ_RS + lane] = make_float2((float)(Gd[lane] + shift * tr), 0.f);
-    Ry[lane] = 0.f;
-    if (lane == 0) trs[0] = (float)(fabs(tr) * 1e-30 + 1e-37);
+    if (lane < b) Gl[lane * CQ_RS + lane] = mk((R)(Gd[lane] + shift * tr), (R)0);
+    Ry[lane] = 0;
+    if (lane == 0) trs[0] = (R)(fabs(tr) * 1e-30 + (sizeof(R) == 8 ? 1e-300 : 1e-37));
   }
   __syncthreads();
   for (int k0 = 0; k0 < b; k0 += 8) {
     if (w == 0) {
       const int col = k0 + lane;
-      float2 c[8];
+      C c[8];
 #pragma unroll
       for (int r = 0; r < 8; r++)
-        c[r] = (col < BW && k0 + r <= col) ? Gl[(k0 + r) * CQ_RS + col] : make_float2(0.f, 0.f);
+        c[r] = (col < BW && k0 + r <= col) ? Gl[(k0 + r) * CQ_RS + col] : czero<C>();
       // dn: the next pivot as seen by its own lane (lane kk + 1 holds
       // R[k][k + 1] itself), so the pivot chain needs no row shuffle
-      float dn = c[0].x;
+      R dn = c[0].x;
 #pragma unroll
       for (int kk = 0; kk < 8; kk++) {
         const int k = k0 + kk;
         if (k < b) {
-          float d = __shfl_sync(0xffffffffu, dn, kk);
-          if (!(d > 0.f)) {
+          R d = __shfl_sync(0xffffffffu, dn, kk);
+          if (!(d > 0)) {
             if (lane == 0 && report) atomicOr(&flags[QT_FLAG_CHOL], 1);
             d = trs[0];
           }
-          const float y = rsqrtf(d);
-          const float2 rk =
-              lane == kk ? make_float2(d * y, 0.f) : (lane > kk ? cscale(c[0], y) : make_float2(0.f, 0.f));
+          // FP64: the FP32 estimate and two Newton steps y <- y (3 - d y^2) / 2
+          // (2^-22 -> 2^-44 -> below 2^-52)
+          R y = (R)rsqrtf((float)d);
+          if (sizeof(R) == 8) {
+            if (!(y > 0) || isinf(y)) y = (R)(1.0 / sqrt((double)d));  // d outside the FP32 range
+            y = y * ((R)1.5 - (R)0.5 * d * y * y);
+            y = y * ((R)1.5 - (R)0.5 * d * y * y);
+          }
+          const C rk =
+              lane == kk ? mk(d * y, (R)0) : (lane > kk ? cscale(c[0], y) : czero<C>());
           dn = c[1].x - (rk.x * rk.x + rk.y * rk.y);
           if (col < BW) Gl[k * CQ_RS + col] = rk;  // row k of R (zeros left of the diagonal)
           if (lane == 0) Ry[k] = y;
 #pragma unroll
           for (int r = 1; r < 8; r++) {
-            float2 rkr;  // R[k][k + r] from lane kk + r (slots past the block are discarded)
+            C rkr;  // R[k][k + r] from lane kk + r (slots past the block are discarded)
             rkr.x = __shfl_sync(0xffffffffu, rk.x, min(kk + r, 31));
             rkr.y = __shfl_sync(0xffffffffu, rk.y, min(kk + r, 31));
-            c[r - 1] = csub(c[r], cmul(cconj(rkr), rk));
+            c[r - 1] = c[r];
+            cfms_conj(c[r - 1], rkr, rk);
           }
         }
       }
@@ -318,11 +246,11 @@ __device__ void cq_factor(float2* __restrict__ Gl, const double* __restrict__ Gd
     // lane j column j (two partial sums)
     for (int i = k0 + 8 + w; i < BW; i += 8) {
       if (lane >= i) {
-        float2 v0 = Gl[i * CQ_RS + lane], v1 = make_float2(0.f, 0.f);
+        C v0 = Gl[i * CQ_RS + lane], v1 = czero<C>();
 #pragma unroll
         for (int q = 0; q < 8; q += 2) {
-          v0 = csub(v0, cmul(cconj(Gl[(k0 + q) * CQ_RS + i]), Gl[(k0 + q) * CQ_RS + lane]));
-          v1 = csub(v1, cmul(cconj(Gl[(k0 + q + 1) * CQ_RS + i]), Gl[(k0 + q + 1) * CQ_RS + lane]));
+          cfms_conj(v0, Gl[(k0 + q) * CQ_RS + i], Gl[(k0 + q) * CQ_RS + lane]);
+          cfms_conj(v1, Gl[(k0 + q + 1) * CQ_RS + i], Gl[(k0 + q + 1) * CQ_RS + lane]);
         }
         Gl[i * CQ_RS + lane] = cadd(v0, v1);
       }
@@ -332,37 +260,130 @@ __device__ void cq_factor(float2* __restrict__ Gl, const double* __restrict__ Gd
   // diagonal blocks of X; the blocks below the diagonal are zero
   if (w < 4 && lane < 8) {
     const int k0 = 8 * w;
-    float2 x[8];
+    C x[8];
 #pragma unroll
-    for (int r = 0; r < 8; r++) x[r] = make_float2(r == lane ? 1.f : 0.f, 0.f);
+    for (int r = 0; r < 8; r++) x[r] = mk((R)(r == lane ? 1 : 0), (R)0);
 #pragma unroll
     for (int kk = 7; kk >= 0; kk--) {
       x[kk] = cscale(x[kk], Ry[k0 + kk]);
 #pragma unroll
-      for (int i = 0; i < kk; i++) x[i] = csub(x[i], cmul(Gl[(k0 + i) * CQ_RS + k0 + kk], x[kk]));
+      for (int i = 0; i < kk; i++) cfms(x[i], Gl[(k0 + i) * CQ_RS + k0 + kk], x[kk]);
     }
 #pragma unroll
     for (int r = 0; r < 8; r++) Xs[(k0 + r) * BW + k0 + lane] = x[r];
   }
   for (int e = t; e < BW * BW; e += 256)
-    if ((e / BW) / 8 > (e % BW) / 8) Xs[e] = make_float2(0.f, 0.f);
+    if ((e / BW) / 8 > (e % BW) / 8) Xs[e] = czero<C>();
   __syncthreads();
   for (int d = 1; d < 4; d++) {
     const int bi = t / 64, a = (t / 8) % 8, cc = t % 8, bj = bi + d, i = 8 * bi + a, j = 8 * bj + cc;
     if (bj < 4) {
-      float2 v = make_float2(0.f, 0.f);
+      C v = czero<C>();
       for (int l = 8 * (bi + 1); l < 8 * (bj + 1); l++) cfma(v, Gl[i * CQ_RS + l], Xs[l * BW + j]);
       Tb[t] = v;
     }
     __syncthreads();
     if (bj < 4) {
-      float2 v = make_float2(0.f, 0.f);
+      C v = czero<C>();
 #pragma unroll
       for (int q = 0; q < 8; q++) cfma(v, Xs[i * BW + 8 * bi + q], Tb[64 * bi + 8 * q + cc]);
-      Xs[i * BW + j] = make_float2(-v.x, -v.y);
+      Xs[i * BW + j] = mk(-v.x, -v.y);
     }
     __syncthreads();
   }
+}
+
+// State of a block's passes on the device: `done`: the pass (> 0) that left the
+// block orthonormal to rounding, so that the next has nothing to do; `full`:
+// Xinv is not upper triangular.
+struct cq_state { int done, full; };
+// Largest |G - I| that the series below takes: its remainder 5/16 E^3 is then
+// under 1e-16 for a 32 x 32 E of such entries.
+constexpr double CQ_SERIES = 2e-7;
+
+// X with X^H G X = I for the Gram that block_gram_kernel summed; row-major to
+// Xinv.  One CTA.  From G + shift trace(G) I: X = R^{-1}, R the Cholesky factor,
+// in the arithmetic of C.  An FP64 pass without shift mostly meets a G that is
+// the identity to rounding (the pass before it orthonormalised a block of
+// condition up to 1e4): then X = I - E/2 + 3/8 E^2, E = G - I, which needs no
+// FP64 products (E^2 is below 1e-13, and FP32 gives it to 1e-20), and the
+// pass after it is skipped.  FP64: 90 us for the factor -- the FP64
+// instructions of one SM, 16 cycles each -- where one thread per entry and
+// three block barriers per pivot took 117; the series takes under 10.
+template <typename C>
+__global__ void __launch_bounds__(256) chol_kernel(const double2* __restrict__ G, int b, double shift, int pass,
+                                                   C* __restrict__ Xinv, cq_state* __restrict__ st,
+                                                   int* __restrict__ flags) {
+  __shared__ C Gl[BW * CQ_RS], Xs[BW * BW], Tb[256];
+  __shared__ double Gd[BW];
+  __shared__ typename real_of<C>::type Ry[BW + 1];
+  const int t = threadIdx.x;
+  if (pass > 1 && st->done && st->done < pass) return;
+  if constexpr (sizeof(C) == 16) {
+    if (pass > 0) {
+      float2* E = reinterpret_cast<float2*>(Gl);  // the whole Hermitian E, row stride CQ_RS
+      int big = 0;
+      for (int e = t; e < BW * BW; e += 256) {
+        const int i = e % BW, j = e / BW;
+        double2 v = i > j ? cconj(G[j + BW * i]) : G[e];
+        if (i == j) v.x -= 1.0;
+        if (i >= b || j >= b) v = make_double2(0, 0);
+        if (!(fabs(v.x) <= CQ_SERIES && fabs(v.y) <= CQ_SERIES)) big = 1;
+        E[i * CQ_RS + j] = make_float2((float)v.x, (float)v.y);
+        Xs[i * BW + j] = make_double2((i == j && i < b ? 1.0 : 0.0) - 0.5 * v.x, -0.5 * v.y);
+      }
+      if (!__syncthreads_or(big)) {
+        for (int e = t; e < BW * BW; e += 256) {
+          const int i = e / BW, j = e % BW;
+          float2 a = make_float2(0.f, 0.f);
+#pragma unroll 8
+          for (int k = 0; k < BW; k++) cfma(a, E[i * CQ_RS + k], E[k * CQ_RS + j]);
+          const double2 x = Xs[e];
+          Xinv[e] = mk(x.x + 0.375 * (double)a.x, x.y + 0.375 * (double)a.y);
+        }
+        if (t == 0) { st->done = pass; st->full = 1; }
+        return;
+      }
+    }
+  }
+  for (int e = t; e < BW * BW; e += 256) {
+    const int i = e % BW, j = e / BW;
+    const double2 v = i <= j && j < b ? G[e] : make_double2(0, 0);
+    if (i <= j) Gl[i * CQ_RS + j] = ccast<C>(v);
+    if (i == j) Gd[i] = v.x;
+  }
+  __syncthreads();
+  cq_factor<C>(Gl, Gd, Ry, Xs, Tb, b, shift, flags, true);
+  for (int e = t; e < BW * BW; e += 256) Xinv[e] = Xs[e];
+  if (t == 0) { st->done = 0; st->full = 0; }
+}
+
+// Yb <- Yb X with chol_kernel's X, out_j = sum_k y_k X[k][j] in the element
+// precision of Y.  8 rows per CTA; warp w the columns 4 w .. 4 w + 3, lane
+// (row, column), so that a warp stops at its last column's k where X is upper
+// triangular (half the products of lanes across the columns; 128 rows in FP64:
+// 22 -> 15 us).  The block's rows are read into shared memory before any is
+// written.
+constexpr int AR = 8;
+template <typename C>
+__global__ void __launch_bounds__(256) apply_rinv_kernel(C* __restrict__ Y, int64_t m, int b, int pass,
+                                                         const C* __restrict__ Xinv, const cq_state* __restrict__ st) {
+  __shared__ C Xs[BW][BW + 1];
+  __shared__ C Ys[AR][BW + 1];
+  const int t = threadIdx.x, w = t >> 5, rl = t & 7, j = 4 * w + ((t >> 3) & 3);
+  if (pass > 1 && st->done && st->done < pass) return;
+  const int64_t r0 = (int64_t)blockIdx.x * AR;
+  for (int e = t; e < BW * BW; e += 256) Xs[e / BW][e % BW] = Xinv[e];
+  {
+    const int rr = t % AR, c = t / AR;
+    Ys[rr][c] = (r0 + rr < m && c < b) ? Y[r0 + rr + m * (int64_t)c] : czero<C>();
+  }
+  __syncthreads();
+  const int kn = st->full ? BW : 4 * w + 4;
+  C a = czero<C>();
+#pragma unroll 4
+  for (int k = 0; k < kn; k++) cfma(a, Ys[rl][k], Xs[k][j]);
+  if (r0 + rl < m && j < b) Y[r0 + rl + m * (int64_t)j] = a;
 }
 
 // CholeskyQR passes of one FP32 block (m x b, b <= 32) in one launch: a
@@ -501,7 +522,7 @@ __global__ void __launch_bounds__(256, 1) cholqr_cluster_kernel(float2* __restri
     __syncthreads();
     phase(5);  // gather
     // (E) R = chol(G + shift trace(G) I) and X = R^{-1}, the same in every CTA
-    cq_factor(Gl, Gd, Ry, Xs, (float2*)Gt, b, p == 0 ? shift0 : 0.0, flags, crank == 0);
+    cq_factor<float2>(Gl, Gd, Ry, Xs, (float2*)Gt, b, p == 0 ? shift0 : 0.0, flags, crank == 0);
     phase(6);  // Cholesky + inverse
     // (F) rows <- rows X: warp w owns columns 4 cg .. 4 cg + 3 (warps w and
     // w + 4 share a scheduler and take column groups w and 7 - w, which
@@ -645,23 +666,27 @@ int block_cholqr_cluster(qt_handle* h, float2* Yb, int64_t m, int b, int nrb, in
 // proj_coef_kernel owns one chunk and 128 of the j0 columns (4 x 4 entries
 // per thread, rows staged 32 (FP64: 16) at a time, the next stage loaded
 // into registers meanwhile) and writes its partial; the chunks are added in
-// chunk order by coef_reduce_kernel (reproducible, no atomics).
-constexpr int PJ_ROWS = 64;   // rows per coefficient chunk
-constexpr int PJ_K = 128;     // previous columns per coefficient CTA
-constexpr int PJ_R = 16;      // rows per CTA of the update
+// chunk order by coef_reduce_kernel (reproducible, no atomics).  FP64, where a
+// CTA is bound by the SM's two FP64 lanes, takes 32 columns and, up to 512
+// rows, chunks of 16 rows (128 x 128: 260 us a launch on two CTAs before, 22 us).
+template <typename C>
+constexpr int pj_k() { return sizeof(C) == 8 ? 128 : 32; }  // previous columns per coefficient CTA
+template <typename C>
+constexpr int pj_rows(int64_t m) { return sizeof(C) == 16 && m <= 512 ? 16 : 64; }  // rows per coefficient chunk
 template <typename C>
 __global__ void __launch_bounds__(256) proj_coef_kernel(const C* __restrict__ Y, int64_t m, int j0,
-                                                        const C* __restrict__ Yb, int b, C* __restrict__ part) {
+                                                        const C* __restrict__ Yb, int b, int rows, C* __restrict__ part) {
+  constexpr int PJ_K = pj_k<C>(), NA = PJ_K / 32;
   constexpr int SR = sizeof(C) == 8 ? 32 : 16;  // rows staged at a time (static shared memory <= 48 KB)
   constexpr int NY = SR * PJ_K / 256, NB = SR * BW / 256;
   __shared__ C Ys[SR][PJ_K + 1];
   __shared__ C Bs[SR][BW + 1];
-  const int t = threadIdx.x, kq = t & 31, jq = t >> 5;  // entries k = 4 kq + a, j = 4 jq + c
-  const int64_t r_begin = (int64_t)blockIdx.x * PJ_ROWS, r_end = min(m, r_begin + (int64_t)PJ_ROWS);
+  const int t = threadIdx.x, kq = t & 31, jq = t >> 5;  // entries k = NA kq + a, j = 4 jq + c
+  const int64_t r_begin = (int64_t)blockIdx.x * rows, r_end = min(m, r_begin + rows);
   const int k0 = blockIdx.y * PJ_K;
-  C acc[4][4];
+  C acc[NA][4];
 #pragma unroll
-  for (int a = 0; a < 4; a++)
+  for (int a = 0; a < NA; a++)
 #pragma unroll
     for (int c = 0; c < 4; c++) acc[a][c] = czero<C>();
   // the next stage's values wait in registers while the current one is used
@@ -690,13 +715,13 @@ __global__ void __launch_bounds__(256) proj_coef_kernel(const C* __restrict__ Y,
     if (r0 + SR < r_end) fetch(r0 + SR);
 #pragma unroll 4
     for (int rr = 0; rr < SR; rr++) {
-      C y[4], z[4];
+      C y[NA], z[4];
 #pragma unroll
-      for (int a = 0; a < 4; a++) y[a] = Ys[rr][4 * kq + a];
+      for (int a = 0; a < NA; a++) y[a] = Ys[rr][NA * kq + a];
 #pragma unroll
       for (int c = 0; c < 4; c++) z[c] = Bs[rr][4 * jq + c];
 #pragma unroll
-      for (int a = 0; a < 4; a++)
+      for (int a = 0; a < NA; a++)
 #pragma unroll
         for (int c = 0; c < 4; c++) cfma_conj(acc[a][c], y[a], z[c]);
     }
@@ -705,10 +730,10 @@ __global__ void __launch_bounds__(256) proj_coef_kernel(const C* __restrict__ Y,
   // part[chunk][k][j], k over the padded j0
   const int jp = gridDim.y * PJ_K;
 #pragma unroll
-  for (int a = 0; a < 4; a++)
+  for (int a = 0; a < NA; a++)
 #pragma unroll
     for (int c = 0; c < 4; c++)
-      part[((size_t)blockIdx.x * jp + k0 + 4 * kq + a) * BW + 4 * jq + c] = acc[a][c];
+      part[((size_t)blockIdx.x * jp + k0 + NA * kq + a) * BW + 4 * jq + c] = acc[a][c];
 }
 
 template <typename C>
@@ -720,16 +745,21 @@ __global__ void coef_reduce_kernel(const C* __restrict__ part, int nchunk, int j
   coef[e] = v;
 }
 
-// Yb[r][j] -= sum_k Y[r][k] coef[k][j]: PJ_R rows per CTA, thread (row t >> 4,
-// columns 2 (t & 15), + 1), previous columns staged KT at a time.
+// Yb[r][j] -= sum_k Y[r][k] coef[k][j]: 16 rows per CTA, thread (row t >> 4,
+// columns 2 (t & 15), + 1), previous columns staged KT at a time.  FP64: 4 rows
+// per CTA, thread (row, column, half of the previous columns), the halves added
+// at the end -- a quarter of the FP64 work per CTA, four times the CTAs.
+template <typename C>
+constexpr int pj_r() { return sizeof(C) == 8 ? 16 : 4; }
 template <typename C>
 __global__ void __launch_bounds__(256) proj_apply_kernel(const C* __restrict__ Y, int64_t m, int j0,
                                                          const C* __restrict__ coef, C* __restrict__ Yb, int b) {
-  constexpr int KT = sizeof(C) == 8 ? 64 : 32;  // static shared memory <= 48 KB
-  constexpr int NC = KT * BW / 256, NY = PJ_R * KT / 256;
+  constexpr bool F64 = sizeof(C) == 16;
+  constexpr int PJ_R = pj_r<C>(), KT = F64 ? 32 : 64;  // static shared memory <= 48 KB
+  constexpr int NC = KT * BW / 256, NY = PJ_R * KT >= 256 ? PJ_R * KT / 256 : 1;
   __shared__ __align__(16) C Cs[KT][BW];
   __shared__ C Ys[PJ_R][KT + 1];
-  const int t = threadIdx.x, rl = t >> 4, jp = t & 15;
+  const int t = threadIdx.x, rl = F64 ? (t >> 5) & 3 : t >> 4, jp = t & 15, half = t >> 7, j1 = t & 31;
   const int64_t r = (int64_t)blockIdx.x * PJ_R + rl;
   C a0 = czero<C>(), a1 = czero<C>();
   // the next tile waits in registers while the current one is used
@@ -744,7 +774,7 @@ __global__ void __launch_bounds__(256) proj_apply_kernel(const C* __restrict__ Y
     for (int u = 0; u < NY; u++) {
       const int e = t + 256 * u, rr = e % PJ_R, kk = e / PJ_R;
       const int64_t gr = (int64_t)blockIdx.x * PJ_R + rr;
-      py[u] = (gr < m && k0 + kk < j0) ? Y[gr + m * (int64_t)(k0 + kk)] : czero<C>();
+      py[u] = (kk < KT && gr < m && k0 + kk < j0) ? Y[gr + m * (int64_t)(k0 + kk)] : czero<C>();
     }
   };
   fetch(0);
@@ -752,16 +782,28 @@ __global__ void __launch_bounds__(256) proj_apply_kernel(const C* __restrict__ Y
 #pragma unroll
     for (int u = 0; u < NC; u++) { const int e = t + 256 * u; Cs[e / BW][e % BW] = pc[u]; }
 #pragma unroll
-    for (int u = 0; u < NY; u++) { const int e = t + 256 * u; Ys[e % PJ_R][e / PJ_R] = py[u]; }
+    for (int u = 0; u < NY; u++) { const int e = t + 256 * u; if (e < PJ_R * KT) Ys[e % PJ_R][e / PJ_R] = py[u]; }
     __syncthreads();
     if (k0 + KT < j0) fetch(k0 + KT);
+    if constexpr (F64) {
 #pragma unroll 8
-    for (int kk = 0; kk < KT; kk++) {
-      const C y = Ys[rl][kk];
-      cfma(a0, y, Cs[kk][2 * jp]);
-      cfma(a1, y, Cs[kk][2 * jp + 1]);
+      for (int kk = half * (KT / 2); kk < (half + 1) * (KT / 2); kk++) cfma(a0, Ys[rl][kk], Cs[kk][j1]);
+    } else {
+#pragma unroll 8
+      for (int kk = 0; kk < KT; kk++) {
+        const C y = Ys[rl][kk];
+        cfma(a0, y, Cs[kk][2 * jp]);
+        cfma(a1, y, Cs[kk][2 * jp + 1]);
+      }
     }
     __syncthreads();
+  }
+  if constexpr (F64) {
+    if (half) Cs[rl][j1] = a0;
+    __syncthreads();
+    if (!half && r < m && j1 < b)
+      Yb[r + m * (int64_t)j1] = csub(Yb[r + m * (int64_t)j1], cadd(a0, Cs[rl][j1]));
+    return;
   }
   if (r < m) {
     if (2 * jp < b) Yb[r + m * (int64_t)(2 * jp)] = csub(Yb[r + m * (int64_t)(2 * jp)], a0);
@@ -771,26 +813,32 @@ __global__ void __launch_bounds__(256) proj_apply_kernel(const C* __restrict__ Y
 
 template <typename C>
 int block_project(qt_handle* h, const C* Y, int64_t m, int j0, C* Yb, int b, C* part, C* coef) {
-  const int nchunk = (int)((m + PJ_ROWS - 1) / PJ_ROWS), nk = (j0 + PJ_K - 1) / PJ_K;
-  QT_LAUNCH(h, proj_coef_kernel<C>, dim3(nchunk, nk), 256, 0, Y, m, j0, Yb, b, part);
-  QT_LAUNCH(h, coef_reduce_kernel<C>, (unsigned)((j0 * BW + 255) / 256), 256, 0, (const C*)part, nchunk, nk * PJ_K,
-            j0, coef);
-  QT_LAUNCH(h, proj_apply_kernel<C>, (unsigned)((m + PJ_R - 1) / PJ_R), 256, 0, Y, m, j0, (const C*)coef, Yb, b);
+  const int rows = pj_rows<C>(m), nchunk = (int)((m + rows - 1) / rows), nk = (j0 + pj_k<C>() - 1) / pj_k<C>();
+  QT_LAUNCH(h, proj_coef_kernel<C>, dim3(nchunk, nk), 256, 0, Y, m, j0, Yb, b, rows, part);
+  QT_LAUNCH(h, coef_reduce_kernel<C>, (unsigned)((j0 * BW + 255) / 256), 256, 0, (const C*)part, nchunk,
+            nk * pj_k<C>(), j0, coef);
+  QT_LAUNCH(h, proj_apply_kernel<C>, (unsigned)((m + pj_r<C>() - 1) / pj_r<C>()), 256, 0, Y, m, j0, (const C*)coef,
+            Yb, b);
   return QT_OK;
 }
 
+// CholeskyQR pass `pass` (0: shifted) of a block.  dG: the Gram (BW x BW
+// double2), X (BW x BW of C), the state of the block's passes.  Pass 2 of an
+// FP64 block finds on the device whether pass 1 left it anything to do.
 template <typename C>
-int block_cholqr(qt_handle* h, C* Yb, int64_t m, int b, bool shifted, double2* dG) {
-  QT_CHECK_CUDA(h, cudaMemsetAsync(dG, 0, sizeof(double2) * BW * BW, h->stream));  // the Gram; chol writes R, R^{-1}
-  const unsigned gg = (unsigned)std::min<int64_t>((m + GR - 1) / GR, 2 * 152);
-  QT_LAUNCH(h, block_gram_kernel<C>, gg, 256, 0, Yb, m, b, dG);
+int block_cholqr(qt_handle* h, C* Yb, int64_t m, int b, int pass, double2* dG) {
+  QT_CHECK_CUDA(h, cudaMemsetAsync(dG, 0, sizeof(double2) * BW * BW, h->stream));
+  C* Xinv = reinterpret_cast<C*>(dG + BW * BW);
+  cq_state* st = reinterpret_cast<cq_state*>(dG + 2 * BW * BW);
+  const unsigned gg = (unsigned)std::min<int64_t>((m + gram_rows<C>() - 1) / gram_rows<C>(), 2 * 152);
+  QT_LAUNCH(h, block_gram_kernel<C>, gg, 256, 0, Yb, m, b, dG, pass > 1 ? (const int*)&st->done : nullptr);
   // shift of shifted CholeskyQR3, sized by the unit roundoff of the stored
-  // basis (the Gram and the Cholesky run in FP64, but Y R^{-1} is formed and
-  // stored in the element type of Y)
+  // basis (Y R^{-1} is formed and stored in the element type of Y)
   const double u = (sizeof(typename real_of<C>::type) == 8) ? 1.11e-16 : 5.96e-8;
-  const double shift = shifted ? 11.0 * ((double)m * b + (double)b * (b + 1)) * u : 0.0;
-  QT_LAUNCH(h, chol_kernel<typename real_of<C>::type>, 1, BW * BW, 0, dG, b, shift, h->d_flags);
-  QT_LAUNCH(h, apply_rinv_kernel<C>, (unsigned)((m + 15) / 16), 256, 0, Yb, m, b, (const double2*)dG + BW * BW);
+  const double shift = pass == 0 ? 11.0 * ((double)m * b + (double)b * (b + 1)) * u : 0.0;
+  QT_LAUNCH(h, chol_kernel<C>, 1, 256, 0, (const double2*)dG, b, shift, pass, Xinv, st, h->d_flags);
+  QT_LAUNCH(h, apply_rinv_kernel<C>, (unsigned)((m + AR - 1) / AR), 256, 0, Yb, m, b, pass,
+            (const C*)Xinv, (const cq_state*)st);
   return QT_OK;
 }
 
@@ -1112,7 +1160,7 @@ __device__ bool op_cholqr(const OrthArgs& a, float2* Ys, float2* Gl, float2* Xs,
   }
   __syncthreads();
   op_mark(a, 6);  // Gram gather
-  cq_factor(Gl, Gd, Ry, Xs, Tb, b, shift, a.flags, c == 0);
+  cq_factor<float2>(Gl, Gd, Ry, Xs, Tb, b, shift, a.flags, c == 0);
   op_mark(a, 7);  // Cholesky + inverse
   {
     const int r = t >> 4, jc = 2 * (t & 15);
@@ -1330,8 +1378,8 @@ int qt_orthonormalize(qt_handle* h, C* Y, int64_t m, int64_t l, int use) {
   qt_scratch s(h);
   double2* dG;
   C *coef, *part;
-  const int64_t nchunk = (m + PJ_ROWS - 1) / PJ_ROWS, lpad = (l + PJ_K - 1) / PJ_K * PJ_K;
-  QT_TRY(s.get(&dG, 2 * BW * BW));
+  const int64_t nchunk = (m + pj_rows<C>(m) - 1) / pj_rows<C>(m), lpad = (l + pj_k<C>() - 1) / pj_k<C>() * pj_k<C>();
+  QT_TRY(s.get(&dG, 2 * BW * BW + 1));
   QT_TRY(s.get(&coef, (size_t)l * BW));
   QT_TRY(s.get(&part, (size_t)nchunk * lpad * BW));
   int nrb = 0, cs = 0;
@@ -1371,13 +1419,13 @@ int qt_orthonormalize(qt_handle* h, C* Y, int64_t m, int64_t l, int use) {
     }
     for (int pass = 0; pass < 2; pass++) {
       if (j0 > 0) QT_TRY(block_project<C>(h, Y, m, (int)j0, Yb, b, part, coef));
-      QT_TRY(block_cholqr<C>(h, Yb, m, b, pass == 0, dG));
+      QT_TRY(block_cholqr<C>(h, Yb, m, b, pass, dG));
     }
     // one more CholeskyQR (shifted CholeskyQR3): after a shifted pass the
     // block is only well conditioned, not orthonormal, and the next pass
     // leaves cond^2 u of that -- with the FP64 shift 5e-7 to 6e-3 for blocks
     // of 7 to 31 columns whose norms fall over 14 decades
-    QT_TRY(block_cholqr<C>(h, Yb, m, b, false, dG));
+    QT_TRY(block_cholqr<C>(h, Yb, m, b, 2, dG));
   }
   if (phase_ns && cq_launches > 0) {
     unsigned long long hp[8];
