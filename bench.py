@@ -419,7 +419,7 @@ def roofline(prof, work, n_prof, sm_mhz=2070.0):
     peaks, src = load_peaks()
     name, launches, ms = prof[0]
     per_launch_s = ms / 1e3 / launches
-    fp32_kernels = ("pair_round_kernel", "jacobi_sweep32_kernel", "(gram_kernel", "pair_eig32_kernel",
+    fp32_kernels = ("pair_round_kernel", "jacobi_sweep32_kernel", "jacobi_ring32_kernel", "(gram_kernel", "pair_eig32_kernel",
                     "apply_kernel", "pair_apply32_kernel")
     if name.startswith(fp32_kernels):
         if work["jacobi_rounds"] <= 0:
@@ -427,6 +427,10 @@ def roofline(prof, work, n_prof, sm_mhz=2070.0):
         fma = 8.0 * work["jacobi_rot_bytes"] + 4.25 * work["jacobi_gram_bytes"]
         if name.startswith("pair_eig32_kernel") or name.startswith("(gram_kernel"):
             fma = 4.25 * work["jacobi_gram_bytes"]
+        elif name.startswith("jacobi_ring32_kernel"):
+            # per row and round of a CTA's eight columns: 80 FMAs for the sums
+            # of 16 pairs, 192 for their rotations
+            fma = 3.0 * work["jacobi_rot_bytes"] + 1.25 * work["jacobi_gram_bytes"]
         elif name.startswith("pair_apply32_kernel") or name.startswith("apply_kernel"):
             fma = 8.0 * work["jacobi_rot_bytes"]
         # work counters are per update; the profile covers n_prof updates

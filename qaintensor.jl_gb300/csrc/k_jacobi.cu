@@ -12,8 +12,13 @@
 // (the pair solver) and the resulting unitary applied to the pair's columns
 // of X (and rows of V).  A sweep in which no pair rotates ends the iteration.
 // Round implementations:
-//   FP32 storage, default: jacobi_sweep32_kernel -- one cooperative launch
-//     per sweep, each round rebuilding its columns from the previous round's
+//   FP32 storage, where the caller takes pairwise rotations (a sketched
+//     matrix): jacobi_ring32_kernel -- one cooperative launch per sweep,
+//     single column pairs rotated in the registers of a CTA that holds eight
+//     columns, blocks of four columns passed between CTAs (see the comment
+//     above that kernel);
+//   FP32 storage otherwise: jacobi_sweep32_kernel -- one cooperative launch per
+//     sweep, each round rebuilding its columns from the previous round's
 //     unitaries (see the comment above that kernel);
 //   FP32 storage, two launches per round: pair_eig32_kernel (Gram + test +
 //     pair solver) and pair_apply32_kernel (rotation);
@@ -1886,6 +1891,463 @@ jacobi_sweep32_kernel(float2* __restrict__ xb0, float2* __restrict__ xb1, int64_
   }
 }
 
+// ---------------------------------------------------------------------------
+// FP32 storage: columns resident in registers, one cooperative launch per sweep
+// ---------------------------------------------------------------------------
+//
+// CTA c holds two blocks of RB = 4 columns in registers (warp w rows
+// 64 RP w ..., lane l rows l, l + 32, ... of them).  A round rotates the 16 cross pairs of its two blocks, four
+// disjoint pairs at a time: every warp sums its rows, the sums meet in shared
+// memory, every warp adds them in the same order, finds the same four
+// rotations and rotates its rows.  A sweep's first round also rotates the pairs
+// inside each block.  No Gram, no unitary, no second pass over the rows.
+//
+// Between rounds one block stays and the other moves on, for most of the sweep
+// (ring_blocks): on K CTAs the K moving blocks pass once round the ring of CTAs
+// (K rounds), which pairs every staying block with every moving one; then the
+// staying blocks pair up among themselves on half of the CTAs and the moving
+// ones on the other half, and so on; an odd number of CTAs plays a tournament.
+// K + K/2 + ... = 2 K - 1 rounds cover every pair of the 2 K blocks once, and
+// half the traffic of a tournament.  A block that leaves is written to its slot
+// of the mailbox by the warps that hold it, every number in one 8-byte half of
+// a 16-byte store with the number of the round in the other 4 bytes; the warp of
+// the same rows in the next CTA reads the slot until every number carries that
+// round.  So the data is its own flag: no fence and no second trip to L2 (a flag
+// behind a fence cost 4.5 us a round, twice this), and no CTA-wide barrier.  A
+// slot is written only by the CTA that holds its block, i.e. that has read it.
+// Every wait is bounded (QT_FLAG_ABORT ends them all and becomes QT_ETIMEOUT);
+// leaving blocks are written before any wait and all CTAs are resident, so the
+// waits end.
+//
+// The rotation: FP32 on the scaled sums (cosine and ratio of the norms, O(1)
+// numbers at any scale), then brought to unit length from its exactly formed
+// defect, as near to unitary as FP32 stores it.
+//
+// What bounds it: 20 FMAs per row and column pair (2048 x 1152: 0.67 ms a sweep
+// over the chip), the four sub-rounds' barrier and rotation chain, and the
+// exchange's latency.  Eight columns of 2048 rows are half of an SM's
+// registers, and 1152 columns its 144 CTAs.  Measured on the chi = 1024 sketch
+// (2048 x 1152): 2.6 ms a sweep, 9.0 us a round (four sub-rounds 4.7, exchange
+// 3.5 to 4), against 5.2 ms of the Gram-based sweep kernel, in as many sweeps;
+// 512 x 320: 0.35 against 1.03 ms a sweep, 4.4 us a round.  Not taken where the
+// caller needs the split of theta' itself: every column is rounded once per
+// pair and not once per round of 16 columns, and a 14-qubit circuit came out
+// 4.6e-6 off instead of 3.5e-6; a sketch's own error hides that.
+
+constexpr int RB = 4;            // columns per block
+constexpr int RING_WARPS = 16;   // warps per CTA at most (128 registers a thread)
+constexpr int RING_CTAS = 512;   // CTAs at most (the schedule table in shared memory)
+
+// Rounds of a sweep on K CTAs.
+__host__ __device__ inline int ring_rounds(int K) {
+  int r = 0;
+  while (K % 2 == 0) { r += K; K /= 2; }
+  return r + 2 * K - 1;
+}
+
+// Blocks (of 2 K) that CTA c holds in round r.
+__device__ inline void ring_blocks(int K, int r, int c, int& a, int& b) {
+  int size[10], lev = 0, k = K, upper = 0;  // levels above: their group sizes, bit lev of `upper`: second half
+  while (k % 2 == 0 && r >= k) {
+    r -= k;
+    size[lev] = k;
+    k /= 2;
+    if (c >= k) { upper |= 1 << lev; c -= k; }
+    lev++;
+  }
+  int m[2] = {0, 1}, i[2];  // list (0: staying, 1: moving) and place in it
+  if (k % 2 == 0 || k == 1) {
+    i[0] = c;
+    i[1] = (c + r) % k;
+  } else {  // tournament over the 2 k blocks: 0 .. k - 1 the first list
+    int x, y;
+    tournament(r, c, 2 * k, x, y);
+    m[0] = x >= k; i[0] = x - m[0] * k;
+    m[1] = y >= k; i[1] = y - m[1] * k;
+  }
+  for (int h = 0; h < 2; h++) {
+    int mm = m[h], ii = i[h];
+    for (int l = lev - 1; l >= 0; l--) {
+      const int n = size[l], half = n / 2;
+      if ((upper >> l) & 1) { ii = mm ? (ii - 1 + n) % n : (ii + half - 1) % n; mm = 1; }
+      else { ii = mm ? ii + half : ii; mm = 0; }
+    }
+    (h ? b : a) = mm * K + ii;
+  }
+}
+
+struct RingArgs {
+  float2* X;
+  int64_t ldx;
+  int mm, nn;
+  int g0;          // rounds before this sweep
+  float tol;
+  double nu_rel2;
+  const double* xnorm2;
+  uint4* mail;     // a slot of warps x RB x rows-per-lane x 32 entries for each of the 2 K blocks
+  int* flags;
+  float keep2;
+  float* dnorm;    // the columns' squared norms at the end of the sweep (nullptr: not wanted)
+  int spin, stall;
+};
+
+// Two FP32 values in a 64-bit register, one instruction for both (sm_100 on).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 x2_pack(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 x2_unpack(f32x2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+  return r;
+}
+__device__ __forceinline__ f32x2 x2_fma(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 x2_mul(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float x2_sum(f32x2 a) {
+  const float2 v = x2_unpack(a);
+  return v.x + v.y;
+}
+
+// An entry of the mailbox: each 8-byte half arrives whole, so a number is there
+// when its round is.
+__device__ __forceinline__ void mail_store(uint4* p, float re, float im, unsigned stamp) {
+  asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %2};" ::"l"(p), "r"(__float_as_uint(re)), "r"(stamp),
+               "r"(__float_as_uint(im))
+               : "memory");
+}
+__device__ __forceinline__ uint4 mail_load(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p)
+               : "memory");
+  return v;
+}
+
+// The rows a lane holds of one column: pairs of rows, real and imaginary parts
+// apart, so that every product of a rotation is one instruction for two rows.
+template <int RP>
+struct ring_col { f32x2 re[RP], im[RP]; };
+
+// RP: row pairs per lane (2 RP rows).
+template <int RP>
+__global__ void __launch_bounds__(32 * RING_WARPS, 1) jacobi_ring32_kernel(RingArgs A) {
+  typedef ring_col<RP> Col;
+  __shared__ float part[2][RING_WARPS * 4 * RB];
+  __shared__ int table[2 * RING_CTAS];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5, nw = blockDim.x >> 5, K = gridDim.x, cta = blockIdx.x;
+  const int rounds = ring_rounds(K);
+  for (int r = t; r < rounds; r += blockDim.x) {
+    int x, y;
+    ring_blocks(K, r, cta, x, y);
+    table[r] = x << 16 | y;
+  }
+  if (A.stall && cta == 0 && t == 0) {
+    // test hook (QT_JACOBI_STALL_TEST): a bounded wait on a status word that
+    // nothing sets, which must end in QT_ETIMEOUT with the context usable
+    int it = 0;
+    while (it < A.spin && ld_acquire_gpu(A.flags + QT_FLAG_STALL) == 0) { it++; __nanosleep(64); }
+    if (it >= A.spin) atomicExch(A.flags + QT_FLAG_ABORT, 1);
+  }
+  __syncthreads();
+  const int row0 = w * 64 * RP + lane;
+  const float nu2 = (float)(A.nu_rel2 * (*A.xnorm2)), big2 = (float)(1e-6 * (*A.xnorm2)), tol2 = A.tol * A.tol;
+
+  auto load = [&](Col (&x)[RB], int blk) {
+    float2 v[RB][2 * RP];
+#pragma unroll
+    for (int j = 0; j < RB; j++) {
+      const int c = blk * RB + j;
+#pragma unroll
+      for (int k = 0; k < 2 * RP; k++) {
+        const int r = row0 + 32 * k;
+        v[j][k] = (c < A.nn && r < A.mm) ? __ldcg(A.X + r + A.ldx * c) : make_float2(0.f, 0.f);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < RB; j++)
+#pragma unroll
+      for (int k = 0; k < RP; k++) {
+        x[j].re[k] = x2_pack(v[j][2 * k].x, v[j][2 * k + 1].x);
+        x[j].im[k] = x2_pack(v[j][2 * k].y, v[j][2 * k + 1].y);
+      }
+  };
+  auto store = [&](const Col (&x)[RB], int blk) {
+#pragma unroll
+    for (int j = 0; j < RB; j++) {
+      const int c = blk * RB + j;
+#pragma unroll
+      for (int k = 0; k < RP; k++) {
+        const float2 re = x2_unpack(x[j].re[k]), im = x2_unpack(x[j].im[k]);
+        const int r = row0 + 64 * k;
+        if (c < A.nn && r < A.mm) __stcg(A.X + r + A.ldx * c, make_float2(re.x, im.x));
+        if (c < A.nn && r + 32 < A.mm) __stcg(A.X + r + 32 + A.ldx * c, make_float2(re.y, im.y));
+      }
+    }
+  };
+  auto slot = [&](int blk) { return A.mail + ((size_t)blk * nw + w) * (RB * 2 * RP * 32) + lane; };
+  auto publish = [&](const Col (&x)[RB], int blk, unsigned stamp) {
+    uint4* m = slot(blk);
+#pragma unroll
+    for (int j = 0; j < RB; j++)
+#pragma unroll
+      for (int k = 0; k < RP; k++) {
+        const float2 re = x2_unpack(x[j].re[k]), im = x2_unpack(x[j].im[k]);
+        mail_store(m + (j * 2 * RP + 2 * k) * 32, re.x, im.x, stamp);
+        mail_store(m + (j * 2 * RP + 2 * k + 1) * 32, re.y, im.y, stamp);
+      }
+  };
+  auto fetch = [&](Col (&x)[RB], int blk, unsigned stamp) {
+    const uint4* m = slot(blk);
+    for (int it = 0;; it++) {
+      uint4 v[RB][2 * RP];
+#pragma unroll
+      for (int j = 0; j < RB; j++)
+#pragma unroll
+        for (int k = 0; k < 2 * RP; k++) v[j][k] = mail_load(m + (j * 2 * RP + k) * 32);
+      bool here = true;
+#pragma unroll
+      for (int j = 0; j < RB; j++)
+#pragma unroll
+        for (int k = 0; k < 2 * RP; k++) here = here && v[j][k].y == stamp && v[j][k].w == stamp;
+#pragma unroll
+      for (int j = 0; j < RB; j++)
+#pragma unroll
+        for (int k = 0; k < RP; k++) {
+          x[j].re[k] = x2_pack(__uint_as_float(v[j][2 * k].x), __uint_as_float(v[j][2 * k + 1].x));
+          x[j].im[k] = x2_pack(__uint_as_float(v[j][2 * k].z), __uint_as_float(v[j][2 * k + 1].z));
+        }
+      if (__all_sync(0xffffffffu, here)) break;
+      // given up, here or elsewhere: every wait ends, the sweep runs out and the host reports it
+      const bool last = it >= A.spin;
+      if (last && lane == 0) atomicExch(A.flags + QT_FLAG_ABORT, 1);
+      if (last || ((it & 7) == 7 && *(volatile int*)(A.flags + QT_FLAG_ABORT))) break;
+    }
+  };
+  float relmax = 0.f, relbig = 0.f, relkept = 0.f;  // of the lane's pairs that rotated (warp 0)
+  float aa = 0.f, bb = 0.f;                         // squared norms of pair lane / 8
+  int buf = 0;
+  // `n` sums per pair (v, pair by pair) over the CTA's rows of X; lane l ends
+  // with sum l n / 32 of every warp, added in the same order in each
+  auto total = [&](auto& v, auto count) -> float {
+    constexpr int CNT = decltype(count)::value;  // 16 or 8
+    constexpr int SH = 32 / CNT;                 // lanes per sum
+    int off = 16;
+#pragma unroll
+    for (int cnt = CNT; cnt > 1; cnt >>= 1, off >>= 1) {
+      const bool up = lane & off;
+#pragma unroll
+      for (int i = 0; i < cnt / 2; i++) {
+        const float send = up ? v[i] : v[i + cnt / 2];
+        const float keep = up ? v[i + cnt / 2] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+      }
+    }
+    float s = v[0];
+#pragma unroll
+    for (int o = SH / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (nw > 1) {
+      // each of a sum's lanes adds every SH-th warp's part, then the lanes meet
+      if ((lane & (SH - 1)) == 0) part[buf][w * CNT + lane / SH] = s;
+      __syncthreads();
+      s = 0.f;
+      for (int u = lane & (SH - 1); u < nw; u += SH) s += part[buf][u * CNT + lane / SH];
+#pragma unroll
+      for (int o = 1; o < SH; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      buf ^= 1;
+    }
+    return s;
+  };
+  // four disjoint pairs (p[g], q[g]): the same answer in every warp.  `fresh`:
+  // the squared norms from the columns; otherwise as the last rotations left
+  // them (a round measures them once and rotates each column three times more)
+  auto rotate = [&](Col (&p)[RB], Col (&q)[RB], auto fresh) -> bool {
+    constexpr bool FRESH = decltype(fresh)::value;
+    constexpr int PER = FRESH ? 4 : 2;
+    float v[PER * RB];
+#pragma unroll
+    for (int g = 0; g < RB; g++) {
+      f32x2 na = 0, nb = 0, gr = 0, g1 = 0, g2 = 0;
+#pragma unroll
+      for (int k = 0; k < RP; k++) {
+        const f32x2 xr = p[g].re[k], xi = p[g].im[k], yr = q[g].re[k], yi = q[g].im[k];
+        if (FRESH) {
+          na = x2_fma(xr, xr, x2_fma(xi, xi, na));
+          nb = x2_fma(yr, yr, x2_fma(yi, yi, nb));
+        }
+        gr = x2_fma(xr, yr, x2_fma(xi, yi, gr));
+        g1 = x2_fma(xr, yi, g1);
+        g2 = x2_fma(xi, yr, g2);
+      }
+      v[PER * g] = x2_sum(gr);
+      v[PER * g + 1] = x2_sum(g1) - x2_sum(g2);
+      if (FRESH) {
+        v[PER * g + 2] = x2_sum(na);
+        v[PER * g + 3] = x2_sum(nb);
+      }
+    }
+    const float s = total(v, std::integral_constant<int, PER * RB>());
+    const int base = lane & ~7;
+    const float gr = __shfl_sync(0xffffffffu, s, base), gi = __shfl_sync(0xffffffffu, s, base + 8 / PER);
+    if (FRESH) {
+      aa = __shfl_sync(0xffffffffu, s, base + 4);
+      bb = __shfl_sync(0xffffffffu, s, base + 6);
+    }
+    const float ra = rsqrtf(aa), rb = rsqrtf(bb);
+    const float er = gr * ra * rb, ei = gi * ra * rb;  // e^{i phi} times the cosine
+    const float c2 = fmaf(er, er, ei * ei);
+    const bool rot = aa > nu2 && bb > nu2 && c2 > tol2;
+    const unsigned on = __ballot_sync(0xffffffffu, rot);
+    if (!on) return false;
+    float c = 1.f, sr = 0.f, si = 0.f;
+    if (rot) {
+      const float rc = rsqrtf(c2);
+      const float zeta = 0.5f * ((bb - aa) * ra * rb) * rc;
+      const float az = fabsf(zeta);
+      const float tt = copysignf(__fdividef(1.f, az > 1e6f ? 2.f * az : az + sqrtf(fmaf(az, az, 1.f))), zeta);
+      const float c0 = rsqrtf(fmaf(tt, tt, 1.f));
+      const float s0 = c0 * tt * rc;
+      const float sr0 = s0 * er, si0 = s0 * ei;
+      // the defect 1 - |(c0, sr0, si0)|^2, each step one rounding of a number <= 1
+      const float h = 0.5f * fmaf(-si0, si0, fmaf(-sr0, sr0, fmaf(-c0, c0, 1.f)));
+      c = fmaf(h, c0, c0);
+      sr = fmaf(h, sr0, sr0);
+      si = fmaf(h, si0, si0);
+      const float rel = fminf(c2 * rc, 1.f);
+      if (w == 0) {
+        relmax = fmaxf(relmax, rel);
+        if (aa > big2 && bb > big2) relbig = fmaxf(relbig, rel);
+        if (fmaxf(aa, bb) > A.keep2) relkept = fmaxf(relkept, rel);
+      }
+      const float d = tt * rel * (aa * ra) * (bb * rb);  // t |gamma|
+      aa = fmaxf(aa - d, 0.f);
+      bb = bb + d;
+    }
+#pragma unroll
+    for (int g = 0; g < RB; g++) {
+      const float cg = __shfl_sync(0xffffffffu, c, 8 * g);
+      const float srg = __shfl_sync(0xffffffffu, sr, 8 * g), sig = __shfl_sync(0xffffffffu, si, 8 * g);
+      if (!((on >> (8 * g)) & 1)) continue;
+      const f32x2 cc = x2_pack(cg, cg), ss = x2_pack(srg, srg), ns = x2_pack(-srg, -srg), ii = x2_pack(sig, sig),
+                  ni = x2_pack(-sig, -sig);
+#pragma unroll
+      for (int k = 0; k < RP; k++) {
+        // x_p' = c x_p - conj(se) x_q ;  x_q' = se x_p + c x_q
+        const f32x2 xr = p[g].re[k], xi = p[g].im[k], yr = q[g].re[k], yi = q[g].im[k];
+        p[g].re[k] = x2_fma(cc, xr, x2_fma(ns, yr, x2_mul(ni, yi)));
+        p[g].im[k] = x2_fma(cc, xi, x2_fma(ns, yi, x2_mul(ii, yr)));
+        q[g].re[k] = x2_fma(cc, yr, x2_fma(ss, xr, x2_mul(ni, xi)));
+        q[g].im[k] = x2_fma(cc, yi, x2_fma(ss, xi, x2_mul(ii, xr)));
+      }
+    }
+    return true;
+  };
+
+  const std::true_type fresh;
+  const std::false_type tracked;
+  Col xa[RB], xb[RB];
+  int ka = table[0] >> 16, kb = table[0] & 0xffff;
+  load(xa, ka);
+  load(xb, kb);
+  int rotated = 0;
+  for (int r = 0; r < rounds; r++) {
+    bool ch = false;
+    if (r == 0) {
+      // the pairs inside each block, once a sweep: columns 1, 2, 3 of each move
+      // round one place per step
+#pragma unroll 1
+      for (int st = 0; st < 3; st++) {
+        Col p[RB] = {xa[0], xa[2], xb[0], xb[2]}, q[RB] = {xa[1], xa[3], xb[1], xb[3]};
+        ch |= rotate(p, q, fresh);
+        xa[0] = p[0]; xa[1] = p[1]; xa[2] = q[1]; xa[3] = q[0];
+        xb[0] = p[2]; xb[1] = p[3]; xb[2] = q[3]; xb[3] = q[2];
+      }
+    }
+    // the cross pairs; b's columns move one place per step
+    ch |= rotate(xa, xb, fresh);
+#pragma unroll 1
+    for (int st = 1; st < RB; st++) {
+      const Col f = xb[0];
+      xb[0] = xb[1]; xb[1] = xb[2]; xb[2] = xb[3]; xb[3] = f;
+      bb = __shfl_sync(0xffffffffu, bb, (lane + 8) & 31);
+      ch |= rotate(xa, xb, tracked);
+    }
+    {
+      const Col f = xb[0];
+      xb[0] = xb[1]; xb[1] = xb[2]; xb[2] = xb[3]; xb[3] = f;
+    }
+    rotated += ch;
+    if (r + 1 == rounds) break;
+    // ---- exchange: publish what leaves, then wait for what comes
+    const int na = table[r + 1] >> 16, nb = table[r + 1] & 0xffff;
+    const unsigned stamp = A.g0 + r + 1;
+    if (kb == na || ka == nb) {
+#pragma unroll
+      for (int j = 0; j < RB; j++) { const Col f = xa[j]; xa[j] = xb[j]; xb[j] = f; }
+      const int f = ka; ka = kb; kb = f;
+    }
+    const bool fa = na != ka, fb = nb != kb;
+    if (fa) publish(xa, ka, stamp);
+    if (fb) publish(xb, kb, stamp);
+    ka = na;
+    kb = nb;
+    if (fa) fetch(xa, ka, stamp);
+    if (fb) fetch(xb, kb, stamp);
+  }
+  store(xa, ka);
+  store(xb, kb);
+  if (A.dnorm) {
+    float v[2 * RB];
+#pragma unroll
+    for (int j = 0; j < RB; j++) {
+      f32x2 f = 0, g = 0;
+#pragma unroll
+      for (int k = 0; k < RP; k++) {
+        f = x2_fma(xa[j].re[k], xa[j].re[k], x2_fma(xa[j].im[k], xa[j].im[k], f));
+        g = x2_fma(xb[j].re[k], xb[j].re[k], x2_fma(xb[j].im[k], xb[j].im[k], g));
+      }
+      v[j] = x2_sum(f);
+      v[RB + j] = x2_sum(g);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 2 * RB; j++) {
+      for (int o = 16; o > 0; o >>= 1) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
+      if (lane == 0) part[0][w * 2 * RB + j] = v[j];
+    }
+    __syncthreads();
+    if (t < 2 * RB) {
+      float f = 0.f;
+      for (int u = 0; u < nw; u++) f += part[0][u * 2 * RB + t];
+      const int c = (t < RB ? ka : kb) * RB + t % RB;
+      if (c < A.nn) A.dnorm[c] = f;
+    }
+  }
+  if (w == 0) {
+    for (int o = 16; o > 0; o >>= 1) {
+      relmax = fmaxf(relmax, __shfl_xor_sync(0xffffffffu, relmax, o));
+      relbig = fmaxf(relbig, __shfl_xor_sync(0xffffffffu, relbig, o));
+      relkept = fmaxf(relkept, __shfl_xor_sync(0xffffffffu, relkept, o));
+    }
+    if (lane == 0) {
+      if (rotated) atomicAdd(&A.flags[QT_FLAG_ROTATED], rotated);
+      if (relmax > 0.f) atomicMax(&A.flags[QT_FLAG_OFFMAX], __float_as_int(relmax));
+      if (relbig > 0.f) atomicMax(&A.flags[QT_FLAG_OFFBIG], __float_as_int(relbig));
+      if (relkept > 0.f) atomicMax(&A.flags[QT_FLAG_OFFKEPT], __float_as_int(relkept));
+    }
+  }
+}
+
 // ||X||_F^2 in FP64, one CTA per column, added into *out.
 template <typename TS>
 __global__ void frob_kernel(const TS* __restrict__ X, int64_t ldx, int mm, double* out) {
@@ -2094,9 +2556,68 @@ static int launch_sweep32(qt_handle* h, int pairs, float2* x0, float2* x1, int64
   return QT_OK;
 }
 
+// Launch shape of jacobi_ring32_kernel: two rows per lane up to 512 rows, then
+// four, so that a CTA has up to 8 warps, 16 only from 1024 rows on (a warp's
+// share of a round beside its products -- shuffles, rotation, barrier -- is the
+// same however few rows it holds).
+struct ring_shape {
+  int rows = 0, warps = 0, ctas = 0;  // rows per lane
+};
+static const void* ring_kernel(int rows) {
+  return rows == 2 ? (const void*)jacobi_ring32_kernel<1> : (const void*)jacobi_ring32_kernel<2>;
+}
+// ctas = 0 where it does not apply: more rows than 16 warps hold, or more
+// blocks than the resident CTAs.  QT_JACOBI_RING=0 turns it off.
+static ring_shape shape_ring32(int64_t mm, int64_t nn) {
+  ring_shape s;
+  const char* env = std::getenv("QT_JACOBI_RING");
+  if (env && env[0] == '0') return s;
+  s.rows = mm <= 512 ? 2 : 4;
+  const int64_t warps = (mm + 32 * s.rows - 1) / (32 * s.rows), ctas = ((nn + RB - 1) / RB + 1) / 2;
+  if (warps > RING_WARPS || ctas > RING_CTAS) return s;
+  s.warps = (int)warps;
+  int dev = 0, coop = 0, sms = 0, per_sm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ring_kernel(s.rows), 32 * s.warps, 0) != cudaSuccess) {
+    cudaGetLastError();
+    return s;
+  }
+  if (ctas <= (int64_t)per_sm * sms) s.ctas = (int)ctas;
+  return s;
+}
+
+static int launch_ring32(qt_handle* h, const ring_shape& s, RingArgs a) {
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3((unsigned)s.ctas);
+  lc.blockDim = dim3(32 * s.warps);
+  lc.stream = h->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  lc.attrs = attr;
+  lc.numAttrs = 1;
+  // QT_JACOBI_STALL_TEST=N (tests only): CTA 0 waits at most N polls on a
+  // status word nothing sets, and every block wait is limited to N polls
+  const char* stall_env = std::getenv("QT_JACOBI_STALL_TEST");
+  const int stall_polls = stall_env ? std::atoi(stall_env) : 0;
+  a.spin = stall_polls > 0 ? stall_polls : PS_SPIN;
+  a.stall = stall_polls > 0 ? 1 : 0;
+  void* args[] = {&a};
+  if (h->prof) qt_prof_before(h, "jacobi_ring32_kernel");
+  const cudaError_t e = cudaLaunchKernelExC(&lc, ring_kernel(s.rows), args);
+  if (h->prof) qt_prof_after(h);
+  h->launches++;
+  if (e != cudaSuccess)
+    return qt_fail(h, QT_ECUDA, std::string("launch jacobi_ring32_kernel: ") + cudaGetErrorString(e));
+  return QT_OK;
+}
+
 template <typename TS>
 int qt_jacobi_svd_ws(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, TS* V, int64_t ldv, double tol,
-                     int max_sweeps, int* sweeps_out, double2* parts, double nu_rel_in, int keep_count) {
+                     int max_sweeps, int* sweeps_out, double2* parts, double nu_rel_in, int keep_count,
+                     bool pairwise) {
   typedef typename gram_of<TS>::type TG;
   if (mm < nn) return qt_fail(h, QT_EINVAL, "jacobi: needs rows >= columns");
   if (V) QT_TRY(qt_set_identity<TS>(h, V, nn, ldv));
@@ -2130,17 +2651,20 @@ int qt_jacobi_svd_ws(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, T
   const double nu_rel = nu_rel_in > 0 ? nu_rel_in
                         : (fp32 ? 4.0 * u : 4.0 * std::sqrt((double)std::max<int64_t>(mm, 16)) * u);
   const double nu_rel2 = nu_rel * nu_rel;
-  // Round implementation (cfg.jacobi_kernel): FP32 storage by default runs
-  // two launches per round (Gram + pair solver, then the rotation); 2 asks
-  // for the one-launch cluster round, 1 for the three-kernel round.  FP64
+  // Round implementation (cfg.jacobi_kernel): FP32 storage by default rotates
+  // register-resident columns in one launch per sweep where the caller takes
+  // pairwise rotations, else (and with more columns than that holds) runs the
+  // Gram-based sweep kernel, beyond its size two launches per round (Gram + pair solver, then the rotation; also 3); 2 asks for the
+  // one-launch cluster round, 1 for the three-kernel round.  FP64
   // storage uses the one-launch round where a pair's rows fit a cluster's
   // shared memory.
   const int jk = h->cfg.jacobi_kernel;
-  const bool sweep_kernel = fp32 && jk == 0 && sweep32_fits(h, pairs);
-  const bool two_launch = fp32 && (jk == 3 || (jk == 0 && !sweep_kernel));
+  const ring_shape ring = fp32 && jk == 0 && pairwise && !V ? shape_ring32(mm, nn) : ring_shape();
+  const bool sweep_kernel = fp32 && jk == 0 && !ring.ctas && sweep32_fits(h, pairs);
+  const bool two_launch = fp32 && (jk == 3 || (jk == 0 && !sweep_kernel && !ring.ctas));
   int xrows_c = 0, lds = 0;
   size_t smem = 0;
-  const bool one_launch = jk != 1 && !two_launch && !sweep_kernel;
+  const bool one_launch = jk != 1 && !two_launch && !sweep_kernel && !ring.ctas;
   const round64_shape r64 = one_launch && !fp32 ? shape_round64(mm, V ? nn : 0, pairs) : round64_shape();
   const int csize = !one_launch ? 0 : fp32 ? fused_shape(mm, pairs, &xrows_c, &lds, &smem) : r64.csize;
   // two-launch shape: one row per rotation thread, about eight CTAs per SM
@@ -2181,7 +2705,7 @@ int qt_jacobi_svd_ws(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, T
   static const double keep_margin =
       std::getenv("QT_JACOBI_KEEP_MARGIN") ? std::atof(std::getenv("QT_JACOBI_KEEP_MARGIN")) : 0.25;
   static const bool keep_stop = !std::getenv("QT_JACOBI_KEEP_STOP") || std::atoi(std::getenv("QT_JACOBI_KEEP_STOP"));
-  const bool keep_track = sweep_kernel && keep_count > 0 && keep_count < nn;
+  const bool keep_track = (sweep_kernel || ring.ctas) && keep_count > 0 && keep_count < nn;
   float* dnorm = nullptr;
   std::vector<float> hnorm;
   float keep2 = 0.f;
@@ -2213,11 +2737,19 @@ int qt_jacobi_svd_ws(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, T
     QT_TRY(pscratch.get(&X1, (size_t)ldx * nn));
     if (V) QT_TRY(pscratch.get(&V1, (size_t)ldv * nn));
     QT_CHECK_CUDA(h, cudaMemsetAsync(done, 0xff, sizeof(int) * pairs * halves, h->stream));
-    if (keep_track) {
-      QT_TRY(pscratch.get(&dnorm, (size_t)nn));
-      hnorm.resize(nn);
-    }
   }
+  uint4* ring_mail = nullptr;
+  if (ring.ctas) {
+    const size_t n = (size_t)2 * ring.ctas * ring.warps * RB * ring.rows * 32;
+    QT_TRY(pscratch.get(&ring_mail, n));
+    QT_CHECK_CUDA(h, cudaMemsetAsync(ring_mail, 0, sizeof(uint4) * n, h->stream));  // round 0: nothing sent
+  }
+  if (keep_track) {
+    QT_TRY(pscratch.get(&dnorm, (size_t)nn));
+    hnorm.resize(nn);
+  }
+  const int sweep_rounds = ring.ctas ? ring_rounds(ring.ctas) : rounds;
+  const int pair_cols = ring.ctas ? 2 * RB : JC;  // columns of a CTA's pair of blocks
   int sweep = 0;
   for (; sweep < max_sweeps; sweep++) {
     // FP32 storage: up to 2 inner sweeps of the pair solver in the first two
@@ -2240,7 +2772,16 @@ int qt_jacobi_svd_ws(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, T
       gcount += rounds;
       pending = true;
     }
-    for (int r = 0; r < rounds && !sweep_kernel; r++) {
+    if (ring.ctas) {
+      if constexpr (sizeof(typename real_of<TS>::type) == 4) {
+        RingArgs a = {};
+        a.X = (float2*)X; a.ldx = ldx; a.mm = (int)mm; a.nn = (int)nn; a.g0 = gcount; a.tol = (float)tol; a.nu_rel2 = nu_rel2; a.xnorm2 = xnorm2;
+        a.mail = ring_mail; a.flags = h->d_flags; a.keep2 = keep2; a.dnorm = dnorm;
+        QT_TRY(launch_ring32(h, ring, a));
+      }
+      gcount += sweep_rounds;
+    }
+    for (int r = 0; r < rounds && !sweep_kernel && !ring.ctas; r++) {
       if (two_launch) {
         if constexpr (sizeof(typename real_of<TS>::type) == 4) {
           QT_LAUNCH(h, pair_eig32_kernel, pairs, NTG, 0, (const float2*)X, ldx, (int)mm, (int)nn, nb, r, tol,
@@ -2273,18 +2814,19 @@ int qt_jacobi_svd_ws(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, T
     QT_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
     {
       const double es = (double)sizeof(TS);
-      h->work_jacobi_rounds += rounds;
+      h->work_jacobi_rounds += sweep_rounds;
       h->work_jacobi_pairs += h->h_flags[QT_FLAG_ROTATED];
       h->work_jacobi_inner += h->h_flags[QT_FLAG_INNER];
-      h->work_jacobi_bytes += (double)rounds * (double)mm * (double)nn * es +
-                              (double)h->h_flags[QT_FLAG_ROTATED] * JC * es * ((double)mm + (V ? 2.0 * (double)nn : 0.0));
-      h->work_jacobi_gram_bytes += (double)rounds * (double)mm * (double)nn * es;
-      h->work_jacobi_rot_bytes += (double)h->h_flags[QT_FLAG_ROTATED] * JC * es * ((double)mm + (V ? (double)nn : 0.0));
+      const double read = (double)sweep_rounds * (double)mm * (double)nn * es;
+      const double pair = (double)h->h_flags[QT_FLAG_ROTATED] * pair_cols * es;
+      h->work_jacobi_bytes += read + pair * ((double)mm + (V ? 2.0 * (double)nn : 0.0));
+      h->work_jacobi_gram_bytes += read;
+      h->work_jacobi_rot_bytes += pair * ((double)mm + (V ? (double)nn : 0.0));
     }
     float offkept = 0.f;
     std::memcpy(&offkept, &h->h_flags[QT_FLAG_OFFKEPT], sizeof(float));
     const float keep2_used = keep2;
-    double tail2 = -1.0, tail2_change = -1.0;
+    double tail2 = -1.0, tail2_change = -1.0, all2 = 0.0;
     if (keep_track) {
       // the weight left outside the keep_count largest columns bounds the
       // truncation error of the final split from above (those columns span
@@ -2295,6 +2837,7 @@ int qt_jacobi_svd_ws(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, T
       keep2 = (float)(keep_margin * keep_margin) * srt[keep_count - 1];
       tail2 = 0.0;
       for (int64_t c = keep_count; c < nn; c++) tail2 += (double)srt[c];
+      for (float v : srt) all2 += (double)v;
       if (prev_tail2 >= 0.0) tail2_change = prev_tail2 - tail2;
       prev_tail2 = tail2;
     }
@@ -2320,8 +2863,14 @@ int qt_jacobi_svd_ws(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, T
     // tail by about as much again: the truncation error is then final to
     // ~keep_tol / 2 relative)
     if (keep_track && keep_stop && keep2_used > 0.f && offkept == 0.f) break;
+    // The kept space itself is off by about the root of what the tail has yet
+    // to lose.  The ring's sweeps rotate each pair once, and their tail can
+    // settle to 1e-3 with the kept space still 4e-5 off (a bond of 45 whose
+    // truncation error is large), so what the next sweep would take, by the
+    // ratio of the last two, has to be below 1e-12 ||X||_F^2 too.
+    const bool settled = !ring.ctas || tail2_change * tail2_change <= 1e-12 * all2 * prev_change;
     if (keep_track && keep_stop && tail2_change >= 0.0 && prev_change >= 0.0 && tail2_change <= keep_tol * tail2 &&
-        prev_change <= 10.0 * keep_tol * tail2)
+        prev_change <= 10.0 * keep_tol * tail2 && settled)
       break;
     prev_change = tail2_change;
   }
@@ -2388,21 +2937,22 @@ int qt_jacobi_svd_ws(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, T
   return QT_OK;
 }
 template int qt_jacobi_svd_ws<double2>(qt_handle*, double2*, int64_t, int64_t, int64_t, double2*, int64_t, double,
-                                       int, int*, double2*, double, int);
+                                       int, int*, double2*, double, int, bool);
 template int qt_jacobi_svd_ws<float2>(qt_handle*, float2*, int64_t, int64_t, int64_t, float2*, int64_t, double, int,
-                                      int*, double2*, double, int);
+                                      int*, double2*, double, int, bool);
 
 template <typename TS>
 int qt_jacobi_svd(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, TS* V, int64_t ldv, double tol,
-                  int max_sweeps, int* sweeps_out, double nu_rel, int keep_count) {
+                  int max_sweeps, int* sweeps_out, double nu_rel, int keep_count, bool pairwise) {
   int nb = 0, chunks = 0;
   const int nparts = qt_jacobi_layout(mm, nn, &nb, &chunks);
   qt_scratch s(h);
   double2* parts;
   QT_TRY(s.get(&parts, (size_t)nparts));
-  return qt_jacobi_svd_ws<TS>(h, X, mm, nn, ldx, V, ldv, tol, max_sweeps, sweeps_out, parts, nu_rel, keep_count);
+  return qt_jacobi_svd_ws<TS>(h, X, mm, nn, ldx, V, ldv, tol, max_sweeps, sweeps_out, parts, nu_rel, keep_count,
+                              pairwise);
 }
 template int qt_jacobi_svd<double2>(qt_handle*, double2*, int64_t, int64_t, int64_t, double2*, int64_t, double, int,
-                                    int*, double, int);
+                                    int*, double, int, bool);
 template int qt_jacobi_svd<float2>(qt_handle*, float2*, int64_t, int64_t, int64_t, float2*, int64_t, double, int,
-                                   int*, double, int);
+                                   int*, double, int, bool);

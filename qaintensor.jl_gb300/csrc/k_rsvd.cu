@@ -154,14 +154,15 @@ __host__ __device__ constexpr size_t cq_smem_bytes(int nrb) {
          BW * sizeof(double) + BW * sizeof(float) + 16;
 }
 
-// acc -= conj(a) * b and acc -= a * b, four fused products each
-template <typename C>
-__device__ inline void cfms_conj(C& acc, C a, C b) {
+// acc -= conj(a) * b and acc -= a * b.  FP64: four fused products each, where an
+// instruction more is 16 cycles of the SM; FP32 rounds the product first.
+__device__ inline void cfms_conj(float2& acc, float2 a, float2 b) { acc = csub(acc, cmul(cconj(a), b)); }
+__device__ inline void cfms(float2& acc, float2 a, float2 b) { acc = csub(acc, cmul(a, b)); }
+__device__ inline void cfms_conj(double2& acc, double2 a, double2 b) {
   acc.x = fma(-a.x, b.x, acc.x); acc.x = fma(-a.y, b.y, acc.x);
   acc.y = fma(-a.x, b.y, acc.y); acc.y = fma(a.y, b.x, acc.y);
 }
-template <typename C>
-__device__ inline void cfms(C& acc, C a, C b) {
+__device__ inline void cfms(double2& acc, double2 a, double2 b) {
   acc.x = fma(-a.x, b.x, acc.x); acc.x = fma(a.y, b.y, acc.x);
   acc.y = fma(-a.x, b.y, acc.y); acc.y = fma(-a.y, b.x, acc.y);
 }

@@ -722,9 +722,13 @@ int svd_split_direct32(qt_handle* h, const float2* theta, int64_t m, int64_t n, 
   // QT_JACOBI_FREEZE scales the fast freeze threshold (tuning)
   static const double freeze_scale =
       std::getenv("QT_JACOBI_FREEZE") ? std::atof(std::getenv("QT_JACOBI_FREEZE")) : 1.0;
+  // Rotations pair by pair on a sketch (proj), whose random basis is further
+  // off than their rounding; the split of theta' itself keeps a round's 16
+  // columns times one unitary (see jacobi_ring32_kernel).
+  const bool pairwise = proj != nullptr;
   QT_TRY(qt_jacobi_svd<float2>(h, X, rows, cols, rows, V, cols, auto_tol(h, rows, true), h->cfg.max_sweeps,
                                &o->sweeps, fast_freeze ? freeze_scale * std::sqrt((double)rows) * 5.96e-8 : -1.0,
-                               keep_hint));
+                               keep_hint, pairwise));
   double* sig;
   int* perm;
   QT_TRY(s.get(&sig, (size_t)cols));
@@ -760,9 +764,16 @@ int svd_split_direct32(qt_handle* h, const float2* theta, int64_t m, int64_t n, 
   QT_TRY(s.get(&W, (size_t)k * k));
   if (!wide) QT_LAUNCH(h, gather_unit_cols_kernel<float2>, 256, 256, 0, X, m, m, perm, sig, k, A0);
   else QT_LAUNCH(h, gather_cols_kernel<float2>, 256, 256, 0, V, m, m, perm, k, A0);
-  QT_TRY(qt_gemm_any(h, QT_OP_C, QT_OP_N, k, k, m, one, A0, m, A0, m, zero, G, k));
-  QT_LAUNCH(h, newton_schulz_kernel, 256, 256, 0, G, k, W);
-  QT_TRY(qt_gemm_any(h, QT_OP_N, QT_OP_N, m, k, k, one, A0, m, W, k, zero, At, m));
+  // A kept-set stop leaves cosines of up to ~1e-2 between kept columns, whose
+  // Gram is then ~1e-2 from I in norm: one step leaves 3/4 of its square (1.2x
+  // the exact truncation error after a pairwise sketch at chi = 1024), a second
+  // one rounding.
+  for (int step = 0; step < (keep_hint > 0 && proj ? 2 : 1); step++) {
+    if (step) std::swap(A0, At);
+    QT_TRY(qt_gemm_any(h, QT_OP_C, QT_OP_N, k, k, m, one, A0, m, A0, m, zero, G, k));
+    QT_LAUNCH(h, newton_schulz_kernel, 256, 256, 0, G, k, W);
+    QT_TRY(qt_gemm_any(h, QT_OP_N, QT_OP_N, m, k, k, one, A0, m, W, k, zero, At, m));
+  }
   QT_TRY(qt_gemm_any(h, QT_OP_C, QT_OP_N, k, pn, m, one, At, m, psrc, m, zero, Bt, k));
   {
     // the kept values as reported: norms of the rows of B' = A'^H theta (an

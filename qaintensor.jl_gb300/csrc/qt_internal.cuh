@@ -240,7 +240,8 @@ int qt_norm2(qt_handle* h, const C* x, int64_t n, double* d_out);
 // TS = storage type.
 template <typename TS>
 int qt_jacobi_svd(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, TS* V, int64_t ldv,
-                  double tol, int max_sweeps, int* sweeps_out, double nu_rel = -1.0, int keep_count = 0);
+                  double tol, int max_sweeps, int* sweeps_out, double nu_rel = -1.0, int keep_count = 0,
+                  bool pairwise = false);
 // The same with a caller-supplied partial-Gram workspace of qt_jacobi_layout() double2 entries.
 // nu_rel > 0: columns with norm <= nu_rel ||X||_F are frozen (not rotated,
 // not tested); <= 0: the default for the storage precision.
@@ -251,9 +252,13 @@ int qt_jacobi_svd(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, TS* 
 // 1e-2 over the one before -- or once a sweep rotated no pair holding a
 // column within a factor 4 of the cut or above it.  Only columns far below
 // the cut, which the caller discards, are left unconverged.
+// pairwise (FP32): column pairs may be rotated one at a time in registers
+// (jacobi_ring32_kernel) instead of 16 columns by one unitary per round: two to
+// three times faster, every column rounded once per pair and not once per round.
 template <typename TS>
 int qt_jacobi_svd_ws(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, TS* V, int64_t ldv, double tol,
-                     int max_sweeps, int* sweeps_out, double2* parts, double nu_rel = -1.0, int keep_count = 0);
+                     int max_sweeps, int* sweeps_out, double2* parts, double nu_rel = -1.0, int keep_count = 0,
+                     bool pairwise = false);
 int qt_jacobi_layout(int64_t mm, int64_t nn, int* nb_out, int* chunks_out);
 
 // k_trunc.cu -----------------------------------------------------------------
