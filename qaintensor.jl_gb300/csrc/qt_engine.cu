@@ -1229,8 +1229,7 @@ extern "C" int qt_switch(qt_handle* h, qt_mps* mps, int site) {
 extern "C" int qt_expect_z(qt_handle* h, const qt_mps* mps, int site, double* out) {
   if (!h || !mps || !out) return qt_fail(h, QT_EINVAL, "expect_z: null argument");
   double num = 0, den = 0;
-  QT_TRY(qt_mps_expect(h, mps, site, 1, &num));
-  QT_TRY(qt_mps_expect(h, mps, 0, 0, &den));
+  QT_TRY(qt_mps_expect2(h, mps, site, 1, &num, &den));
   *out = num / den;
   return QT_OK;
 }
@@ -1238,8 +1237,7 @@ extern "C" int qt_expect_z(qt_handle* h, const qt_mps* mps, int site, double* ou
 extern "C" int qt_expect_zz(qt_handle* h, const qt_mps* mps, int site, double* out) {
   if (!h || !mps || !out) return qt_fail(h, QT_EINVAL, "expect_zz: null argument");
   double num = 0, den = 0;
-  QT_TRY(qt_mps_expect(h, mps, site, 2, &num));
-  QT_TRY(qt_mps_expect(h, mps, 0, 0, &den));
+  QT_TRY(qt_mps_expect2(h, mps, site, 2, &num, &den));
   *out = num / den;
   return QT_OK;
 }

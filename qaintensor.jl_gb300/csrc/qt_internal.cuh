@@ -297,3 +297,5 @@ int qt_split_device(qt_handle* h, int dtype, const void* M, int64_t m, int64_t n
 
 // k_obs.cu -------------------------------------------------------------------
 int qt_mps_expect(qt_handle* h, const qt_mps* mps, int site, int nops, double* out);
+// the same and <psi|psi>, from one pass over the sites (either may be null)
+int qt_mps_expect2(qt_handle* h, const qt_mps* mps, int site, int nops, double* num, double* den);
