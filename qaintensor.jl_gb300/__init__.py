@@ -720,20 +720,27 @@ class Batch:
         eng._check(eng._lib.qt_batch_create(eng._h, nq.size, _ptr(nq), _ptr(cm), C.byref(self._p)))
         self.ntask = 0
 
+    @staticmethod
+    def _pack_gates(gates) -> np.ndarray:
+        """Every gate's 16 entries, column-major, as interleaved doubles.  Gates
+        of one shape are packed in one pass (4 us a gate one by one)."""
+        if not gates:
+            return np.zeros(32, dtype=np.float64)
+        if len({np.shape(g) for g in gates}) == 1:
+            g = np.array(gates, dtype=np.complex128)
+            g = np.ascontiguousarray(g.transpose((0,) + tuple(range(g.ndim - 1, 0, -1))))
+            return g.reshape(-1).view(np.float64)
+        flat = [np.asarray(g, dtype=np.complex128).reshape(-1, order="F") for g in gates]
+        return np.concatenate(flat).view(np.float64)
+
     def run(self, layers, cutoff: float, use_graph: bool = True):
         """layers: list of lists of (circuit, wire 1-based, 4x4 gate)."""
-        starts, circ, site, gates = [0], [], [], []
-        for layer in layers:
-            for (c, w, g) in layer:
-                circ.append(c)
-                site.append(w - 1)
-                gf = np.asarray(g, dtype=np.complex128).reshape(-1, order="F")
-                gates.append(np.stack([gf.real, gf.imag], axis=1).ravel())
-            starts.append(len(circ))
-        st = np.asarray(starts, dtype=np.int32)
+        tasks = [t for layer in layers for t in layer]
+        st = np.cumsum([0] + [len(layer) for layer in layers], dtype=np.int32)
+        circ = [t[0] for t in tasks]
         ci = np.asarray(circ, dtype=np.int32)
-        si = np.asarray(site, dtype=np.int32)
-        ga = np.ascontiguousarray(np.concatenate(gates) if gates else np.zeros(32), dtype=np.float64)
+        si = np.asarray([t[1] for t in tasks], dtype=np.int32) - np.int32(1)
+        ga = self._pack_gates([t[2] for t in tasks])
         self.ntask = len(circ)
         self.eng._check(self.eng._lib.qt_batch_run(self.eng._h, self._p, len(layers), _ptr(st), _ptr(ci), _ptr(si),
                                                    _ptr(ga), float(cutoff), int(use_graph)))
