@@ -15,14 +15,17 @@
 //   sigma_j = ||x_j||           FP64, bitonic sort, tail rule (FP64, sequential) at
 //                               the caller's cutoff, cap; a decision below the FP32
 //                               resolution without a certificate (cap or exact rank
-//                               bound) is redone as an FP64 split in the same CTA
+//                               bound) is left to an FP64 split
 //   A' = x_perm(j) / sigma_j    written into site slot w
 //   B' = A'^H theta'            written into site slot w+1 (no V accumulation)
 //   bonds[w+1] = k
-// Tasks of one brickwork layer touch disjoint sites, so CTAs never race.  A
-// whole program (every layer) is a fixed sequence of (counter reset, kernel)
-// pairs that the host captures once in a CUDA graph.  There are no waits on
+// The tasks left to the FP64 split are listed, and a second kernel of the layer
+// takes them, a cluster of eight CTAs each (batch_split64_kernel).  Tasks of
+// one brickwork layer touch disjoint sites, so CTAs never race.  A whole program
+// (every layer) is a fixed sequence of a counter reset and kernels that the
+// host captures once in a CUDA graph.  There are no waits on
 // other CTAs: a CTA stops when the counter passes the task count.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -53,8 +56,10 @@ struct BatchArgs {
   const int* task_grank;     // per task: the gate's operator-Schmidt rank
   int task_begin, task_end;
   int* counter;
-  float2* slab;              // per CTA: 4 * slab_elems float2 (FP32 X, T; or the FP64 X, T of a fallback)
+  float2* slab;              // per CTA: 4 * slab_elems float2 (FP32 X, T; per cluster the FP64 T, X)
   int slab_elems;
+  int* left;                 // tasks of this layer left to the FP64 split, and how many
+  int* nleft;
   int smem_elems;            // float2 entries of the CTA's dynamic shared memory
   double cutoff;
   double floor_rel;          // FP32 resolution relative to ||theta'||_F (<= 0: 4 sqrt(max(m, n)) u)
@@ -68,9 +73,9 @@ struct BatchArgs {
 
 // theta' = G (A B) into T (m x n, ld m) and X (ld ldx): the product into T, then the
 // gate on the four physical values of each (a, b).  C = float2 (FP32 products)
-// or double2 (FP64, from double2 copies of the sites).
+// or double2 (FP64).
 template <int NT, int TMAX, typename C>
-__device__ void form_theta(const C* A, const C* B, int chil, int chim, int chir, const C* g, C* X, int ldx, C* T,
+__device__ void form_theta(const float2* A, const float2* B, int chil, int chim, int chir, const C* g, C* X, int ldx, C* T,
                            void* sm) {
   const int m = 2 * chil, n = 2 * chir;
   cta_gemm<NT, TMAX, C>(false, false, m, n, chim, A, m, nullptr, B, chim, sm,
@@ -108,6 +113,28 @@ __device__ double fro2_of(const C* X, int cnt, double* s_red) {
   return fro2;
 }
 
+// Bitonic sort, descending by value, ties by index; np2 entries, a power of two.
+template <int NT>
+__device__ void sort_values(int np2, double* s_sig, int* s_perm) {
+  for (int k2 = 2; k2 <= np2; k2 <<= 1)
+    for (int j2 = k2 >> 1; j2 > 0; j2 >>= 1) {
+      for (int i = threadIdx.x; i < np2; i += NT) {
+        const int l = i ^ j2;
+        if (l > i) {
+          const bool desc = ((i & k2) == 0);
+          const double x = s_sig[i], y = s_sig[l];
+          const bool sw = desc ? (x < y || (x == y && s_perm[i] > s_perm[l]))
+                               : (x > y || (x == y && s_perm[i] < s_perm[l]));
+          if (sw) {
+            s_sig[i] = y; s_sig[l] = x;
+            const int tp = s_perm[i]; s_perm[i] = s_perm[l]; s_perm[l] = tp;
+          }
+        }
+      }
+      __syncthreads();
+    }
+}
+
 // Column norms of X in FP64, sorted descending into s_sig / s_perm (bitonic).
 template <int NT, typename C>
 __device__ void sorted_norms(const C* X, int ld, int m, int n, double* s_sig, int* s_perm) {
@@ -128,23 +155,7 @@ __device__ void sorted_norms(const C* X, int ld, int m, int n, double* s_sig, in
     s_perm[j] = j;
   }
   __syncthreads();
-  for (int k2 = 2; k2 <= np2; k2 <<= 1)
-    for (int j2 = k2 >> 1; j2 > 0; j2 >>= 1) {
-      for (int i = threadIdx.x; i < np2; i += NT) {
-        const int l = i ^ j2;
-        if (l > i) {
-          const bool desc = ((i & k2) == 0);
-          const double x = s_sig[i], y = s_sig[l];
-          const bool sw = desc ? (x < y || (x == y && s_perm[i] > s_perm[l]))
-                               : (x > y || (x == y && s_perm[i] < s_perm[l]));
-          if (sw) {
-            s_sig[i] = y; s_sig[l] = x;
-            const int tp = s_perm[i]; s_perm[i] = s_perm[l]; s_perm[l] = tp;
-          }
-        }
-      }
-      __syncthreads();
-    }
+  sort_values<NT>(np2, s_sig, s_perm);
 }
 
 // The tail rule of src/svd.jl:29-33 (sequential from the smallest value,
@@ -174,7 +185,6 @@ __global__ void __launch_bounds__(NT) batch_layer_kernel(BatchArgs p) {
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ int s_task, s_k, s_fb;
   __shared__ float2 g[16];
-  __shared__ double2 g64[16];
   __shared__ double s_sig[MAXN];
   __shared__ int s_perm[MAXN];
   __shared__ double s_red[NT / 32];
@@ -199,7 +209,6 @@ __global__ void __launch_bounds__(NT) batch_layer_kernel(BatchArgs p) {
     if (tid < 16) {
       const double2 v = p.task_gate[(size_t)task * 16 + tid];
       g[tid] = make_float2((float)v.x, (float)v.y);
-      g64[tid] = v;
     }
     __syncthreads();
 
@@ -271,66 +280,190 @@ __global__ void __launch_bounds__(NT) batch_layer_kernel(BatchArgs p) {
       // 6. B' (k, 2, chir) = A'^H theta', into site slot w+1
       cta_gemm<NT, TMAX, float2>(true, false, k, n, m, A, m, nullptr, T, m, dyn,
                                  [&](int r, int col, float2 v) { B[r + (size_t)k * col] = v; });
-    } else {
-      // The exact FP64 split: theta' from the complex64 sites in FP64, FP64
-      // Jacobi (tolerance and freeze at FP64 rounding), the rule at the
-      // caller's cutoff.  The FP64 X and T take the whole slab (X the shared
-      // memory where it fits); X holds the widened sites before that.
-      double2* X64 = reinterpret_cast<double2*>(slab);
-      double2* T64 = X64 + p.slab_elems;
-      double2 *A64 = X64, *B64 = X64 + (size_t)m * chim;  // 2 chim (chil + chir) <= slab_elems
-      for (int i = tid; i < m * chim; i += NT) A64[i] = ccast<double2>(A[i]);
-      for (int i = tid; i < chim * n; i += NT) B64[i] = ccast<double2>(B[i]);
-      __syncthreads();
-      form_theta<NT, 32, double2>(A64, B64, chil, chim, chir, g64, T64, m, T64, dyn);
-      double* ws = reinterpret_cast<double*>(dyn);  // 4 n doubles, then X where it fits
-      const bool in_smem64 = 4 * n + 2 * (m + 1) * n <= p.smem_elems;
-      if (in_smem64) X64 = reinterpret_cast<double2*>(ws + 4 * n);
-      const int ld64 = in_smem64 ? m + 1 : m;
-      for (int j = tid >> 5; j < n; j += NT / 32)
-        for (int r = tid & 31; r < m; r += 32) X64[r + (size_t)ld64 * j] = T64[r + (size_t)m * j];
-      const double f64 = fro2_of<NT>(T64, m * n, s_red);
-      const double nu64 = 4.0 * sqrt((double)max(m, 16)) * 1.11e-16;
-      sweeps += cta_jacobi64<NT>(X64, ld64, m, n, 16.0 * sqrt((double)max(m, 16)) * 1.11e-16, nu64 * nu64 * f64,
-                                 p.max_sweeps, ws);
-      sorted_norms<NT, double2>(X64, ld64, m, n, s_sig, s_perm);
-      if (tid == 0) {
-        const int k = min(tail_rule(s_sig, n, p.cutoff), kcap);
-        double disc = 0;
-        for (int i = k; i < n; i++) disc += s_sig[i] * s_sig[i];
-        s_k = k;
-        p.task_rank[task] = k;
-        p.task_sweeps[task] = sweeps;
-        p.task_discarded[task] = (float)disc;
-      }
-      __syncthreads();
-      const int k = s_k;
-      // A' = unit columns, then B' = A'^H theta', both from the FP64 columns.
-      // The product's tiles take the start of the shared memory: columns kept
-      // there move to the slab first.
-      if (in_smem64) {
-        double2* Xs = reinterpret_cast<double2*>(slab);
-        for (int j = tid >> 5; j < n; j += NT / 32)
-          for (int r = tid & 31; r < m; r += 32) Xs[r + (size_t)m * j] = X64[r + (size_t)ld64 * j];
-        X64 = Xs;
-        __syncthreads();
-      }
-      for (int j = tid >> 5; j < k; j += NT / 32) {
-        const double s = s_sig[j];
-        const double inv = s > 0 ? 1.0 / s : 0.0;
-        const double2* x = X64 + (size_t)m * s_perm[j];
-        for (int r = tid & 31; r < m; r += 32) A[r + (size_t)m * j] = make_float2((float)(x[r].x * inv), (float)(x[r].y * inv));
-      }
-      __syncthreads();
-      cta_gemm<NT, 32, double2>(true, false, k, n, m, X64, m, s_perm, T64, m, dyn, [&](int r, int col, double2 v) {
-        const double s = s_sig[r];
-        const double inv = s > 0 ? 1.0 / s : 0.0;
-        B[r + (size_t)k * col] = make_float2((float)(v.x * inv), (float)(v.y * inv));
-      });
+      if (tid == 0) bond[w + 1] = k;
+    } else if (tid == 0) {
+      p.left[atomicAdd(p.nleft, 1)] = task;
     }
-    if (tid == 0) bond[w + 1] = s_k;
     __syncthreads();
   }
+}
+
+// The exact FP64 split of the tasks a layer left: theta' from the complex64
+// sites in FP64, one-sided FP64 Jacobi (tolerance and freeze at FP64 rounding),
+// the tail rule at the caller's cutoff.
+//
+// What bounds it: FP64 products (24 instructions per row of a column pair on
+// the two FP64 lanes of an SM), of few tasks a layer.  So a cluster of eight
+// CTAs takes one task: CTA q holds the rows congruent to q modulo 8 of every
+// column in shared memory (at most 32 x 256); a round's sums meet through
+// distributed shared memory, and every CTA finds the same rotations and
+// rotates its rows.  Four lanes share a pair, a warp eight pairs: an FP64
+// instruction costs the same however many lanes take part.  The sums keep the
+// order of one warp on whole columns (row r on lane r % 32, lanes 16, 8, 4, 2
+// and 1 apart added in turn: the first two inside a CTA, the others between
+// CTAs), because nearly equal columns leave the sign of a rotation to the
+// last bit, and later FP32 splits of the same circuit see which one was taken.
+// A 128 x 128 task (about 27 sweeps): 31 ms, 9 us a round, 8 us of them FP64
+// issue; by one CTA, as the layer kernel's last step, 95 ms.
+constexpr int S64_NT = 256, S64_C = 8, S64_W = S64_NT / 32;
+constexpr int S64_LD = 36;                    // rows of a slice, at most; 4 (mod 8) for the banks
+constexpr size_t S64_ROTS = MAXN / 2 * 5;     // rotations of a round's pairs: c, s, er, ei, on
+constexpr size_t S64_SUMS = MAXN / 2 * 4;     // sums of a round's pairs
+constexpr size_t S64_SMEM = (2 * S64_SUMS + S64_ROTS + 2 * S64_LD * MAXN) * sizeof(double);
+
+// Sums of this CTA's rows of each pair, aa bb gr gi.  4 K rows (zeros past the matrix).
+__device__ __forceinline__ void split64_sums(const double2* Xs, int ld, int K, int n, int round, double* part) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lr = lane & 3, pairs = n / 2;
+  for (int first = 8 * warp; first < pairs; first += 8 * S64_W) {
+    const int q = first + (lane >> 2);
+    int a, b;
+    cta_tourney(round, min(q, pairs - 1), n, a, b);
+    const double2 *xp = Xs + ld * a + lr, *xq = Xs + ld * b + lr;
+    double v0 = 0, v1 = 0, v2 = 0, v3 = 0;
+    for (int k = 0; k < K; k++) {
+      const double2 u = xp[4 * k], w = xq[4 * k];
+      v0 = fma(u.x, u.x, fma(u.y, u.y, v0));
+      v1 = fma(w.x, w.x, fma(w.y, w.y, v1));
+      v2 = fma(u.x, w.x, fma(u.y, w.y, v2));
+      v3 = fma(u.x, w.y, fma(-u.y, w.x, v3));
+    }
+    const bool up2 = lr & 2, up1 = lr & 1;
+    const double x0 = (up2 ? v2 : v0) + __shfl_xor_sync(0xffffffffu, up2 ? v0 : v2, 2);
+    const double x1 = (up2 ? v3 : v1) + __shfl_xor_sync(0xffffffffu, up2 ? v1 : v3, 2);
+    const double s = (up1 ? x1 : x0) + __shfl_xor_sync(0xffffffffu, up1 ? x0 : x1, 1);
+    if (q < pairs) part[4 * q + lr] = s;
+  }
+}
+
+__device__ __forceinline__ void split64_rotate(double2* Xs, int ld, int K, int n, int round, const double* rot) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lr = lane & 3, pairs = n / 2;
+  for (int q = 8 * warp + (lane >> 2); q < pairs; q += 8 * S64_W) {
+    if (rot[5 * q + 4] == 0) continue;
+    const double c = rot[5 * q], s = rot[5 * q + 1], er = rot[5 * q + 2], ei = rot[5 * q + 3];
+    int a, b;
+    cta_tourney(round, q, n, a, b);
+    double2 *xp = Xs + ld * a + lr, *xq = Xs + ld * b + lr;
+    for (int k = 0; k < K; k++) {
+      const double2 u = xp[4 * k], v = xq[4 * k];
+      xp[4 * k] = make_double2(c * u.x - s * (er * v.x + ei * v.y), c * u.y - s * (er * v.y - ei * v.x));
+      xq[4 * k] = make_double2(s * (er * u.x - ei * u.y) + c * v.x, s * (er * u.y + ei * u.x) + c * v.y);
+    }
+  }
+}
+
+__global__ void __cluster_dims__(S64_C, 1, 1) __launch_bounds__(S64_NT) batch_split64_kernel(BatchArgs p) {
+  extern __shared__ __align__(16) unsigned char dyn[];
+  __shared__ int s_next;
+  __shared__ double2 g64[16];
+  __shared__ double s_sig[MAXN], s_red[S64_NT / 32];
+  __shared__ int s_perm[MAXN], s_k;
+  cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rank = (int)cl.block_rank();
+  double* part = reinterpret_cast<double*>(dyn);  // two rounds' sums
+  double* rot = part + 2 * S64_SUMS;
+  double2* Xs = reinterpret_cast<double2*>(rot + S64_ROTS);
+  double2* T = reinterpret_cast<double2*>(p.slab + (size_t)(blockIdx.x - rank) * 4 * p.slab_elems);
+  double2* Xg = T + p.slab_elems;
+  for (;;) {
+    if (rank == 0 && tid == 0) s_next = atomicAdd(p.counter, 1);
+    cl.sync();
+    const int i = *cl.map_shared_rank(&s_next, 0);
+    if (i >= *p.nleft) break;
+    const int task = p.left[i];
+    const int c = p.task_circ[task], w = p.task_site[task];
+    int* bond = p.bonds + p.bond_off[c];
+    const int chil = bond[w], chim = bond[w + 1], chir = bond[w + 2], cap = p.cap[c];
+    const size_t slot = (size_t)cap * 2 * cap;
+    float2* A = p.sites + p.site_off[c] + (size_t)w * slot;
+    float2* B = A + slot;
+    const int m = 2 * chil, n = 2 * chir, pairs = n / 2;
+    // rows S64_C j + rank, j < rc, of which the last CTAs may have one less; 4 K with the zeros
+    const int rc = (m + S64_C - 1) / S64_C, K = (rc + 3) / 4, ld = 4 * (K | 1);
+    if (tid < 16) g64[tid] = p.task_gate[(size_t)task * 16 + tid];
+    __syncthreads();
+    // theta': this CTA's columns (the two values of s2 together), then its rows
+    const int b0 = rank * chir / S64_C, b1 = (rank + 1) * chir / S64_C;
+    double2* Tb = T + (size_t)m * 2 * b0;
+    const float2* Bb = B + (size_t)chim * 2 * b0;
+    if (b1 > b0) form_theta<S64_NT, 32, double2>(A, Bb, chil, chim, b1 - b0, g64, Tb, m, Tb, dyn);
+    cl.sync();
+    for (int j = warp; j < n; j += S64_W)
+      for (int r = lane; r < 4 * K; r += 32)
+        Xs[r + ld * j] = S64_C * r + rank < m ? T[S64_C * r + rank + (size_t)m * j] : make_double2(0, 0);
+    const double f64 = fro2_of<S64_NT>(T, m * n, s_red);  // the same in every CTA
+    const double tol = 16.0 * sqrt((double)max(m, 16)) * 1.11e-16, nu = 4.0 * sqrt((double)max(m, 16)) * 1.11e-16;
+    const double nu2 = nu * nu * f64;
+    int sweeps = 0, buf = 0;
+    for (int sweep = 0; sweep < p.max_sweeps; sweep++) {
+      bool rotated = false;
+      for (int r = 0; r < n - 1; r++) {
+        double* pb = part + buf * S64_SUMS;
+        split64_sums(Xs, ld, K, n, r, pb);
+        cl.sync();  // (two buffers: whoever reads this round's sums has left the last round's)
+        if (tid < pairs) {
+          double2 v[S64_C], u[S64_C];
+#pragma unroll
+          for (int q = 0; q < S64_C; q++) {
+            const double2* o = reinterpret_cast<const double2*>(cl.map_shared_rank(pb, q) + 4 * tid);
+            v[q] = o[0];
+            u[q] = o[1];
+          }
+#pragma unroll
+          for (int off = S64_C / 2; off > 0; off >>= 1)
+#pragma unroll
+            for (int q = 0; q < off; q++) {
+              v[q].x += v[q + off].x; v[q].y += v[q + off].y;
+              u[q].x += u[q + off].x; u[q].y += u[q + off].y;
+            }
+          const cta_rotation<double> o = cta_angle64<double>(v[0].x, v[0].y, u[0].x, u[0].y, tol, nu2);
+          double* d = rot + 5 * tid;
+          d[0] = o.c; d[1] = o.s; d[2] = o.er; d[3] = o.ei;
+          d[4] = o.on ? 1.0 : 0.0;
+          rotated |= o.on;
+        }
+        __syncthreads();
+        split64_rotate(Xs, ld, K, n, r, rot);
+        __syncthreads();
+        buf ^= 1;
+      }
+      sweeps = sweep + 1;
+      if (!__syncthreads_or(rotated)) break;  // the same answer in every CTA
+    }
+    for (int j = warp; j < n; j += S64_W)
+      for (int r = lane; S64_C * r + rank < m; r += 32) Xg[S64_C * r + rank + (size_t)m * j] = Xs[r + ld * j];
+    cl.sync();
+    sorted_norms<S64_NT, double2>(Xg, m, m, n, s_sig, s_perm);  // the same in every CTA
+    if (tid == 0) {
+      const int k = min(tail_rule(s_sig, n, p.cutoff), min(cap, min(m, n)));
+      double disc = 0;
+      for (int j = k; j < n; j++) disc += s_sig[j] * s_sig[j];
+      s_k = k;
+      if (rank == 0) {
+        p.task_rank[task] = k;
+        p.task_sweeps[task] += sweeps;
+        p.task_discarded[task] = (float)disc;
+      }
+    }
+    __syncthreads();
+    const int k = s_k;
+    // A' = unit columns (this CTA's rows), B' = A'^H theta' (its columns), both from the FP64 columns
+    for (int j = warp; j < k; j += S64_W) {
+      const double s = s_sig[j], inv = s > 0 ? 1.0 / s : 0.0;
+      const double2* x = Xs + ld * s_perm[j];
+      for (int r = lane; S64_C * r + rank < m; r += 32)
+        A[S64_C * r + rank + (size_t)m * j] = make_float2((float)(x[r].x * inv), (float)(x[r].y * inv));
+    }
+    __syncthreads();  // the product's tiles take the start of the shared memory
+    if (b1 > b0)
+      cta_gemm<S64_NT, 32, double2>(true, false, k, 2 * (b1 - b0), m, Xg, m, s_perm, Tb, m, dyn,
+                                    [&](int r, int col, double2 v) {
+                                      const double s = s_sig[r], inv = s > 0 ? 1.0 / s : 0.0;
+                                      B[r + (size_t)k * (2 * b0 + col)] = make_float2((float)(v.x * inv), (float)(v.y * inv));
+                                    });
+    if (rank == 0 && tid == 0) bond[w + 1] = k;
+    cl.sync();
+  }
+  cl.sync();  // no CTA leaves while another may still read its shared memory
 }
 
 // <Z_site> per circuit in FP32, one CTA per circuit (grid-stride): the
@@ -436,7 +569,8 @@ struct qt_batch {
   float2* d_slab = nullptr;
   int ctas = 0;
   int bucket_elems[4] = {0, 0, 0, 0};  // entries of the largest theta' per bond-cap bucket (0: no circuit in it)
-  int* d_counter = nullptr;  // one counter per layer
+  int* d_counter = nullptr;  // three counters per launch: tasks taken, tasks left to FP64, of those taken
+  int* d_left = nullptr;     // the tasks left to FP64, in the range of their launch
   int counter_cap = 0;
   // the last program (device copies) and its captured graph
   int* d_tc = nullptr;
@@ -462,6 +596,9 @@ struct qt_batch {
     for (int bk = 0; bk < 4; bk++) need = std::max(need, (size_t)ctas * cps[bk] * 4 * bucket_elems[bk]);
     return need;
   }
+  // clusters of the FP64 split of `tasks` tasks: one per eight CTAs of the
+  // slab, an eighth of the chip's SMs at most
+  int split_clusters(int tasks) const { return std::max(1, std::min(tasks, ctas / S64_C)); }
 };
 
 namespace {
@@ -475,7 +612,7 @@ int bucket_of(int cap) { return cap <= 16 ? 0 : cap <= 32 ? 1 : cap <= 64 ? 2 : 
 size_t batch_smem(int bk) {
   static const size_t theta[4] = {33 * 32, 65 * 64, 129 * 128, 25600};
   return std::max(theta[bk] * sizeof(float2),
-                  std::max(cta_gemm_smem<double2>(32), cta_gemm_smem<float2>(bk == 0 ? 32 : 64)));
+                  cta_gemm_smem<float2>(bk == 0 ? 32 : 64));
 }
 
 typedef void (*layer_fn)(BatchArgs);
@@ -503,8 +640,9 @@ static void batch_free_program(qt_batch* b) {
   b->graph = nullptr;
   cudaFree(b->d_tc); cudaFree(b->d_ts); cudaFree(b->d_tg);
   cudaFree(b->d_rank); cudaFree(b->d_sweeps); cudaFree(b->d_disc); cudaFree(b->d_grank); cudaFree(b->d_cert);
+  cudaFree(b->d_left);
   b->d_tc = b->d_ts = nullptr; b->d_tg = nullptr; b->d_rank = b->d_sweeps = nullptr; b->d_disc = nullptr;
-  b->d_grank = b->d_cert = nullptr;
+  b->d_grank = b->d_cert = b->d_left = nullptr;
   b->ntask_cap = 0;
 }
 
@@ -634,7 +772,8 @@ extern "C" int qt_batch_run(qt_handle* h, qt_batch* b, int nlayers, const int* l
               cudaMalloc(&b->d_sweeps, sizeof(int) * ntask) == cudaSuccess &&
               cudaMalloc(&b->d_disc, sizeof(float) * ntask) == cudaSuccess &&
               cudaMalloc(&b->d_grank, sizeof(int) * ntask) == cudaSuccess &&
-              cudaMalloc(&b->d_cert, sizeof(int) * ntask) == cudaSuccess;
+              cudaMalloc(&b->d_cert, sizeof(int) * ntask) == cudaSuccess &&
+              cudaMalloc(&b->d_left, sizeof(int) * ntask) == cudaSuccess;
     if (!ok) {
       cudaGetLastError();
       return qt_fail(h, QT_ENOMEM, "batch_run: device allocation failed");
@@ -652,7 +791,9 @@ extern "C" int qt_batch_run(qt_handle* h, qt_batch* b, int nlayers, const int* l
   }
   if (b->counter_cap < nseg) {
     cudaFree(b->d_counter);
-    if (cudaMalloc(&b->d_counter, sizeof(int) * std::max(nseg, 1)) != cudaSuccess)
+    b->d_counter = nullptr;
+    b->counter_cap = 0;
+    if (cudaMalloc(&b->d_counter, sizeof(int) * 3 * std::max(nseg, 1)) != cudaSuccess)
       return qt_fail(h, QT_ENOMEM, "batch_run: counter allocation failed");
     b->counter_cap = nseg;
   }
@@ -676,19 +817,25 @@ extern "C" int qt_batch_run(qt_handle* h, qt_batch* b, int nlayers, const int* l
     if (b->bucket_elems[bk])
       QT_CHECK_CUDA(h, cudaFuncSetAttribute((const void*)layer_kernel(b->threads[bk], bk),
                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)batch_smem(bk)));
+  QT_CHECK_CUDA(h, cudaFuncSetAttribute((const void*)batch_split64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)S64_SMEM));
   auto launch_all = [&]() -> int {
-    QT_CHECK_CUDA(h, cudaMemsetAsync(b->d_counter, 0, sizeof(int) * std::max(nseg, 1), h->stream));
+    QT_CHECK_CUDA(h, cudaMemsetAsync(b->d_counter, 0, sizeof(int) * 3 * std::max(nseg, 1), h->stream));
     for (int sg = 0; sg < nseg; sg++) {
       const int bk = seg_bucket[sg];
       BatchArgs al = a;
       al.task_begin = seg_begin[sg];
       al.task_end = seg_end[sg];
-      al.counter = b->d_counter + sg;
+      al.counter = b->d_counter + 3 * sg;
+      al.nleft = al.counter + 1;
+      al.left = b->d_left + seg_begin[sg];
       const int grid = std::min(dev_sms * b->cps[bk], seg_end[sg] - seg_begin[sg]);
       al.slab_elems = b->bucket_elems[bk];
       al.smem_elems = (int)(batch_smem(bk) / sizeof(float2));
       const layer_fn batch_layer_kernel_fn = layer_kernel(b->threads[bk], bk);
       QT_LAUNCH(h, batch_layer_kernel_fn, grid, b->threads[bk], batch_smem(bk), al);
+      al.counter += 2;
+      QT_LAUNCH(h, batch_split64_kernel, S64_C * b->split_clusters(seg_end[sg] - seg_begin[sg]), S64_NT, S64_SMEM, al);
     }
     return QT_OK;
   };

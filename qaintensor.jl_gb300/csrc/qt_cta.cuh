@@ -305,67 +305,6 @@ __device__ int cta_jacobi(float2* X, int ld, int m, int n, double tol, double nu
   return sweeps;
 }
 
-// FP64 columns: the sums of a round's pairs go to shared memory, one lane
-// each evaluates the angles of 32 pairs together (a warp instruction takes
-// the same 16 cycles of the two FP64 lanes whether one pair or 32 ride on
-// it), and the warps rotate.  ws: 4 n doubles.
-template <int NT>
-__device__ int cta_jacobi64(double2* X, int ld, int m, int n, double tol, double nu2, int max_sweeps, double* ws) {
-  constexpr int W = NT / 32;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, pairs = n / 2;
-  int sweeps = 0;
-  if (n < 2) return 0;
-  double *sum = ws, *rot = ws + 4 * pairs;
-  for (int sweep = 0; sweep < max_sweeps; sweep++) {
-    bool rotated = false;
-    for (int r = 0; r < n - 1; r++) {
-      for (int q = warp; q < pairs; q += W) {
-        int pc, qc;
-        cta_tourney(r, q, n, pc, qc);
-        const double2 *xp = X + (size_t)ld * pc, *xq = X + (size_t)ld * qc;
-        double v[4] = {0, 0, 0, 0};
-        for (int i = lane; i < m; i += 32) {
-          const double2 u = xp[i], w = xq[i];
-          v[0] = fma(u.x, u.x, fma(u.y, u.y, v[0]));
-          v[1] = fma(w.x, w.x, fma(w.y, w.y, v[1]));
-          v[2] = fma(u.x, w.x, fma(u.y, w.y, v[2]));
-          v[3] = fma(u.x, w.y, fma(-u.y, w.x, v[3]));
-        }
-        const double s = cta_pair_sums<1>(v);
-        if ((lane & 7) == 0) sum[4 * q + (lane >> 3)] = s;
-      }
-      __syncthreads();
-      for (int q = tid; q < pairs; q += NT) {
-        const cta_rotation<double> o = cta_angle64<double>(sum[4 * q], sum[4 * q + 1], sum[4 * q + 2], sum[4 * q + 3],
-                                                           tol, nu2);
-        rot[4 * q] = o.on ? o.c : 2.0;  // 2: left alone
-        rot[4 * q + 1] = o.s;
-        rot[4 * q + 2] = o.er;
-        rot[4 * q + 3] = o.ei;
-      }
-      __syncthreads();
-      for (int q = warp; q < pairs; q += W) {
-        const double c = rot[4 * q];
-        if (c == 2.0) continue;
-        rotated = true;
-        const double s = rot[4 * q + 1], er = rot[4 * q + 2], ei = rot[4 * q + 3];
-        int pc, qc;
-        cta_tourney(r, q, n, pc, qc);
-        double2 *xp = X + (size_t)ld * pc, *xq = X + (size_t)ld * qc;
-        for (int i = lane; i < m; i += 32) {
-          const double2 u = xp[i], v = xq[i];
-          xp[i] = mk(c * u.x - s * (er * v.x + ei * v.y), c * u.y - s * (er * v.y - ei * v.x));
-          xq[i] = mk(s * (er * u.x - ei * u.y) + c * v.x, s * (er * u.y + ei * u.x) + c * v.y);
-        }
-      }
-      __syncthreads();
-    }
-    sweeps = sweep + 1;
-    if (!__syncthreads_or(rotated)) break;
-  }
-  return sweeps;
-}
-
 // m <= 32 RMAX.
 template <int NT, int RMAX>
 __device__ int cta_jacobi_any(float2* X, int ld, int m, int n, double tol, double nu2, int max_sweeps) {
@@ -379,7 +318,7 @@ __device__ int cta_jacobi_any(float2* X, int ld, int m, int n, double tol, doubl
 }
 
 // ---------------------------------------------------------------------------
-// op(A) op(B) (M x N), one CTA, accumulated in the elements' precision
+// op(A) op(B) (M x N), one CTA, in the precision of C (operands widened as read)
 // ---------------------------------------------------------------------------
 //
 // TILE x TILE outputs at a time, 16 deep, through shared memory (both
@@ -391,9 +330,9 @@ constexpr int CTA_GK = 16;
 template <typename C>
 constexpr size_t cta_gemm_smem(int tile) { return 2 * (size_t)CTA_GK * (tile + 1) * sizeof(C); }
 
-template <int NT, int TILE, typename C, typename F>
-__device__ void cta_gemm_tile(bool conj_a, bool conj_b, int M, int N, int K, const C* A, int lda, const int* perm_a,
-                              const C* B, int ldb, void* sm, F store) {
+template <int NT, int TILE, typename C, typename EA, typename EB, typename F>
+__device__ void cta_gemm_tile(bool conj_a, bool conj_b, int M, int N, int K, const EA* A, int lda, const int* perm_a,
+                              const EB* B, int ldb, void* sm, F store) {
   constexpr int TX = (NT <= 512 || TILE < 32) ? 16 : 32, TY = NT / TX;
   constexpr int RM = TILE / TX, RN = TILE / TY;
   static_assert(RM >= 1 && RN >= 1, "tile too small for the CTA");
@@ -412,12 +351,14 @@ __device__ void cta_gemm_tile(bool conj_a, bool conj_b, int M, int N, int K, con
           C v = czero<C>();
           const int mi = conj_a ? idx / CTA_GK : idx % TILE, ka = conj_a ? idx % CTA_GK : idx / TILE;
           if (m0 + mi < M && k0 + ka < K)
-            v = conj_a ? cconj(A[(k0 + ka) + (size_t)lda * (perm_a ? perm_a[m0 + mi] : m0 + mi)]) : A[(m0 + mi) + (size_t)lda * (k0 + ka)];
+            v = conj_a ? cconj(ccast<C>(A[(k0 + ka) + (size_t)lda * (perm_a ? perm_a[m0 + mi] : m0 + mi)]))
+                       : ccast<C>(A[(m0 + mi) + (size_t)lda * (k0 + ka)]);
           As[ka][mi] = v;
           v = czero<C>();
           const int ni = conj_b ? idx % TILE : idx / CTA_GK, kb = conj_b ? idx / TILE : idx % CTA_GK;
           if (n0 + ni < N && k0 + kb < K)
-            v = conj_b ? cconj(B[(n0 + ni) + (size_t)ldb * (k0 + kb)]) : B[(k0 + kb) + (size_t)ldb * (n0 + ni)];
+            v = conj_b ? cconj(ccast<C>(B[(n0 + ni) + (size_t)ldb * (k0 + kb)]))
+                       : ccast<C>(B[(k0 + kb) + (size_t)ldb * (n0 + ni)]);
           Bs[kb][ni] = v;
         }
         __syncthreads();
@@ -450,9 +391,9 @@ __device__ void cta_gemm_tile(bool conj_a, bool conj_b, int M, int N, int K, con
 // TMAX: the largest tile the caller's shared memory holds (32 or 64).  The
 // 64-wide tile reads shared memory half as often per product; a product of
 // at most 32 rows or columns would leave half of it empty.
-template <int NT, int TMAX, typename C, typename F>
-__device__ void cta_gemm(bool conj_a, bool conj_b, int M, int N, int K, const C* A, int lda, const int* perm_a,
-                         const C* B, int ldb, void* sm, F store) {
+template <int NT, int TMAX, typename C, typename EA, typename EB, typename F>
+__device__ void cta_gemm(bool conj_a, bool conj_b, int M, int N, int K, const EA* A, int lda, const int* perm_a,
+                         const EB* B, int ldb, void* sm, F store) {
   if constexpr (TMAX >= 64)
     if (M > 32 && N > 32)
       return cta_gemm_tile<NT, 64, C>(conj_a, conj_b, M, N, K, A, lda, perm_a, B, ldb, sm, store);
