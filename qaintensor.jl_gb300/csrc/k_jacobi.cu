@@ -1773,19 +1773,23 @@ jacobi_sweep32_kernel(float2* __restrict__ xb0, float2* __restrict__ xb1, int64_
     phase(2);  // 1: rebuild + Gram products
     // ---- reduce the row groups in a fixed order: three partial sums of 17
     // groups each, then their sum; the diagonal goes to the solver's D
+    // (stored group-fastest: neighbouring threads hold neighbouring groups, and
+    // the sums start 17 entries apart, so that neither side meets a bank twice;
+    // entry-fastest, every lane of a store met the same bank, 3.8 us a round
+    // from here to the pair solver instead of 1.5)
     float2* red = ps_slab;
     if (act) {
 #pragma unroll
-      for (int e = 0; e < PS_TE; e++) red[(grp * PS_TILES + tile) * PS_TE + e] = acc[e];
+      for (int e = 0; e < PS_TE; e++) red[(tile * PS_TE + e) * PS_NGRP + grp] = acc[e];
     }
     __syncthreads();
     static_assert(PS_NGRP == 3 * 17, "three partial sums of 17 row groups");
     if (t < 3 * PS_TILES * PS_TE) {
       const int ent = t / 3, part = t % 3;
-      const float2* rp0 = red + (size_t)(part * 17) * PS_TILES * PS_TE + ent;
+      const float2* rp0 = red + ent * PS_NGRP + part * 17;
       float2 v = rp0[0];
 #pragma unroll
-      for (int gg = 1; gg < 17; gg++) v = cadd(v, rp0[(size_t)gg * PS_TILES * PS_TE]);
+      for (int gg = 1; gg < 17; gg++) v = cadd(v, rp0[gg]);
       psum[part][ent] = v;
     }
     __syncthreads();
