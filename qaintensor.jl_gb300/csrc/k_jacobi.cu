@@ -1448,35 +1448,52 @@ struct sweep_solver {
   float2 W[2][JC][JC + 1];
 };
 
-// named barrier of the 256 solver threads (warps 0-7)
-__device__ inline void solver_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+constexpr int SOLVER_THREADS = JC / 2 * JC;  // warps 0-3
+__device__ inline void solver_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
-// The scaled pair solver, run by warps 0-7 alone (the caller's other warps
-// skip it and wait at its next block barrier): thread (x, y) computes the
-// rotation of y's pair itself (the two half-warps compute the same 16,
-// bit-identically) and takes x's from lane x by shuffle, then updates
-// Ghat[x][y] and Wt[x][y] into the other buffer -- one named barrier per
-// inner round.  An inner round in which no pair needs a rotation is skipped
-// by every warp alike (a warp vote over the same 16 decisions).  Same
-// iteration as diagonalise_scaled2; the rotation is evaluated with the
-// special-function unit's square roots and reciprocals (a few ulps: the
-// rotation stays unitary to FP32 rounding, and the one-sided iteration
-// re-measures every pair from the data in the next round anyway).
+// The scaled pair solver, run by warps 0-3 alone (the caller's other warps
+// skip it and wait at its next block barrier).  Its inner rounds are a serial
+// chain (three values from shared memory, the rotation, the update, a
+// barrier), so what counts is the chain's length and how many instructions
+// share a scheduler with it: thread (k, y) computes the rotation of y's pair
+// itself (every half-warp computes the same 16, bit-identically), takes those
+// of the k-th pair (x, x') by shuffle, and updates Ghat[x][y], Ghat[x'][y] and
+// two rows of Wt into the other buffer from values loaded before the rotation
+// is known; one warp per scheduler, one named barrier per inner round.  An
+// inner round in which no pair needs a rotation is skipped by every warp alike
+// (a warp vote over the same 16 decisions).  Same iteration as
+// diagonalise_scaled2; the rotation is evaluated with the special-function
+// unit's square roots and reciprocals (a few ulps: the rotation stays unitary
+// to FP32 rounding, and the one-sided iteration re-measures every pair from
+// the data in the next round anyway).  A round of the 74 x 102 split takes 7.7 us
+// here, of a wide one late in the sweeps 3.6; with one thread per entry of the
+// Gram (eight warps) and loads behind the rotation 11.0 and 6.2.
+// The finished unitary goes to wout (JC x JC).
 __device__ int diagonalise_lanes(sweep_solver& sh, const int* col, float tol_inner, float nu2, int max_inner,
-                                 int* buf_out) {
-  const int t = threadIdx.x, x = (t >> 4) & 15, y = t & 15;
-  if (t >= NGRAM) return 0;  // warps 8-15
+                                 float2* __restrict__ wout) {
+  const int t = threadIdx.x, k = t >> 4, y = t & 15;
+  if (t >= SOLVER_THREADS) return 0;  // warps 4-15
   const float tol2 = tol_inner * tol_inner;
+  const unsigned live = __ballot_sync(0xffffffffu, col[y] >= 0);  // bit c of the low half: column c is there
   int cur = 0, sweep = 0;
   for (; sweep < max_inner; sweep++) {
     bool rotated_any = false;
     for (int ir = 0; ir < JC - 1; ir++) {
-      const int yp = inner_partner(ir, y), xp = inner_partner(ir, x);
+      int yp = 2 * ir - y;
+      yp = yp < 0 ? yp + (JC - 1) : yp >= JC - 1 ? yp - (JC - 1) : yp;
+      yp = y == JC - 1 ? ir : y == ir ? JC - 1 : yp;
+      int x = ir + k, xp = ir - k;
+      x = x >= JC - 1 ? x - (JC - 1) : x;
+      xp = k == 0 ? JC - 1 : xp < 0 ? xp + (JC - 1) : xp;
       const int p = min(y, yp), q = max(y, yp);
       const float a = sh.d[cur][p], b = sh.d[cur][q];
       const float2 gs = sh.G[cur][p][q];
+      const float2 g_xy = sh.G[cur][x][y], g_xq = sh.G[cur][x][yp];
+      const float2 g_py = sh.G[cur][xp][y], g_pq = sh.G[cur][xp][yp];
+      const float2 w0_y = sh.W[cur][k][y], w0_q = sh.W[cur][k][yp];
+      const float2 w1_y = sh.W[cur][k + JC / 2][y], w1_q = sh.W[cur][k + JC / 2][yp];
       const float ags2 = gs.x * gs.x + gs.y * gs.y;
-      const bool rotp = col[p] >= 0 && col[q] >= 0 && a > nu2 && b > nu2 && ags2 > tol2;
+      const bool rotp = ((live >> p) & (live >> q) & 1) && a > nu2 && b > nu2 && ags2 > tol2;
       if (!__any_sync(0xffffffffu, rotp)) continue;  // the same vote in every solver warp
       rotated_any = true;
       float2 jpp = make_float2(1.f, 0.f), jqp = make_float2(0.f, 0.f), jpq = jqp, jqq = jpp;
@@ -1500,41 +1517,43 @@ __device__ int diagonalise_lanes(sweep_solver& sh, const int* col, float tol_inn
         jpq = make_float2(sn * e.x * fba, sn * e.y * fba);   //  s e sqrt(a/b')
         jqq = make_float2(c * fb, 0.f);
       }
-      // column y of Jt: rows y and y'
+      // column y of Jt: rows y (real) and y'
       const bool low = y == p;
       const float2 jyy = low ? jpp : jqq, jpy = low ? jqp : jpq;
-      // column x of Jt from lane x (which holds y == x)
-      float2 jxx, jpx;
-      jxx.x = __shfl_sync(0xffffffffu, jyy.x, x);
-      jxx.y = __shfl_sync(0xffffffffu, jyy.y, x);
-      jpx.x = __shfl_sync(0xffffffffu, jpy.x, x);
-      jpx.y = __shfl_sync(0xffffffffu, jpy.y, x);
-      if (x == y) sh.d[cur ^ 1][y] = low ? a2 : b2;
-      float2 gnew = make_float2(0.f, 0.f);
-      if (xp == y && x != y) {
-        const bool rotated = jxx.x != 1.f || jxx.y != 0.f || jpx.x != 0.f || jpx.y != 0.f;
-        if (!rotated) gnew = sh.G[cur][x][y];
-      } else if (x != y) {
-        const float2 g_xy = sh.G[cur][x][y], g_xq = sh.G[cur][x][yp];
-        const float2 g_py = sh.G[cur][xp][y], g_pq = sh.G[cur][xp][yp];
-        const float2 hx = cadd(cmul(g_xy, jyy), cmul(g_xq, jpy));
-        const float2 hp = cadd(cmul(g_py, jyy), cmul(g_pq, jpy));
-        gnew = cadd(cmul(cconj(jxx), hx), cmul(cconj(jpx), hp));
+      // columns x and x' of Jt from lanes x and x' (which hold y == x, x')
+      const float2 jxx = make_float2(__shfl_sync(0xffffffffu, jyy.x, x), 0.f);
+      const float2 jpx = make_float2(__shfl_sync(0xffffffffu, jpy.x, x), __shfl_sync(0xffffffffu, jpy.y, x));
+      const float2 jXX = make_float2(__shfl_sync(0xffffffffu, jyy.x, xp), 0.f);
+      const float2 jPX = make_float2(__shfl_sync(0xffffffffu, jpy.x, xp), __shfl_sync(0xffffffffu, jpy.y, xp));
+      if (k == 0) sh.d[cur ^ 1][y] = low ? a2 : b2;
+      const float2 hx = cadd(cmul(g_xy, jyy), cmul(g_xq, jpy));
+      const float2 hp = cadd(cmul(g_py, jyy), cmul(g_pq, jpy));
+      float2 gx = cadd(cmul(cconj(jxx), hx), cmul(cconj(jpx), hp));
+      float2 gp = cadd(cmul(cconj(jXX), hp), cmul(cconj(jPX), hx));
+      const float2 zero = make_float2(0.f, 0.f);
+      if (y == x) {
+        gx = zero;
+        gp = jXX.x != 1.f || jPX.x != 0.f || jPX.y != 0.f ? zero : g_py;
+      } else if (y == xp) {
+        gx = jxx.x != 1.f || jpx.x != 0.f || jpx.y != 0.f ? zero : g_xy;
+        gp = zero;
       }
-      sh.G[cur ^ 1][x][y] = gnew;
-      const float2 w_xy = sh.W[cur][x][y], w_xq = sh.W[cur][x][yp];
-      sh.W[cur ^ 1][x][y] = cadd(cmul(w_xy, jyy), cmul(w_xq, jpy));
+      sh.G[cur ^ 1][x][y] = gx;
+      sh.G[cur ^ 1][xp][y] = gp;
+      sh.W[cur ^ 1][k][y] = cadd(cmul(w0_y, jyy), cmul(w0_q, jpy));
+      sh.W[cur ^ 1][k + JC / 2][y] = cadd(cmul(w1_y, jyy), cmul(w1_q, jpy));
       cur ^= 1;
       solver_sync();
     }
     if (!rotated_any) break;  // every solver warp took the same votes
   }
-  {
+#pragma unroll
+  for (int h = 0; h < 2; h++) {  // the rows this thread updated itself
+    const int x = k + h * (JC / 2);
     const float d0 = sh.d0[x];
-    sh.W[cur][x][y] = d0 > 0.f ? cscale(sh.W[cur][x][y], sqrtf(sh.d[cur][y]) * rsqrtf(d0))
-                               : make_float2(x == y ? 1.f : 0.f, 0.f);
+    __stcg(wout + x * JC + y, d0 > 0.f ? cscale(sh.W[cur][x][y], sqrtf(sh.d[cur][y]) * rsqrtf(d0))
+                                       : make_float2(x == y ? 1.f : 0.f, 0.f));
   }
-  *buf_out = cur;
   return sweep + (sweep < max_inner ? 1 : 0);
 }
 
@@ -1881,11 +1900,9 @@ jacobi_sweep32_kernel(float2* __restrict__ xb0, float2* __restrict__ xb1, int64_
     }
     phase(3);  // 2: reduction, scaled Gram, test
     if (any_rot) {
-      int buf = 0;
-      const int inner = diagonalise_lanes(sh, col, tol_inner, nu2, max_inner, &buf);
+      const int inner = diagonalise_lanes(sh, col, tol_inner, nu2, max_inner,
+                                          wbuf + (size_t)(g & 1) * pairs * NGRAM + (size_t)q * NGRAM);
       if (t == 0 && hf == 0) atomicAdd(&flags[QT_FLAG_INNER], inner);
-      // each solver thread stores the entry it finished itself
-      if (owner) __stcg(wbuf + (size_t)(g & 1) * pairs * NGRAM + (size_t)q * NGRAM + t, sh.W[buf][i][j]);
     }
     phase(4);  // 3: pair solver
     // ---- publish round g
