@@ -1401,6 +1401,14 @@ pair_apply32_kernel(float2* __restrict__ X, int64_t ldx, int mm, float2* __restr
 // of its rows) in gx and its round in xflag, waits (bounded) for the other's,
 // and both add the two partials in the same order.  Both then run the same
 // pair solver on the same Gram and reach the same unitary, bit for bit.
+//
+// What bounds a round of up to 512 rows: latency, about 15 us of it at any size,
+// half of that the pair solver's chain.  So the rest is kept short: the decision,
+// the unitary and the rows of both source blocks are loaded at once, before it
+// is known which are needed; V's rows are rebuilt by warps that have no rows of
+// X, or loaded ahead of the Gram products; one release publishes the round.
+// Measured (us a round, 74 x 102 split / 240 x 160 late in the sweeps): 5.4 / 3.7
+// -> 4.1 / 2.5 from the end of the wait to the end of the products.
 
 constexpr int PS_SLAB = 256;                 // rows per slab
 constexpr int PS_LDS = JC + 2;               // slab row stride in float2 (16-byte aligned rows)
@@ -1573,7 +1581,7 @@ jacobi_sweep32_kernel(float2* __restrict__ xb0, float2* __restrict__ xb1, int64_
   __shared__ float2 psum[3][PS_TILES * PS_TE];
   __shared__ float2 gram[NGRAM];
   __shared__ sweep_solver sh;
-  __shared__ int col[JC], scol[2][JC], srcq[2], sside[2], srot[2];
+  __shared__ int col[JC];
   __shared__ int any_rot, bad, offmax_blk, offbig_blk, offkept_blk;
   const int H = halves, t = threadIdx.x, q = blockIdx.x / H, hf = blockIdx.x % H, pairs = gridDim.x / H,
             R = nb - 1;
@@ -1612,6 +1620,16 @@ jacobi_sweep32_kernel(float2* __restrict__ xb0, float2* __restrict__ xb1, int64_
     phase(0);
     int bi, bj;
     tournament(r, q, nb, bi, bj);
+    // ---- what does not depend on other CTAs: this round's columns, and where
+    // this half's block was in round g - 1 (pair qq, first or second block, with partner blocks a2 and b2)
+    pair_columns(r, q, nb, nn, col);
+    if (t == 0) { any_rot = 0; bad = 0; offmax_blk = 0; offbig_blk = 0; offkept_blk = 0; }
+    const int blk = h == 0 ? bi : bj;
+    int srcq = 0, sside = 0, a2 = blk, b2 = blk;
+    if (prev) {
+      pair_of(rp, blk, nb, srcq, sside);
+      tournament(rp, srcq, nb, a2, b2);
+    }
     // ---- wait for the round g - 1 CTAs this round depends on
     int gave_up = 0;
     if (stall && q == 0 && t == 0 && r == 0) {
@@ -1655,53 +1673,58 @@ jacobi_sweep32_kernel(float2* __restrict__ xb0, float2* __restrict__ xb1, int64_
     }
     if (__syncthreads_or(gave_up)) return;
     phase(1);  // 0: waits
-    pair_columns(r, q, nb, nn, col);
-    if (t == 0) { any_rot = 0; bad = 0; offmax_blk = 0; offbig_blk = 0; offkept_blk = 0; }
-    if (prev && t < 2) {
-      int qq, s;
-      pair_of(rp, t == 0 ? bi : bj, nb, qq, s);
-      srcq[t] = qq;
-      sside[t] = s;
-      srot[t] = __ldcg(rotbuf + (size_t)((g - 1) & 1) * pairs + qq);
-    }
-    if (!prev && t < 2) srot[t] = 0;
-    __syncthreads();
-    if (t < 2 * JC) {  // source columns of each half: the round g - 1 pair, or the block itself
-      const int hh = t / JC, c = t % JC;
-      int gc;
-      if (srot[hh]) {
-        int a2, b2;
-        tournament(rp, srcq[hh], nb, a2, b2);
-        gc = c < JW ? a2 * JW + c : b2 * JW + (c - JW);
-      } else {
-        gc = c < JW ? (hh == 0 ? bi : bj) * JW + c : -1;
-      }
-      scol[hh][c] = gc < nn ? gc : -1;
-    }
-    if (t < 2 * JC * JW) {
-      const int hh = t / (JC * JW), k = (t / JW) % JC, c = t % JW;
-      if (srot[hh])
-        wsub[hh][k][c] = __ldcg(wbuf + (size_t)((g - 1) & 1) * pairs * NGRAM + (size_t)srcq[hh] * NGRAM + k * JC +
-                                sside[hh] * JW + c);
-    }
-    __syncthreads();
     const float2* __restrict__ src = prev ? (((g - 1) & 1) ? xb1 : xb0) : ((g & 1) ? xb1 : xb0);
     float2* __restrict__ dst = (g & 1) ? xb1 : xb0;
-    const bool hrot = srot[h] != 0;
+    const float2* __restrict__ vsrc = ((g - 1) & 1) ? vb1 : vb0;
+    float2* __restrict__ vdst = (g & 1) ? vb1 : vb0;
+    const bool vwork = prev && vb0 != nullptr;
+    // V's rows go to the warps in reverse order: those whose X rows lie past
+    // the matrix (only one slab then) take them instead, at the same time
+    const int vrow = vrow_lo + (PS_SLAB - 32 - (lr & ~31)) + (lr & 31);
+    const bool vfirst = vwork && nslab <= 1 && row_lo + (lr & ~31) >= row_hi;
     // column indices stay in shared memory (warp-uniform broadcast reads)
-    const int* sc = scol[h];
     const int* oc = col + h * JW;
-    // ---- rebuild the rows slab by slab; Gram products on the previous slab meanwhile
+    // ---- the first rows of both source blocks, the unitary and whether there
+    // is one, all under one latency
     float2 xr[JC];
+    bool hrot = false;
+    {
+      const int rr = vfirst ? vrow : row_lo + lr, lim = vfirst ? vrow_hi : row_hi;
+      const float2* __restrict__ M = (vfirst ? vsrc : src) + rr;
+      const int64_t ld = vfirst ? ldv : ldx;
+      const size_t slot = (size_t)((g - 1) & 1) * pairs + srcq;
+      const int tt = t & (PS_SLAB - 1);
+      int rotated = 0;
+      float2 wv = make_float2(0.f, 0.f);
+      if (prev) {
+        rotated = __ldcg(rotbuf + slot);
+        // (left over from an earlier round where the pair did not rotate, and not used then)
+        if (tt < JC * JW) wv = __ldcg(wbuf + slot * NGRAM + (tt / JW) * JC + sside * JW + tt % JW);
+      }
+#pragma unroll
+      for (int k = 0; k < JC; k++) {
+        const int gc = (k < JW ? a2 : b2) * JW + k % JW;
+        xr[k] = (gc < nn && rr < lim && (k < JW || prev)) ? __ldcg(M + ld * gc) : make_float2(0.f, 0.f);
+      }
+      hrot = rotated != 0;
+      if (!hrot) {
+        if (sside)
+#pragma unroll
+          for (int k = 0; k < JW; k++) xr[k] = xr[k + JW];
+        a2 = blk;
+      }
+      if (tt < JC * JW) wsub[h][tt / JW][tt % JW] = wv;
+    }
+    __syncthreads();
+    // ---- rebuild the rows slab by slab; Gram products on the previous slab meanwhile
     auto load_row = [&](const float2* __restrict__ M, int64_t ld, int lim, int rr) {
+#pragma unroll
+      for (int k = 0; k < JW; k++)
+        xr[k] = (a2 * JW + k < nn && rr < lim) ? __ldcg(M + rr + ld * (a2 * JW + k)) : make_float2(0.f, 0.f);
       if (hrot) {
 #pragma unroll
-        for (int k = 0; k < JC; k++)
-          xr[k] = (sc[k] >= 0 && rr < lim) ? __ldcg(M + rr + ld * sc[k]) : make_float2(0.f, 0.f);
-      } else {
-#pragma unroll
         for (int k = 0; k < JW; k++)
-          xr[k] = (sc[k] >= 0 && rr < lim) ? __ldcg(M + rr + ld * sc[k]) : make_float2(0.f, 0.f);
+          xr[JW + k] = (b2 * JW + k < nn && rr < lim) ? __ldcg(M + rr + ld * (b2 * JW + k)) : make_float2(0.f, 0.f);
       }
     };
     auto rebuild = [&](float2* out) {
@@ -1748,14 +1771,25 @@ jacobi_sweep32_kernel(float2* __restrict__ xb0, float2* __restrict__ xb1, int64_
 #pragma unroll
       for (int c = 0; c < JW; c += 2) sp[c / 2] = make_float4(o[c].x, o[c].y, o[c + 1].x, o[c + 1].y);
     };
+    auto build_vrow = [&](int rr) {
+      if (rr - (lr & 31) >= vrow_hi) return;  // the whole warp
+      float2 o[JW];
+      rebuild(o);
+      if (rr < vrow_hi) {
+#pragma unroll
+        for (int c = 0; c < JW; c++)
+          if (oc[c] >= 0) __stcg(vdst + rr + ldv * oc[c], o[c]);
+      }
+    };
     float2 acc[PS_TE];
 #pragma unroll
     for (int e = 0; e < PS_TE; e++) acc[e] = make_float2(0.f, 0.f);
-    load_row(src, ldx, row_hi, row_lo + lr);
-    build_slab(0);
+    if (vfirst) build_vrow(vrow);
+    else build_slab(0);
     __syncthreads();
     for (int s = 0; s < nslab; s++) {
       if (s + 1 < nslab) load_row(src, ldx, row_hi, row_lo + (s + 1) * PS_SLAB + lr);
+      else if (vwork && !vfirst) load_row(vsrc, ldv, vrow_hi, vrow);
       if (act) {
         const float2* base = ps_slab + (size_t)(s & 1) * PS_SLAB * PS_LDS;
         const int rows = min(PS_SLAB, row_hi - row_lo - s * PS_SLAB);
@@ -1777,16 +1811,11 @@ jacobi_sweep32_kernel(float2* __restrict__ xb0, float2* __restrict__ xb1, int64_
       __syncthreads();
     }
     // ---- V rows (rotation only)
-    if (prev && vb0) {
-      const float2* __restrict__ vsrc = ((g - 1) & 1) ? vb1 : vb0;
-      float2* __restrict__ vdst = (g & 1) ? vb1 : vb0;
-      for (int rr = vrow_lo + lr; rr < vrow_hi; rr += PS_SLAB) {
+    if (vwork) {
+      if (!vfirst) build_vrow(vrow);
+      for (int rr = vrow + PS_SLAB; rr < vrow_hi; rr += PS_SLAB) {
         load_row(vsrc, ldv, vrow_hi, rr);
-        float2 o[JW];
-        rebuild(o);
-#pragma unroll
-        for (int c = 0; c < JW; c++)
-          if (oc[c] >= 0) __stcg(vdst + rr + ldv * oc[c], o[c]);
+        build_vrow(rr);
       }
     }
     phase(2);  // 1: rebuild + Gram products
@@ -1905,8 +1934,8 @@ jacobi_sweep32_kernel(float2* __restrict__ xb0, float2* __restrict__ xb1, int64_
       if (t == 0 && hf == 0) atomicAdd(&flags[QT_FLAG_INNER], inner);
     }
     phase(4);  // 3: pair solver
-    // ---- publish round g
-    __threadfence();
+    // ---- publish round g (the barrier orders every thread's stores before
+    // thread 0's release, which is cumulative: no fence per thread)
     __syncthreads();
     if (t == 0) st_release_gpu(done + q, g);
   }
