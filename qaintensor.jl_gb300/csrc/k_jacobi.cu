@@ -18,8 +18,9 @@
 //     columns, blocks of four columns passed between CTAs (see the comment
 //     above that kernel);
 //   FP32 storage otherwise: jacobi_sweep32_kernel -- one cooperative launch per
-//     sweep, each round rebuilding its columns from the previous round's
-//     unitaries (see the comment above that kernel);
+//     sweep, or for all sweeps where only a sweep without rotations ends them,
+//     each round rebuilding its columns from the previous round's unitaries
+//     (see the comment above that kernel);
 //   FP32 storage, two launches per round: pair_eig32_kernel (Gram + test +
 //     pair solver) and pair_apply32_kernel (rotation);
 //   FP64 storage, default: pair_round64_kernel -- one launch per round, a
@@ -1565,16 +1566,20 @@ __device__ int diagonalise_lanes(sweep_solver& sh, const int* col, float tol_inn
   return sweep + (sweep < max_inner ? 1 : 0);
 }
 
-// One sweep (rounds g0 .. g0 + nb - 2).  xb[0] is X itself, xb[1] a scratch
-// copy of its shape (likewise vb for V); wbuf holds 2 x pairs unitaries,
-// rotbuf 2 x pairs decisions, done[pairs] the completed round of each CTA.
+// Sweeps of nb - 1 rounds from round g0 on: nsweeps of them at most, ending with
+// the first that rotates nothing (one sweep only where the caller has a rule
+// of its own for the end: MULTI = false, as the code for more costs a round 2 %).
+// xb[0] is X itself, xb[1] a scratch copy of its shape (likewise vb for V);
+// wbuf holds 2 x pairs unitaries, rotbuf 2 x pairs decisions, done[pairs] the
+// completed round of each CTA.
+template <bool MULTI>
 __global__ void __launch_bounds__(NTG, 1)
 jacobi_sweep32_kernel(float2* __restrict__ xb0, float2* __restrict__ xb1, int64_t ldx, int mm,
                       float2* __restrict__ vb0, float2* __restrict__ vb1, int64_t ldv, int nn, int nb, int g0,
                       int has_prev, double tol, float tol_inner, double nu_rel2, const double* __restrict__ xnorm2,
                       float2* __restrict__ wbuf, int* __restrict__ rotbuf, int* __restrict__ done,
-                      int* __restrict__ flags, int max_inner, float keep2, float* __restrict__ dnorm,
-                      unsigned long long* phase_ns, int spin, int stall, int halves, int row_mid, int vrow_mid,
+                      int* __restrict__ flags, int max_inner, int max_inner0, int nsweeps, float keep2,
+                      float* __restrict__ dnorm, unsigned long long* phase_ns, int spin, int stall, int halves, int row_mid, int vrow_mid,
                       float2* __restrict__ gx, int* __restrict__ xflag) {
   extern __shared__ __align__(16) float2 ps_slab[];  // [2][PS_SLAB][PS_LDS]
   __shared__ __align__(16) float2 wsub[2][JC][JW];    // 16x8 unitary blocks that rebuild the two blocks
@@ -1593,6 +1598,7 @@ jacobi_sweep32_kernel(float2* __restrict__ xb0, float2* __restrict__ xb1, int64_
   rotbuf += (size_t)hf * 2 * pairs;
   if (hf) { phase_ns = nullptr; dnorm = nullptr; }  // half 0 reports for the pair
   __shared__ unsigned long long tp;
+  int swept = 0;  // thread 0: what this CTA has to say about this sweep
   auto phase = [&](int ph) {  // optional diagnostics: time per phase into phase_ns[ph - 1]
     if (phase_ns && t == 0) {
       unsigned long long tn;
@@ -1612,9 +1618,10 @@ jacobi_sweep32_kernel(float2* __restrict__ xb0, float2* __restrict__ xb1, int64_
   int ti = 0, tj = 0;
   if (act) ps_tile(tile, ti, tj);
   const int nslab = (row_hi - row_lo + PS_SLAB - 1) / PS_SLAB;
-  for (int r = 0; r < R; r++) {
-    const int g = g0 + r;
-    const bool prev = r > 0 || has_prev;
+  for (int rs = 0; rs < (MULTI ? R * nsweeps : R); rs++) {
+    const int r = MULTI ? rs % R : rs, sweep = MULTI ? rs / R : 0;
+    const int g = g0 + rs;
+    const bool prev = rs > 0 || has_prev;
     const int rp = r > 0 ? r - 1 : R - 1;  // round (within its sweep) of g - 1
     const int rpp = (r + 2 * R - 2) % R;   // ... of g - 2
     phase(0);
@@ -1632,7 +1639,7 @@ jacobi_sweep32_kernel(float2* __restrict__ xb0, float2* __restrict__ xb1, int64_
     }
     // ---- wait for the round g - 1 CTAs this round depends on
     int gave_up = 0;
-    if (stall && q == 0 && t == 0 && r == 0) {
+    if (stall && q == 0 && t == 0 && rs == 0) {
       // test hook (QT_JACOBI_STALL_TEST): a bounded wait on a status word that
       // nothing sets, which must end in QT_ETIMEOUT with the context usable
       int it = 0;
@@ -1929,7 +1936,7 @@ jacobi_sweep32_kernel(float2* __restrict__ xb0, float2* __restrict__ xb1, int64_
     }
     phase(3);  // 2: reduction, scaled Gram, test
     if (any_rot) {
-      const int inner = diagonalise_lanes(sh, col, tol_inner, nu2, max_inner,
+      const int inner = diagonalise_lanes(sh, col, tol_inner, nu2, sweep < 2 ? max_inner0 : max_inner,
                                           wbuf + (size_t)(g & 1) * pairs * NGRAM + (size_t)q * NGRAM);
       if (t == 0 && hf == 0) atomicAdd(&flags[QT_FLAG_INNER], inner);
     }
@@ -1938,6 +1945,37 @@ jacobi_sweep32_kernel(float2* __restrict__ xb0, float2* __restrict__ xb1, int64_
     // thread 0's release, which is cumulative: no fence per thread)
     __syncthreads();
     if (t == 0) st_release_gpu(done + q, g);
+    if (!MULTI) continue;
+    // ---- several sweeps in this launch: the end of one waits (bounded) until
+    // every CTA has said whether it rotated (1) or met a non-finite value
+    // (65536), and a sweep without the first or with the second is the last.
+    // Sweep s adds up in slot s % 3; CTA 0 clears the next slot before it
+    // arrives: whoever read that slot two sweeps ago has arrived since.
+    if (t == 0) swept = (r > 0 ? swept : 0) | (any_rot ? 1 : 0) | (bad ? 65536 : 0);
+    if (r < R - 1) continue;
+    int stop = 0;
+    gave_up = 0;
+    if (t == 0) {
+      int* count = flags + QT_FLAG_SWEPT;
+      if (swept) atomicAdd(count + sweep % 3, swept);
+      if (blockIdx.x == 0) atomicExch(count + (sweep + 1) % 3, 0);
+      __threadfence();
+      atomicAdd(flags + QT_FLAG_ARRIVED, 1);
+      int it = 0;
+      for (; it < spin; it++) {
+        if (ld_acquire_gpu(flags + QT_FLAG_ARRIVED) >= (sweep + 1) * (int)gridDim.x) break;
+        if ((it & 7) == 7 && *(volatile int*)(flags + QT_FLAG_ABORT)) { it = spin; break; }
+        __nanosleep(64);
+      }
+      if (it >= spin) { gave_up = 1; atomicExch(flags + QT_FLAG_ABORT, 1); }
+      const int said = ld_acquire_gpu(count + sweep % 3);
+      stop = said == 0 || said >= 65536;
+      if (blockIdx.x == 0) {
+        flags[QT_FLAG_SWEEPS] = sweep + 1;
+        flags[QT_FLAG_CONVERGED] = said == 0;
+      }
+    }
+    if (__syncthreads_or(gave_up || stop)) return;
   }
 }
 
@@ -2554,15 +2592,17 @@ static int launch_pair_round64(qt_handle* h, const round64_shape& sh, int pairs,
 static bool sweep32_fits(qt_handle* h, int pairs) {
   static int max_ctas = -1;
   if (max_ctas < 0) {
-    int dev = 0, coop = 0, sms = 0, per_sm = 0;
+    int dev = 0, coop = 0, sms = 0, per_sm[2] = {0, 0};
+    auto resident = [](auto kernel, int* ctas) {
+      return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PS_SMEM) == cudaSuccess &&
+             cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas, kernel, NTG, PS_SMEM) == cudaSuccess;
+    };
     max_ctas = 0;
     if (cudaGetDevice(&dev) == cudaSuccess &&
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop &&
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-        cudaFuncSetAttribute(jacobi_sweep32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PS_SMEM) ==
-            cudaSuccess &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, jacobi_sweep32_kernel, NTG, PS_SMEM) == cudaSuccess)
-      max_ctas = per_sm * sms;
+        resident(jacobi_sweep32_kernel<false>, &per_sm[0]) && resident(jacobi_sweep32_kernel<true>, &per_sm[1]))
+      max_ctas = std::min(per_sm[0], per_sm[1]) * sms;
     cudaGetLastError();
   }
   (void)h;
@@ -2572,8 +2612,8 @@ static bool sweep32_fits(qt_handle* h, int pairs) {
 static int launch_sweep32(qt_handle* h, int pairs, float2* x0, float2* x1, int64_t ldx, int mm, float2* v0,
                           float2* v1, int64_t ldv, int nn, int nb, int g0, int has_prev, double tol, float tol_inner,
                           double nu_rel2, const double* xnorm2, float2* wbuf, int* rotbuf, int* done, int max_inner,
-                          float keep2, float* dnorm, unsigned long long* phase_ns, int halves, float2* gx,
-                          int* xflag) {
+                          int max_inner0, int nsweeps, float keep2, float* dnorm, unsigned long long* phase_ns,
+                          int halves, float2* gx, int* xflag) {
   // row split of the two halves of a pair: at a multiple of 32 rows, never
   // past the last row (a V of fewer than 32 rows belongs to half 0 alone)
   const int row_mid = std::min(((mm / 2 + 31) / 32) * 32, mm);
@@ -2595,10 +2635,11 @@ static int launch_sweep32(qt_handle* h, int pairs, float2* x0, float2* x1, int64
   const int spin = stall_polls > 0 ? stall_polls : PS_SPIN;
   const int stall = stall_polls > 0 ? 1 : 0;
   if (h->prof) qt_prof_before(h, "jacobi_sweep32_kernel");
-  const cudaError_t e = cudaLaunchKernelEx(&lc, jacobi_sweep32_kernel, x0, x1, ldx, mm, v0, v1, ldv, nn, nb, g0,
-                                           has_prev, tol, tol_inner, nu_rel2, xnorm2, wbuf, rotbuf, done, h->d_flags,
-                                           max_inner, keep2, dnorm, phase_ns, spin, stall, halves, row_mid, vrow_mid,
-                                           gx, xflag);
+  const auto kernel = nsweeps > 1 ? jacobi_sweep32_kernel<true> : jacobi_sweep32_kernel<false>;
+  const cudaError_t e =
+      cudaLaunchKernelEx(&lc, kernel, x0, x1, ldx, mm, v0, v1, ldv, nn, nb, g0, has_prev, tol, tol_inner, nu_rel2,
+                         xnorm2, wbuf, rotbuf, done, h->d_flags, max_inner, max_inner0, nsweeps, keep2, dnorm, phase_ns,
+                         spin, stall, halves, row_mid, vrow_mid, gx, xflag);
   if (h->prof) qt_prof_after(h);
   h->launches++;
   if (e != cudaSuccess)
@@ -2812,14 +2853,20 @@ int qt_jacobi_svd_ws(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, T
     static const int inner_cap0 =
         std::getenv("QT_JACOBI_INNER0") ? std::atoi(std::getenv("QT_JACOBI_INNER0")) : (fp32 ? 2 : 1);
     const int max_inner = std::max(1, std::min(sweep < 2 ? inner_cap0 : inner_cap, MAX_INNER));
+    // The sweep kernel goes on to the next sweep by itself where "no pair
+    // rotated" is the only rule that ends the sweeps: a launch, its status
+    // copy and synchronisation per sweep cost 25 us each, a sweep of 64 x 64
+    // 100 us.  (The trace wants every sweep's figures.)
+    const bool multi = sweep_kernel && !keep_track && !trace && max_sweeps > 1;
+    const int inner_rest = std::max(1, std::min(inner_cap, MAX_INNER));
     QT_CHECK_CUDA(h, cudaMemsetAsync(h->d_flags, 0, sizeof(int) * QT_FLAG_COUNT, h->stream));
     if (sweep_kernel) {
       if constexpr (sizeof(typename real_of<TS>::type) == 4) {
         QT_TRY(launch_sweep32(h, pairs, (float2*)X, (float2*)X1, ldx, (int)mm, (float2*)V, (float2*)V1, ldv, (int)nn,
                               nb, gcount, pending ? 1 : 0, tol, (float)tol_inner, nu_rel2, (const double*)xnorm2,
-                              (float2*)wbuf, rotf, done, max_inner, keep2, dnorm, phase_ns, halves, gx, xflag));
+                              (float2*)wbuf, rotf, done, multi ? inner_rest : max_inner, max_inner, multi ? max_sweeps : 1,
+                              keep2, dnorm, phase_ns, halves, gx, xflag));
       }
-      gcount += rounds;
       pending = true;
     }
     if (ring.ctas) {
@@ -2862,12 +2909,15 @@ int qt_jacobi_svd_ws(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, T
     if (keep_track)
       QT_CHECK_CUDA(h, cudaMemcpyAsync(hnorm.data(), dnorm, sizeof(float) * nn, cudaMemcpyDeviceToHost, h->stream));
     QT_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
+    const int ran = multi ? std::max(1, h->h_flags[QT_FLAG_SWEEPS]) : 1;  // sweeps of this launch
+    if (sweep_kernel) gcount += ran * rounds;
+    sweep += ran - 1;
     {
       const double es = (double)sizeof(TS);
-      h->work_jacobi_rounds += sweep_rounds;
+      h->work_jacobi_rounds += ran * sweep_rounds;
       h->work_jacobi_pairs += h->h_flags[QT_FLAG_ROTATED];
       h->work_jacobi_inner += h->h_flags[QT_FLAG_INNER];
-      const double read = (double)sweep_rounds * (double)mm * (double)nn * es;
+      const double read = (double)ran * sweep_rounds * (double)mm * (double)nn * es;
       const double pair = (double)h->h_flags[QT_FLAG_ROTATED] * pair_cols * es;
       h->work_jacobi_bytes += read + pair * ((double)mm + (V ? 2.0 * (double)nn : 0.0));
       h->work_jacobi_gram_bytes += read;
@@ -2905,7 +2955,7 @@ int qt_jacobi_svd_ws(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, T
     }
     if (h->h_flags[QT_FLAG_ABORT]) return qt_fail(h, QT_ETIMEOUT, "jacobi: a round of the sweep kernel gave up waiting");
     if (h->h_flags[QT_FLAG_NONFINITE]) return qt_fail(h, QT_ENUMERIC, "jacobi: non-finite value in the matrix");
-    if (h->h_flags[QT_FLAG_ROTATED] == 0) break;
+    if (multi ? h->h_flags[QT_FLAG_CONVERGED] : h->h_flags[QT_FLAG_ROTATED] == 0) break;
     // kept set converged: no pair with a column above the threshold rotated,
     // or the tail weight moved by at most keep_tol of itself over this sweep
     // after at most 10 keep_tol over the previous one (the iteration is in

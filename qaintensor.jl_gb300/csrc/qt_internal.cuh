@@ -70,7 +70,11 @@ enum {
   QT_FLAG_ABORT = 6,     // Jacobi sweep kernel: a bounded round wait gave up
   QT_FLAG_OFFKEPT = 7,   // Jacobi sweep kernel: OFFMAX over pairs with a column above the keep threshold
   QT_FLAG_STALL = 8,     // never set: the bounded-wait test hook of the sweep kernel waits on it
-  QT_FLAG_COUNT = 9
+  QT_FLAG_SWEPT = 9,     // Jacobi sweep kernel, several sweeps a launch: what the CTAs say of sweep s, in slot 9 + s % 3
+  QT_FLAG_ARRIVED = 12,  // ... CTAs that finished a sweep, over all sweeps
+  QT_FLAG_SWEEPS = 13,   // ... sweeps run
+  QT_FLAG_CONVERGED = 14, // ... the last of them rotated nothing
+  QT_FLAG_COUNT = 15
 };
 
 struct qt_mps {
