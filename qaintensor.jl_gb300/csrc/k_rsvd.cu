@@ -862,17 +862,23 @@ int block_cholqr(qt_handle* h, C* Yb, int64_t m, int b, int pass, double2* dG) {
 //   CholeskyQR pass:
 //     (1) the CTA's partial Gram of the block (FP32 over its rows) to
 //         gpart[c];                                               barrier
-//     (2) CTA c adds its slice of the 32 x 32 entries over the CTAs in
+//     (2) CTA c adds its slice of the upper triangle over the CTAs in
 //         float-float, CTAs in order, to gsum;                    barrier
 //     (3) every CTA reads the summed Gram, forms the same R and R^{-1}
 //         (cq_factor) and replaces its rows of the block by rows R^{-1}.
 // The rows go back to global memory once, at the end.  Sums run in a fixed
 // order, so the result is reproducible for a given m.  The barrier is a
-// monotone arrival counter whose last arriving CTA publishes the barrier's
-// number; every wait is bounded, and a wait that gives up sets an abort
-// word (ending the other CTAs' waits) and the handle's sticky device status
-// (2).  Data written by other CTAs is read past L1 (ld.global.cg /
-// cp.async.cg).
+// monotone arrival counter that every CTA polls; every wait is bounded, and a
+// wait that gives up sets an abort word (ending the other CTAs' waits) and the
+// handle's sticky device status (2).  Data written by other CTAs is read past
+// L1 (ld.global.cg / cp.async.cg).
+//
+// What bounds it: up to some 32 CTAs the serial parts, of which the factor's
+// pivot chain is the longest (9.3 us a pass) and the exchanges come next.  So
+// a barrier is one release and one acquire away (2.6 -> 1.5 us against a last
+// arrival that publishes a second word between fences), and the sums of step
+// (2) take all their loads under one latency: 480 x 240, 775 -> 610 us; 512 x
+// 320, 595 -> 470; 2048 x 1152 (whose products weigh as much), 2.49 -> 2.21 ms.
 // ---------------------------------------------------------------------------
 constexpr int OP_NT = 256;     // threads per CTA
 constexpr int OP_R = 16;       // rows per CTA
@@ -890,7 +896,7 @@ struct OrthArgs {
   float2* coef;   // [l][BW] summed coefficients
   float2* gpart;  // [ncta][BW * BW] Gram partials
   float4* gsum;   // [BW * BW] summed Gram (re hi, re lo, im hi, im lo)
-  int* bar;       // [0] arrivals, [1] abort word, [2] the last completed barrier, [3] the test hook's word
+  int* bar;       // [0] arrivals, [1] abort word, [3] the test hook's word
   int* flags;     // QT_FLAG_CHOL
   int* status;    // sticky device status
   int spin;
@@ -927,32 +933,27 @@ __device__ inline void op_cp_async16(void* dst, const void* src) {
                : "memory");
 }
 
-// Grid barrier: false (in every thread of the CTA) when a wait gave up.  The
-// last CTA to arrive publishes the barrier's number in bar[2]; the others
-// poll that word (written once per barrier), not the arrival counter.
+// Grid barrier: false (in every thread of the CTA) when a wait gave up.  One
+// arrival and the polls of the same word: the arrival is a release (cumulative
+// behind the CTA's barrier), a poll an acquire.
 __device__ bool op_barrier(const OrthArgs& a, int& epoch) {
   __syncthreads();
   epoch++;
   int ok = 1;
   if (threadIdx.x == 0) {
-    __threadfence();
-    const int arrived = atomicAdd(a.bar, 1) + 1;
-    if (arrived == epoch * (int)gridDim.x) {
-      asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(a.bar + 2), "r"(epoch) : "memory");
-    } else {
-      int it = 0;
-      for (; it < a.spin; it++) {
-        if (op_ld_acquire(a.bar + 2) >= epoch) break;
-        if ((it & 7) == 7 && *(volatile int*)(a.bar + 1)) { it = a.spin; break; }
-        __nanosleep(20);
-      }
-      if (it >= a.spin) {
-        ok = 0;
-        atomicExch(a.bar + 1, 1);
-        atomicExch(a.status, 2);
-      }
+    const int all = epoch * (int)gridDim.x;
+    asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(a.bar) : "memory");
+    int it = 0;
+    for (; it < a.spin; it++) {
+      if (op_ld_acquire(a.bar) >= all) break;
+      if ((it & 7) == 7 && *(volatile int*)(a.bar + 1)) { it = a.spin; break; }
+      __nanosleep(20);
     }
-    __threadfence();
+    if (it >= a.spin) {
+      ok = 0;
+      atomicExch(a.bar + 1, 1);
+      atomicExch(a.status, 2);
+    }
   }
   return __syncthreads_and(ok) != 0;
 }
@@ -1010,15 +1011,18 @@ __device__ bool op_project(const OrthArgs& a, float2* Ys, float2* Cs, int j0, in
     const size_t stride = (size_t)a.l * BW;
     float2* ws = Cs;  // [8][OP_NT]
     for (int w0 = e_lo; w0 < e_hi; w0 += OP_NT) {
-      for (int g = 0; g < OP_NT; g += 32) {
-        const int e = w0 + g + lane;
-        float2 sum = make_float2(0.f, 0.f);
-        if (e < e_hi) {
-#pragma unroll 8
-          for (int q = q0; q < q1; q++) sum = cadd(sum, __ldcg(a.part + (size_t)q * stride + e));
-        }
-        ws[w * OP_NT + g + lane] = sum;
+      float2 sum[OP_NT / 32];  // (all at once: a loop over them would wait for L2 each time)
+#pragma unroll
+      for (int g = 0; g < OP_NT / 32; g++) sum[g] = make_float2(0.f, 0.f);
+#pragma unroll 4
+      for (int q = q0; q < q1; q++) {
+        const float2* p = a.part + (size_t)q * stride + w0 + lane;
+#pragma unroll
+        for (int g = 0; g < OP_NT / 32; g++)
+          if (w0 + 32 * g + lane < e_hi) sum[g] = cadd(sum[g], __ldcg(p + 32 * g));
       }
+#pragma unroll
+      for (int g = 0; g < OP_NT / 32; g++) ws[w * OP_NT + 32 * g + lane] = sum[g];
       __syncthreads();
       const int e = w0 + t;
       if (e < e_hi) {
@@ -1101,6 +1105,52 @@ __device__ bool op_project(const OrthArgs& a, float2* Ys, float2* Cs, int j0, in
   return true;
 }
 
+// Entries e_lo .. e_hi - 1 of the upper triangle (column by column) of the
+// summed Gram: warp w the entries e_lo + w + 8 v, NE of them under one latency
+// (4, or 1 where every warp has one at most), lane l the CTAs l, l + 32, ...
+// in float-float, then a fixed shuffle tree.
+template <int NE>
+__device__ void op_gram_sums(const OrthArgs& a, int e_lo, int e_hi) {
+  constexpr int E = BW * (BW + 1) / 2, W = OP_NT / 32;
+  const int lane = threadIdx.x & 31, nc = gridDim.x;
+  for (int e0 = e_lo + (threadIdx.x >> 5); e0 < e_hi; e0 += NE * W) {
+    float4 v[NE];
+    int at[NE];
+#pragma unroll
+    for (int u = 0; u < NE; u++) {
+      const int e = min(e0 + u * W, E - 1);
+      int j = (int)((sqrtf(8.f * e + 1.f) - 1.f) * 0.5f);
+      if (j * (j + 1) / 2 > e) j--;
+      if ((j + 1) * (j + 2) / 2 <= e) j++;
+      at[u] = (e - j * (j + 1) / 2) + BW * j;
+      v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll(NE == 1 ? 4 : 1)
+    for (int q = lane; q < nc; q += 32) {
+      float2 x[NE];
+#pragma unroll
+      for (int u = 0; u < NE; u++) x[u] = __ldcg(a.gpart + (size_t)q * BW * BW + at[u]);
+#pragma unroll
+      for (int u = 0; u < NE; u++) v[u] = ff4_add(v[u], make_float4(x[u].x, 0.f, x[u].y, 0.f));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+      for (int u = 0; u < NE; u++) {
+        float4 y;
+        y.x = __shfl_xor_sync(0xffffffffu, v[u].x, o);
+        y.y = __shfl_xor_sync(0xffffffffu, v[u].y, o);
+        y.z = __shfl_xor_sync(0xffffffffu, v[u].z, o);
+        y.w = __shfl_xor_sync(0xffffffffu, v[u].w, o);
+        v[u] = ff4_add(v[u], y);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < NE; u++)
+      if (lane == 0 && e0 + u * W < e_hi) __stcg(a.gsum + at[u], v[u]);
+  }
+}
+
 // One CholeskyQR pass of the block at column j0 (b columns).
 __device__ bool op_cholqr(const OrthArgs& a, float2* Ys, float2* Gl, float2* Xs, float2* Tb, double* Gd, float* Ry,
                           int j0, int b, double shift, int& epoch) {
@@ -1124,28 +1174,12 @@ __device__ bool op_cholqr(const OrthArgs& a, float2* Ys, float2* Gl, float2* Xs,
   op_mark(a, 4);  // Gram partials
   if (!op_barrier(a, epoch)) return false;
   op_mark(a, 1);
-  // (2) this CTA's slice of the entries: warp w the entries e_lo + w + 8 v,
-  // lane l the CTAs l, l + 32, ... in float-float, then a fixed shuffle tree
+  // (2) this CTA's slice of the upper triangle's entries
   {
-    const int per = (BW * BW + nc - 1) / nc, e_lo = c * per, e_hi = min(BW * BW, e_lo + per);
-    const int w = t >> 5, lane = t & 31;
-    for (int e = e_lo + w; e < e_hi; e += OP_NT / 32) {
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (int q = lane; q < nc; q += 32) {
-        const float2 x = __ldcg(a.gpart + (size_t)q * BW * BW + e);
-        v = ff4_add(v, make_float4(x.x, 0.f, x.y, 0.f));
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        float4 u;
-        u.x = __shfl_xor_sync(0xffffffffu, v.x, o);
-        u.y = __shfl_xor_sync(0xffffffffu, v.y, o);
-        u.z = __shfl_xor_sync(0xffffffffu, v.z, o);
-        u.w = __shfl_xor_sync(0xffffffffu, v.w, o);
-        v = ff4_add(v, u);
-      }
-      if (lane == 0) __stcg(a.gsum + e, v);
-    }
+    constexpr int E = BW * (BW + 1) / 2;
+    const int per = (E + nc - 1) / nc, e_lo = c * per, e_hi = min(E, e_lo + per);
+    if (per > OP_NT / 32) op_gram_sums<4>(a, e_lo, e_hi);
+    else op_gram_sums<1>(a, e_lo, e_hi);
   }
   op_mark(a, 5);  // Gram sums
   if (!op_barrier(a, epoch)) return false;
