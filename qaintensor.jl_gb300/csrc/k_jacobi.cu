@@ -1505,27 +1505,27 @@ __device__ int diagonalise_lanes(sweep_solver& sh, const int* col, float tol_inn
       const bool rotp = ((live >> p) & (live >> q) & 1) && a > nu2 && b > nu2 && ags2 > tol2;
       if (!__any_sync(0xffffffffu, rotp)) continue;  // the same vote in every solver warp
       rotated_any = true;
-      float2 jpp = make_float2(1.f, 0.f), jqp = make_float2(0.f, 0.f), jpq = jqp, jqq = jpp;
-      float a2 = a, b2 = b;
-      if (rotp) {
-        const float ria = rsqrtf(a), rib = rsqrtf(b), rags = rsqrtf(ags2);
-        const float sqa = a * ria, sqb = b * rib;
-        const float ag = ags2 * rags * sqa * sqb;  // |gamma|
-        const float zeta = __fdividef(b - a, 2.f * ag);
-        const float z2 = fmaf(zeta, zeta, 1.f);
-        const float r1 = z2 * rsqrtf(z2);
-        const float tt = copysignf(__fdividef(1.f, fabsf(zeta) + r1), zeta);
-        const float c = rsqrtf(fmaf(tt, tt, 1.f)), sn = c * tt;
-        const float2 e = make_float2(gs.x * rags, gs.y * rags);
-        a2 = fmaxf(fmaf(-tt, ag, a), nu2);  // a column driven to the noise level is frozen
-        b2 = fmaf(tt, ag, b);
-        const float ia2 = rsqrtf(a2), ib2 = rsqrtf(b2);
-        const float fa = sqa * ia2, fb = sqb * ib2, fab = sqb * ia2, fba = sqa * ib2;
-        jpp = make_float2(c * fa, 0.f);
-        jqp = make_float2(-sn * e.x * fab, sn * e.y * fab);  // -s conj(e) sqrt(b/a')
-        jpq = make_float2(sn * e.x * fba, sn * e.y * fba);   //  s e sqrt(a/b')
-        jqq = make_float2(c * fb, 0.f);
-      }
+      // (evaluated by every lane and dropped where its pair does not rotate: a
+      // branch would cost the others its reconvergence)
+      const float ria = rsqrtf(a), rib = rsqrtf(b), rags = rsqrtf(ags2);
+      const float sqa = a * ria, sqb = b * rib;
+      const float ag = ags2 * rags * sqa * sqb;  // |gamma|
+      const float zeta = __fdividef(b - a, 2.f * ag);
+      const float z2 = fmaf(zeta, zeta, 1.f);
+      const float r1 = z2 * rsqrtf(z2);
+      const float tt = copysignf(__fdividef(1.f, fabsf(zeta) + r1), zeta);
+      const float c = rsqrtf(fmaf(tt, tt, 1.f)), sn = c * tt;
+      const float2 e = make_float2(gs.x * rags, gs.y * rags);
+      float a2 = fmaxf(fmaf(-tt, ag, a), nu2);  // a column driven to the noise level is frozen
+      float b2 = fmaf(tt, ag, b);
+      const float ia2 = rsqrtf(a2), ib2 = rsqrtf(b2);
+      const float fa = sqa * ia2, fb = sqb * ib2, fab = sqb * ia2, fba = sqa * ib2;
+      const float2 jpp = make_float2(rotp ? c * fa : 1.f, 0.f);
+      const float2 jqp = make_float2(rotp ? -sn * e.x * fab : 0.f, rotp ? sn * e.y * fab : 0.f);  // -s conj(e) sqrt(b/a')
+      const float2 jpq = make_float2(rotp ? sn * e.x * fba : 0.f, rotp ? sn * e.y * fba : 0.f);   //  s e sqrt(a/b')
+      const float2 jqq = make_float2(rotp ? c * fb : 1.f, 0.f);
+      a2 = rotp ? a2 : a;
+      b2 = rotp ? b2 : b;
       // column y of Jt: rows y (real) and y'
       const bool low = y == p;
       const float2 jyy = low ? jpp : jqq, jpy = low ? jqp : jpq;
