@@ -1598,7 +1598,7 @@ jacobi_sweep32_kernel(float2* __restrict__ xb0, float2* __restrict__ xb1, int64_
   rotbuf += (size_t)hf * 2 * pairs;
   if (hf) { phase_ns = nullptr; dnorm = nullptr; }  // half 0 reports for the pair
   __shared__ unsigned long long tp;
-  int swept = 0;  // thread 0: what this CTA has to say about this sweep
+  int swept = 0, swept_off = 0, swept_big = 0;  // thread 0: what this CTA has to say about this sweep
   auto phase = [&](int ph) {  // optional diagnostics: time per phase into phase_ns[ph - 1]
     if (phase_ns && t == 0) {
       unsigned long long tn;
@@ -1928,8 +1928,13 @@ jacobi_sweep32_kernel(float2* __restrict__ xb0, float2* __restrict__ xb1, int64_
       if (bad) atomicOr(&flags[QT_FLAG_NONFINITE], 1);
       __stcg(rotbuf + (size_t)(g & 1) * pairs + q, any_rot);
       if (hf == 0) {  // the pair's statistics, once
-        if (offmax_blk > 0) atomicMax(&flags[QT_FLAG_OFFMAX], offmax_blk);
-        if (offbig_blk > 0) atomicMax(&flags[QT_FLAG_OFFBIG], offbig_blk);
+        if (MULTI) {
+          swept_off = max(r > 0 ? swept_off : 0, offmax_blk);
+          swept_big = max(r > 0 ? swept_big : 0, offbig_blk);
+        } else {
+          if (offmax_blk > 0) atomicMax(&flags[QT_FLAG_OFFMAX], offmax_blk);
+          if (offbig_blk > 0) atomicMax(&flags[QT_FLAG_OFFBIG], offbig_blk);
+        }
         if (offkept_blk > 0) atomicMax(&flags[QT_FLAG_OFFKEPT], offkept_blk);
         if (any_rot) atomicAdd(&flags[QT_FLAG_ROTATED], 1);
       }
@@ -1949,16 +1954,26 @@ jacobi_sweep32_kernel(float2* __restrict__ xb0, float2* __restrict__ xb1, int64_
     // ---- several sweeps in this launch: the end of one waits (bounded) until
     // every CTA has said whether it rotated (1) or met a non-finite value
     // (65536), and a sweep without the first or with the second is the last.
-    // Sweep s adds up in slot s % 3; CTA 0 clears the next slot before it
-    // arrives: whoever read that slot two sweeps ago has arrived since.
+    // Sweep s adds up in slot s % 3, its largest off-diagonals beside that (the
+    // rule at the sweep limit is about the last sweep alone); CTA 0 clears the
+    // next slots before it arrives: whoever read them two sweeps ago has arrived
+    // since.
     if (t == 0) swept = (r > 0 ? swept : 0) | (any_rot ? 1 : 0) | (bad ? 65536 : 0);
     if (r < R - 1) continue;
     int stop = 0;
     gave_up = 0;
     if (t == 0) {
       int* count = flags + QT_FLAG_SWEPT;
+      int *off = flags + QT_FLAG_SWEPT_OFF + sweep % 3, *big = flags + QT_FLAG_SWEPT_BIG + sweep % 3;
       if (swept) atomicAdd(count + sweep % 3, swept);
-      if (blockIdx.x == 0) atomicExch(count + (sweep + 1) % 3, 0);
+      if (swept_off > 0) atomicMax(off, swept_off);
+      if (swept_big > 0) atomicMax(big, swept_big);
+      if (blockIdx.x == 0) {
+        const int next = (sweep + 1) % 3;
+        atomicExch(count + next, 0);
+        atomicExch(flags + QT_FLAG_SWEPT_OFF + next, 0);
+        atomicExch(flags + QT_FLAG_SWEPT_BIG + next, 0);
+      }
       __threadfence();
       atomicAdd(flags + QT_FLAG_ARRIVED, 1);
       int it = 0;
@@ -1973,6 +1988,8 @@ jacobi_sweep32_kernel(float2* __restrict__ xb0, float2* __restrict__ xb1, int64_
       if (blockIdx.x == 0) {
         flags[QT_FLAG_SWEEPS] = sweep + 1;
         flags[QT_FLAG_CONVERGED] = said == 0;
+        flags[QT_FLAG_OFFMAX] = ld_acquire_gpu(off);
+        flags[QT_FLAG_OFFBIG] = ld_acquire_gpu(big);
       }
     }
     if (__syncthreads_or(gave_up || stop)) return;

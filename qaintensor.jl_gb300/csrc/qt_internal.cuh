@@ -74,7 +74,9 @@ enum {
   QT_FLAG_ARRIVED = 12,  // ... CTAs that finished a sweep, over all sweeps
   QT_FLAG_SWEEPS = 13,   // ... sweeps run
   QT_FLAG_CONVERGED = 14, // ... the last of them rotated nothing
-  QT_FLAG_COUNT = 15
+  QT_FLAG_SWEPT_OFF = 15, // ... OFFMAX of sweep s, in slot 15 + s % 3 (OFFMAX itself: the last sweep's)
+  QT_FLAG_SWEPT_BIG = 18, // ... OFFBIG of sweep s, likewise
+  QT_FLAG_COUNT = 21
 };
 
 struct qt_mps {
