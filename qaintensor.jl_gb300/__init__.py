@@ -735,12 +735,17 @@ class Batch:
 
     def run(self, layers, cutoff: float, use_graph: bool = True):
         """layers: list of lists of (circuit, wire 1-based, 4x4 gate)."""
-        tasks = [t for layer in layers for t in layer]
-        st = np.cumsum([0] + [len(layer) for layer in layers], dtype=np.int32)
-        circ = [t[0] for t in tasks]
+        starts, circ, site, gates = [0], [], [], []
+        for layer in layers:  # (read once: a layer may be an iterator)
+            for c, w, g in layer:
+                circ.append(c)
+                site.append(w - 1)
+                gates.append(g)
+            starts.append(len(circ))
+        st = np.asarray(starts, dtype=np.int32)
         ci = np.asarray(circ, dtype=np.int32)
-        si = np.asarray([t[1] for t in tasks], dtype=np.int32) - np.int32(1)
-        ga = self._pack_gates([t[2] for t in tasks])
+        si = np.asarray(site, dtype=np.int32)
+        ga = self._pack_gates(gates)
         self.ntask = len(circ)
         self.eng._check(self.eng._lib.qt_batch_run(self.eng._h, self._p, len(layers), _ptr(st), _ptr(ci), _ptr(si),
                                                    _ptr(ga), float(cutoff), int(use_graph)))
