@@ -20,8 +20,8 @@
 //   B' = A'^H theta'            written into site slot w+1 (no V accumulation)
 //   bonds[w+1] = k
 // The tasks left to the FP64 split are listed, and a second kernel of the layer
-// takes them, a cluster of eight CTAs each (batch_split64_kernel).  Tasks of
-// one brickwork layer touch disjoint sites, so CTAs never race.  A whole program
+// takes them, a cluster of eight CTAs each or, where many are left, one CTA
+// each (batch_split64_kernel).  Tasks of one brickwork layer touch disjoint sites, so CTAs never race.  A whole program
 // (every layer) is a fixed sequence of a counter reset and kernels that the
 // host captures once in a CUDA graph.  There are no waits on
 // other CTAs: a CTA stops when the counter passes the task count.
@@ -56,10 +56,11 @@ struct BatchArgs {
   const int* task_grank;     // per task: the gate's operator-Schmidt rank
   int task_begin, task_end;
   int* counter;
-  float2* slab;              // per CTA: 4 * slab_elems float2 (FP32 X, T; per cluster the FP64 T, X)
+  float2* slab;              // per CTA: 4 * slab_elems float2 (FP32 X, T; per cluster or CTA the FP64 T, X)
   int slab_elems;
   int* left;                 // tasks of this layer left to the FP64 split, and how many
   int* nleft;
+  int alone_above;           // more tasks left than this: one CTA each, not a cluster
   int smem_elems;            // float2 entries of the CTA's dynamic shared memory
   double cutoff;
   double floor_rel;          // FP32 resolution relative to ||theta'||_F (<= 0: 4 sqrt(max(m, n)) u)
@@ -305,163 +306,210 @@ __global__ void __launch_bounds__(NT) batch_layer_kernel(BatchArgs p) {
 // last bit, and later FP32 splits of the same circuit see which one was taken.
 // A 128 x 128 task (about 27 sweeps): 31 ms, 9 us a round, 8 us of them FP64
 // issue; by one CTA, as the layer kernel's last step, 95 ms.
+// That pays while few tasks are left.  From some number on (see
+// split64_alone_above) every CTA takes a task by itself, a warp to a pair and
+// the columns in the slab where shared memory does not hold them: the same sums
+// in the same order, so that a circuit's results do not depend on how many
+// others run beside it.
 constexpr int S64_NT = 256, S64_C = 8, S64_W = S64_NT / 32;
 constexpr int S64_LD = 36;                    // rows of a slice, at most; 4 (mod 8) for the banks
 constexpr size_t S64_ROTS = MAXN / 2 * 5;     // rotations of a round's pairs: c, s, er, ei, on
 constexpr size_t S64_SUMS = MAXN / 2 * 4;     // sums of a round's pairs
 constexpr size_t S64_SMEM = (2 * S64_SUMS + S64_ROTS + 2 * S64_LD * MAXN) * sizeof(double);
 
-// Sums of this CTA's rows of each pair, aa bb gr gi.  4 K rows (zeros past the matrix).
-__device__ __forceinline__ void split64_sums(const double2* Xs, int ld, int K, int n, int round, double* part) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lr = lane & 3, pairs = n / 2;
-  for (int first = 8 * warp; first < pairs; first += 8 * S64_W) {
-    const int q = first + (lane >> 2);
+// Sums of this CTA's rows of each pair, aa bb gr gi, LP lanes on a pair.
+template <int LP>
+__device__ __forceinline__ void split64_sums(const double2* X, int ld, int rows, int n, int round, double* part) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lr = lane % LP, pairs = n / 2;
+  constexpr int PW = 32 / LP;
+  for (int first = PW * warp; first < pairs; first += PW * S64_W) {
+    const int q = first + lane / LP;
     int a, b;
     cta_tourney(round, min(q, pairs - 1), n, a, b);
-    const double2 *xp = Xs + ld * a + lr, *xq = Xs + ld * b + lr;
+    const double2 *xp = X + (size_t)ld * a, *xq = X + (size_t)ld * b;
     double v0 = 0, v1 = 0, v2 = 0, v3 = 0;
-    for (int k = 0; k < K; k++) {
-      const double2 u = xp[4 * k], w = xq[4 * k];
+    for (int j = lr; j < rows; j += LP) {
+      const double2 u = xp[j], w = xq[j];
       v0 = fma(u.x, u.x, fma(u.y, u.y, v0));
       v1 = fma(w.x, w.x, fma(w.y, w.y, v1));
       v2 = fma(u.x, w.x, fma(u.y, w.y, v2));
       v3 = fma(u.x, w.y, fma(-u.y, w.x, v3));
     }
-    const bool up2 = lr & 2, up1 = lr & 1;
-    const double x0 = (up2 ? v2 : v0) + __shfl_xor_sync(0xffffffffu, up2 ? v0 : v2, 2);
-    const double x1 = (up2 ? v3 : v1) + __shfl_xor_sync(0xffffffffu, up2 ? v1 : v3, 2);
-    const double s = (up1 ? x1 : x0) + __shfl_xor_sync(0xffffffffu, up1 ? x0 : x1, 1);
-    if (q < pairs) part[4 * q + lr] = s;
+    const bool up2 = lr & (LP / 2), up1 = lr & (LP / 4);
+    const double x0 = (up2 ? v2 : v0) + __shfl_xor_sync(0xffffffffu, up2 ? v0 : v2, LP / 2);
+    const double x1 = (up2 ? v3 : v1) + __shfl_xor_sync(0xffffffffu, up2 ? v1 : v3, LP / 2);
+    double s = (up1 ? x1 : x0) + __shfl_xor_sync(0xffffffffu, up1 ? x0 : x1, LP / 4);
+#pragma unroll
+    for (int o = LP / 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (q < pairs && lr % (LP / 4) == 0) part[4 * q + lr / (LP / 4)] = s;
   }
 }
 
-__device__ __forceinline__ void split64_rotate(double2* Xs, int ld, int K, int n, int round, const double* rot) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lr = lane & 3, pairs = n / 2;
-  for (int q = 8 * warp + (lane >> 2); q < pairs; q += 8 * S64_W) {
+// (every rounding written out, as in cta_store_rotated: the same bits with every LP)
+template <int LP>
+__device__ __forceinline__ void split64_rotate(double2* X, int ld, int rows, int n, int round, const double* rot) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lr = lane % LP, pairs = n / 2;
+  constexpr int PW = 32 / LP;
+  for (int q = PW * warp + lane / LP; q < pairs; q += PW * S64_W) {
     if (rot[5 * q + 4] == 0) continue;
     const double c = rot[5 * q], s = rot[5 * q + 1], er = rot[5 * q + 2], ei = rot[5 * q + 3];
     int a, b;
     cta_tourney(round, q, n, a, b);
-    double2 *xp = Xs + ld * a + lr, *xq = Xs + ld * b + lr;
-    for (int k = 0; k < K; k++) {
-      const double2 u = xp[4 * k], v = xq[4 * k];
-      xp[4 * k] = make_double2(c * u.x - s * (er * v.x + ei * v.y), c * u.y - s * (er * v.y - ei * v.x));
-      xq[4 * k] = make_double2(s * (er * u.x - ei * u.y) + c * v.x, s * (er * u.y + ei * u.x) + c * v.y);
+    double2 *xp = X + (size_t)ld * a, *xq = X + (size_t)ld * b;
+    for (int j = lr; j < rows; j += LP) {
+      const double2 u = xp[j], v = xq[j];
+      xp[j] = make_double2(fma(c, u.x, -__dmul_rn(s, fma(er, v.x, __dmul_rn(ei, v.y)))),
+                           fma(c, u.y, -__dmul_rn(s, fma(er, v.y, -__dmul_rn(ei, v.x)))));
+      xq[j] = make_double2(fma(c, v.x, __dmul_rn(s, fma(er, u.x, -__dmul_rn(ei, u.y)))),
+                           fma(s, fma(ei, u.x, __dmul_rn(er, u.y)), __dmul_rn(c, v.y)));
     }
   }
 }
 
-__global__ void __cluster_dims__(S64_C, 1, 1) __launch_bounds__(S64_NT) batch_split64_kernel(BatchArgs p) {
-  extern __shared__ __align__(16) unsigned char dyn[];
-  __shared__ int s_next;
-  __shared__ double2 g64[16];
-  __shared__ double s_sig[MAXN], s_red[S64_NT / 32];
-  __shared__ int s_perm[MAXN], s_k;
+struct split64_shared {
+  double2 g64[16];
+  double sig[MAXN], red[S64_NT / 32];
+  int perm[MAXN], k, next;
+};
+
+// One task by CW CTAs (CW = 1: this one alone), `rank` of them.
+template <int CW>
+__device__ void split64_task(const BatchArgs& p, int task, int rank, double2* T, double2* Xg, unsigned char* dyn,
+                             split64_shared& sh) {
   cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rank = (int)cl.block_rank();
+  auto meet = [&]() {
+    if constexpr (CW > 1) cl.sync();
+    else __syncthreads();
+  };
+  constexpr int LP = 32 / CW;  // lanes per pair
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   double* part = reinterpret_cast<double*>(dyn);  // two rounds' sums
   double* rot = part + 2 * S64_SUMS;
   double2* Xs = reinterpret_cast<double2*>(rot + S64_ROTS);
-  double2* T = reinterpret_cast<double2*>(p.slab + (size_t)(blockIdx.x - rank) * 4 * p.slab_elems);
-  double2* Xg = T + p.slab_elems;
-  for (;;) {
-    if (rank == 0 && tid == 0) s_next = atomicAdd(p.counter, 1);
-    cl.sync();
-    const int i = *cl.map_shared_rank(&s_next, 0);
-    if (i >= *p.nleft) break;
-    const int task = p.left[i];
-    const int c = p.task_circ[task], w = p.task_site[task];
-    int* bond = p.bonds + p.bond_off[c];
-    const int chil = bond[w], chim = bond[w + 1], chir = bond[w + 2], cap = p.cap[c];
-    const size_t slot = (size_t)cap * 2 * cap;
-    float2* A = p.sites + p.site_off[c] + (size_t)w * slot;
-    float2* B = A + slot;
-    const int m = 2 * chil, n = 2 * chir, pairs = n / 2;
-    // rows S64_C j + rank, j < rc, of which the last CTAs may have one less; 4 K with the zeros
-    const int rc = (m + S64_C - 1) / S64_C, K = (rc + 3) / 4, ld = 4 * (K | 1);
-    if (tid < 16) g64[tid] = p.task_gate[(size_t)task * 16 + tid];
-    __syncthreads();
-    // theta': this CTA's columns (the two values of s2 together), then its rows
-    const int b0 = rank * chir / S64_C, b1 = (rank + 1) * chir / S64_C;
-    double2* Tb = T + (size_t)m * 2 * b0;
-    const float2* Bb = B + (size_t)chim * 2 * b0;
-    if (b1 > b0) form_theta<S64_NT, 32, double2>(A, Bb, chil, chim, b1 - b0, g64, Tb, m, Tb, dyn);
-    cl.sync();
-    for (int j = warp; j < n; j += S64_W)
-      for (int r = lane; r < 4 * K; r += 32)
-        Xs[r + ld * j] = S64_C * r + rank < m ? T[S64_C * r + rank + (size_t)m * j] : make_double2(0, 0);
-    const double f64 = fro2_of<S64_NT>(T, m * n, s_red);  // the same in every CTA
-    const double tol = 16.0 * sqrt((double)max(m, 16)) * 1.11e-16, nu = 4.0 * sqrt((double)max(m, 16)) * 1.11e-16;
-    const double nu2 = nu * nu * f64;
-    int sweeps = 0, buf = 0;
-    for (int sweep = 0; sweep < p.max_sweeps; sweep++) {
-      bool rotated = false;
-      for (int r = 0; r < n - 1; r++) {
-        double* pb = part + buf * S64_SUMS;
-        split64_sums(Xs, ld, K, n, r, pb);
-        cl.sync();  // (two buffers: whoever reads this round's sums has left the last round's)
-        if (tid < pairs) {
-          double2 v[S64_C], u[S64_C];
+  const int c = p.task_circ[task], w = p.task_site[task];
+  int* bond = p.bonds + p.bond_off[c];
+  const int chil = bond[w], chim = bond[w + 1], chir = bond[w + 2], cap = p.cap[c];
+  const size_t slot = (size_t)cap * 2 * cap;
+  float2* A = p.sites + p.site_off[c] + (size_t)w * slot;
+  float2* B = A + slot;
+  const int m = 2 * chil, n = 2 * chir, pairs = n / 2;
+  // a cluster: rows CW j + rank of every column in shared memory, j < 4 K with
+  // the zeros, of which the last CTAs have one more; one CTA: every row, in the slab
+  // where shared memory does not hold them (ld odd: columns start in different banks)
+  const int K = ((m + CW - 1) / CW + 3) / 4;
+  const bool in_smem = CW > 1 || (m | 1) * n <= S64_LD * MAXN;
+  double2* X = in_smem ? Xs : Xg;
+  const int ld = CW > 1 ? 4 * (K | 1) : in_smem ? m | 1 : m, rows = CW > 1 ? 4 * K : m;
+  if (tid < 16) sh.g64[tid] = p.task_gate[(size_t)task * 16 + tid];
+  __syncthreads();
+  // theta': this CTA's columns (the two values of s2 together), then its rows
+  const int b0 = rank * chir / CW, b1 = (rank + 1) * chir / CW;
+  double2* Tb = T + (size_t)m * 2 * b0;
+  const float2* Bb = B + (size_t)chim * 2 * b0;
+  if (b1 > b0) form_theta<S64_NT, 32, double2>(A, Bb, chil, chim, b1 - b0, sh.g64, Tb, m, Tb, dyn);
+  meet();
+  for (int j = warp; j < n; j += S64_W)
+    for (int r = lane; r < rows; r += 32)
+      X[r + (size_t)ld * j] = CW * r + rank < m ? T[CW * r + rank + (size_t)m * j] : make_double2(0, 0);
+  const double f64 = fro2_of<S64_NT>(T, m * n, sh.red);  // the same in every CTA
+  const double tol = 16.0 * sqrt((double)max(m, 16)) * 1.11e-16, nu = 4.0 * sqrt((double)max(m, 16)) * 1.11e-16;
+  const double nu2 = nu * nu * f64;
+  int sweeps = 0, buf = 0;
+  for (int sweep = 0; sweep < p.max_sweeps; sweep++) {
+    bool rotated = false;
+    for (int r = 0; r < n - 1; r++) {
+      double* pb = part + buf * S64_SUMS;
+      split64_sums<LP>(X, ld, rows, n, r, pb);
+      meet();  // (two buffers: whoever reads this round's sums has left the last round's)
+      if (tid < pairs) {
+        double2 v[CW], u[CW];
 #pragma unroll
-          for (int q = 0; q < S64_C; q++) {
-            const double2* o = reinterpret_cast<const double2*>(cl.map_shared_rank(pb, q) + 4 * tid);
-            v[q] = o[0];
-            u[q] = o[1];
-          }
-#pragma unroll
-          for (int off = S64_C / 2; off > 0; off >>= 1)
-#pragma unroll
-            for (int q = 0; q < off; q++) {
-              v[q].x += v[q + off].x; v[q].y += v[q + off].y;
-              u[q].x += u[q + off].x; u[q].y += u[q + off].y;
-            }
-          const cta_rotation<double> o = cta_angle64<double>(v[0].x, v[0].y, u[0].x, u[0].y, tol, nu2);
-          double* d = rot + 5 * tid;
-          d[0] = o.c; d[1] = o.s; d[2] = o.er; d[3] = o.ei;
-          d[4] = o.on ? 1.0 : 0.0;
-          rotated |= o.on;
+        for (int q = 0; q < CW; q++) {
+          const double2* o = reinterpret_cast<const double2*>((CW > 1 ? cl.map_shared_rank(pb, q) : pb) + 4 * tid);
+          v[q] = o[0];
+          u[q] = o[1];
         }
-        __syncthreads();
-        split64_rotate(Xs, ld, K, n, r, rot);
-        __syncthreads();
-        buf ^= 1;
+#pragma unroll
+        for (int off = CW / 2; off > 0; off >>= 1)
+#pragma unroll
+          for (int q = 0; q < off; q++) {
+            v[q].x += v[q + off].x; v[q].y += v[q + off].y;
+            u[q].x += u[q + off].x; u[q].y += u[q + off].y;
+          }
+        const cta_rotation<double> o = cta_angle64<double>(v[0].x, v[0].y, u[0].x, u[0].y, tol, nu2);
+        double* d = rot + 5 * tid;
+        d[0] = o.c; d[1] = o.s; d[2] = o.er; d[3] = o.ei;
+        d[4] = o.on ? 1.0 : 0.0;
+        rotated |= o.on;
       }
-      sweeps = sweep + 1;
-      if (!__syncthreads_or(rotated)) break;  // the same answer in every CTA
+      __syncthreads();
+      split64_rotate<LP>(X, ld, rows, n, r, rot);
+      __syncthreads();
+      buf ^= 1;
     }
+    sweeps = sweep + 1;
+    if (!__syncthreads_or(rotated)) break;  // the same answer in every CTA
+  }
+  if (in_smem)
     for (int j = warp; j < n; j += S64_W)
-      for (int r = lane; S64_C * r + rank < m; r += 32) Xg[S64_C * r + rank + (size_t)m * j] = Xs[r + ld * j];
-    cl.sync();
-    sorted_norms<S64_NT, double2>(Xg, m, m, n, s_sig, s_perm);  // the same in every CTA
-    if (tid == 0) {
-      const int k = min(tail_rule(s_sig, n, p.cutoff), min(cap, min(m, n)));
-      double disc = 0;
-      for (int j = k; j < n; j++) disc += s_sig[j] * s_sig[j];
-      s_k = k;
-      if (rank == 0) {
-        p.task_rank[task] = k;
-        p.task_sweeps[task] += sweeps;
-        p.task_discarded[task] = (float)disc;
-      }
+      for (int r = lane; CW * r + rank < m; r += 32) Xg[CW * r + rank + (size_t)m * j] = X[r + (size_t)ld * j];
+  meet();
+  sorted_norms<S64_NT, double2>(Xg, m, m, n, sh.sig, sh.perm);  // the same in every CTA
+  if (tid == 0) {
+    const int k = min(tail_rule(sh.sig, n, p.cutoff), min(cap, min(m, n)));
+    double disc = 0;
+    for (int j = k; j < n; j++) disc += sh.sig[j] * sh.sig[j];
+    sh.k = k;
+    if (rank == 0) {
+      p.task_rank[task] = k;
+      p.task_sweeps[task] += sweeps;
+      p.task_discarded[task] = (float)disc;
     }
-    __syncthreads();
-    const int k = s_k;
-    // A' = unit columns (this CTA's rows), B' = A'^H theta' (its columns), both from the FP64 columns
-    for (int j = warp; j < k; j += S64_W) {
-      const double s = s_sig[j], inv = s > 0 ? 1.0 / s : 0.0;
-      const double2* x = Xs + ld * s_perm[j];
-      for (int r = lane; S64_C * r + rank < m; r += 32)
-        A[S64_C * r + rank + (size_t)m * j] = make_float2((float)(x[r].x * inv), (float)(x[r].y * inv));
+  }
+  __syncthreads();
+  const int k = sh.k;
+  // A' = unit columns (this CTA's rows), B' = A'^H theta' (its columns), both from the FP64 columns
+  for (int j = warp; j < k; j += S64_W) {
+    const double s = sh.sig[j], inv = s > 0 ? 1.0 / s : 0.0;
+    const double2* x = X + (size_t)ld * sh.perm[j];
+    for (int r = lane; CW * r + rank < m; r += 32)
+      A[CW * r + rank + (size_t)m * j] = make_float2((float)(x[r].x * inv), (float)(x[r].y * inv));
+  }
+  __syncthreads();  // the product's tiles take the start of the shared memory
+  if (b1 > b0)
+    cta_gemm<S64_NT, 32, double2>(true, false, k, 2 * (b1 - b0), m, Xg, m, sh.perm, Tb, m, dyn,
+                                  [&](int r, int col, double2 v) {
+                                    const double s = sh.sig[r], inv = s > 0 ? 1.0 / s : 0.0;
+                                    B[r + (size_t)k * (2 * b0 + col)] = make_float2((float)(v.x * inv), (float)(v.y * inv));
+                                  });
+  if (rank == 0 && tid == 0) bond[w + 1] = k;
+  meet();
+}
+
+__global__ void __cluster_dims__(S64_C, 1, 1) __launch_bounds__(S64_NT) batch_split64_kernel(BatchArgs p) {
+  extern __shared__ __align__(16) unsigned char dyn[];
+  __shared__ split64_shared sh;
+  const int left = *p.nleft, tid = threadIdx.x;
+  if (left == 0) return;
+  if (left > p.alone_above) {
+    double2* T = reinterpret_cast<double2*>(p.slab + (size_t)blockIdx.x * 4 * p.slab_elems);
+    for (;;) {
+      if (tid == 0) sh.next = atomicAdd(p.counter, 1);
+      __syncthreads();
+      const int i = sh.next;
+      if (i >= left) return;
+      split64_task<1>(p, p.left[i], 0, T, T + p.slab_elems, dyn, sh);
     }
-    __syncthreads();  // the product's tiles take the start of the shared memory
-    if (b1 > b0)
-      cta_gemm<S64_NT, 32, double2>(true, false, k, 2 * (b1 - b0), m, Xg, m, s_perm, Tb, m, dyn,
-                                    [&](int r, int col, double2 v) {
-                                      const double s = s_sig[r], inv = s > 0 ? 1.0 / s : 0.0;
-                                      B[r + (size_t)k * (2 * b0 + col)] = make_float2((float)(v.x * inv), (float)(v.y * inv));
-                                    });
-    if (rank == 0 && tid == 0) bond[w + 1] = k;
+  }
+  cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  const int rank = (int)cl.block_rank();
+  double2* T = reinterpret_cast<double2*>(p.slab + (size_t)(blockIdx.x - rank) * 4 * p.slab_elems);
+  for (;;) {
+    if (rank == 0 && tid == 0) sh.next = atomicAdd(p.counter, 1);
     cl.sync();
+    const int i = *cl.map_shared_rank(&sh.next, 0);
+    if (i >= left) break;
+    split64_task<S64_C>(p, p.left[i], rank, T, T + p.slab_elems, dyn, sh);
   }
   cl.sync();  // no CTA leaves while another may still read its shared memory
 }
@@ -613,6 +661,19 @@ size_t batch_smem(int bk) {
   static const size_t theta[4] = {33 * 32, 65 * 64, 129 * 128, 25600};
   return std::max(theta[bk] * sizeof(float2),
                   cta_gemm_smem<float2>(bk == 0 ? 32 : 64));
+}
+
+// From how many tasks left in a launch on its FP64 splits take one CTA each
+// instead of a cluster of eight: a cluster ends a task sooner, alone more of
+// them run at once (152 against 19).  The line lies where the two take the
+// same time for whole programs (ms at tasks per layer, alone / cluster):
+// caps 16: 9.5 / 9.1 at 28, 9.8 / 10.9 at 32; 32: 49.6 / 45.1 at 75, 48.7 /
+// 59.3 at 80 (a wave of clusters more); 64: 85.2 / 66.7 at 90, 85.2 / 90.6 at
+// 108; 128: 854 / 810 at 280, 905 / 982 at 336.  Far from it: 1536 tasks of
+// caps 8 12 / 95, 7 tasks of caps 128 732 / 204.
+int split64_alone_above(int bk) {
+  static const int line[4] = {28, 76, 100, 300};
+  return line[bk];
 }
 
 typedef void (*layer_fn)(BatchArgs);
@@ -835,6 +896,7 @@ extern "C" int qt_batch_run(qt_handle* h, qt_batch* b, int nlayers, const int* l
       const layer_fn batch_layer_kernel_fn = layer_kernel(b->threads[bk], bk);
       QT_LAUNCH(h, batch_layer_kernel_fn, grid, b->threads[bk], batch_smem(bk), al);
       al.counter += 2;
+      al.alone_above = split64_alone_above(bk);
       QT_LAUNCH(h, batch_split64_kernel, S64_C * b->split_clusters(seg_end[sg] - seg_begin[sg]), S64_NT, S64_SMEM, al);
     }
     return QT_OK;

@@ -19,17 +19,18 @@ struct cta_rotation {
 
 // From the pair's sums aa = |x_p|^2, bb = |x_q|^2, gr + i gi = x_p^H x_q:
 // rotate while the relative off-diagonal exceeds tol; the angle in FP64,
-// rounded to the columns' precision.
+// rounded to the columns' precision.  What is fused is written out: the same
+// bits wherever this is inlined.
 template <typename R>
 __device__ __forceinline__ cta_rotation<R> cta_angle64(R aa, R bb, R gr, R gi, double tol, double nu2) {
   cta_rotation<R> o;
   o.c = 1; o.s = 0; o.er = 1; o.ei = 0;
-  const double ag = sqrt((double)gr * gr + (double)gi * gi);
+  const double ag = sqrt(fma((double)gr, (double)gr, __dmul_rn((double)gi, (double)gi)));
   o.on = (double)aa > nu2 && (double)bb > nu2 && ag > tol * sqrt((double)aa * bb);
   if (o.on) {
     const double zeta = ((double)bb - aa) / (2.0 * ag);
-    const double t = copysign(1.0, zeta) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-    const double cs = 1.0 / sqrt(1.0 + t * t);
+    const double t = copysign(1.0, zeta) / (fabs(zeta) + sqrt(fma(zeta, zeta, 1.0)));
+    const double cs = 1.0 / sqrt(fma(t, t, 1.0));
     o.c = (R)cs;
     o.s = (R)(cs * t);
     o.er = (R)(gr / ag);
