@@ -30,7 +30,9 @@ theta_gate_kernel(const TI* __restrict__ A, const TI* __restrict__ B, int chil, 
   __shared__ CR As[2][KC][TA];
   __shared__ CR Bs[2][KC][TB + 1];
   const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
-  const int a0 = blockIdx.x * TA, b0 = blockIdx.y * TB;
+  // tiles along x of the grid, which takes 2^31: y takes 65535, too few for a
+  // bond of more than 524280 in FP64
+  const int ta = (chil + TA - 1) / TA, a0 = blockIdx.x % ta * TA, b0 = blockIdx.x / ta * TB;
   CR acc[RA][RB][2][2];
 #pragma unroll
   for (int i = 0; i < RA; i++)
@@ -267,7 +269,7 @@ int qt_theta_gate(qt_handle* h, int dtype_in, const void* A, const void* B, int6
   for (int e = 0; e < 16; e++) gp.g[e] = make_double2(G[2 * e], G[2 * e + 1]);
   if (chil <= 0 || chim <= 0 || chir <= 0) return qt_fail(h, QT_EINVAL, "theta: empty bond");
   if (prec == 0) {
-    dim3 grid((unsigned)((chil + 7) / 8), (unsigned)((chir + 7) / 8));
+    const unsigned grid = (unsigned)(((chil + 7) / 8) * ((chir + 7) / 8));
     if (dtype_in == QT_C128)
       QT_LAUNCH(h, (theta_gate_kernel<double2, double, double2, 1, 1, 8>), grid, 64, 0, (const double2*)A,
                 (const double2*)B, (int)chil, (int)chim, (int)chir, gp, (double2*)theta_out);
@@ -275,7 +277,7 @@ int qt_theta_gate(qt_handle* h, int dtype_in, const void* A, const void* B, int6
       QT_LAUNCH(h, (theta_gate_kernel<float2, double, double2, 1, 1, 8>), grid, 64, 0, (const float2*)A,
                 (const float2*)B, (int)chil, (int)chim, (int)chir, gp, (double2*)theta_out);
   } else {
-    dim3 grid((unsigned)((chil + 31) / 32), (unsigned)((chir + 31) / 32));
+    const unsigned grid = (unsigned)(((chil + 31) / 32) * ((chir + 31) / 32));
     if (dtype_in == QT_C128)
       QT_LAUNCH(h, (theta_gate_kernel<double2, float, float2, 2, 2, 16>), grid, 256, 0, (const double2*)A,
                 (const double2*)B, (int)chil, (int)chim, (int)chir, gp, (float2*)theta_out);
