@@ -81,11 +81,11 @@ __global__ void __launch_bounds__(ET * ET) env_product_kernel(EnvLaunch l) {
 }
 
 // out[b] = Re tr(L_b R) for Hermitian R (n entries each), one CTA per b
-__global__ void __launch_bounds__(512) env_trace_kernel(const double2* L0, const double2* L1, const double2* R, int n,
-                                                        double* out) {
+__global__ void __launch_bounds__(512) env_trace_kernel(const double2* L0, const double2* L1, const double2* R,
+                                                        int64_t n, double* out) {
   const double2* L = blockIdx.x ? L1 : L0;
   double s = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) s = fma(L[i].x, R[i].x, fma(L[i].y, R[i].y, s));
+  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) s = fma(L[i].x, R[i].x, fma(L[i].y, R[i].y, s));
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   __shared__ double red[16];
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
@@ -170,7 +170,7 @@ int qt_mps_expect2(qt_handle* h, const qt_mps* mps, int site, int nops, double* 
     Ln = Lnum;
   }
   const int64_t c = hi < n ? mps->chil[hi] : mps->chir[n - 1];
-  QT_LAUNCH(h, env_trace_kernel, 2, 512, 0, L, Ln, R, (int)(c * c), out);
+  QT_LAUNCH(h, env_trace_kernel, 2, 512, 0, L, Ln, R, c * c, out);
   double v[2];
   QT_CHECK_CUDA(h, cudaMemcpyAsync(v, out, sizeof(v), cudaMemcpyDeviceToHost, h->stream));
   QT_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
