@@ -34,6 +34,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 #include <functional>
 #include <vector>
@@ -2239,7 +2240,8 @@ __global__ void __launch_bounds__(32 * RING_WARPS, 1) jacobi_ring32_kernel(RingA
       if (last || ((it & 7) == 7 && *(volatile int*)(A.flags + QT_FLAG_ABORT))) break;
     }
   };
-  float relmax = 0.f, relbig = 0.f, relkept = 0.f;  // of the lane's pairs that rotated (warp 0)
+  // of the lane's pairs that rotated (warp 0); relmax is infinite once a column's norm was not finite
+  float relmax = 0.f, relbig = 0.f, relkept = 0.f;
   float aa = 0.f, bb = 0.f;                         // squared norms of pair lane / 8
   int buf = 0;
   // `n` sums per pair (v, pair by pair) over the CTA's rows of X; lane l ends
@@ -2307,6 +2309,8 @@ __global__ void __launch_bounds__(32 * RING_WARPS, 1) jacobi_ring32_kernel(RingA
     if (FRESH) {
       aa = __shfl_sync(0xffffffffu, s, base + 4);
       bb = __shfl_sync(0xffffffffu, s, base + 6);
+      // (every comparison below is false for a NaN: its column would count as converged)
+      if (!(aa <= FLT_MAX && bb <= FLT_MAX)) relmax = INFINITY;
     }
     const float ra = rsqrtf(aa), rb = rsqrtf(bb);
     const float er = gr * ra * rb, ei = gi * ra * rb;  // e^{i phi} times the cosine
@@ -2445,6 +2449,7 @@ __global__ void __launch_bounds__(32 * RING_WARPS, 1) jacobi_ring32_kernel(RingA
       relkept = fmaxf(relkept, __shfl_xor_sync(0xffffffffu, relkept, o));
     }
     if (lane == 0) {
+      if (relmax > 1.f) atomicOr(&A.flags[QT_FLAG_NONFINITE], 1);
       if (rotated) atomicAdd(&A.flags[QT_FLAG_ROTATED], rotated);
       if (relmax > 0.f) atomicMax(&A.flags[QT_FLAG_OFFMAX], __float_as_int(relmax));
       if (relbig > 0.f) atomicMax(&A.flags[QT_FLAG_OFFBIG], __float_as_int(relbig));
