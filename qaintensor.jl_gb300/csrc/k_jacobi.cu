@@ -2015,8 +2015,8 @@ jacobi_sweep32_kernel(float2* __restrict__ xb0, float2* __restrict__ xb1, int64_
 // ones on the other half, and so on; an odd number of CTAs plays a tournament.
 // K + K/2 + ... = 2 K - 1 rounds cover every pair of the 2 K blocks once, and
 // half the traffic of a tournament.  A block that leaves is written to its slot
-// of the mailbox by the warps that hold it, every number in one 8-byte half of
-// a 16-byte store with the number of the round in the other 4 bytes; the warp of
+// of the mailbox by the warps that hold it, every number in one 8-byte element of
+// a two-element store with the number of the round in its other 4 bytes; the warp of
 // the same rows in the next CTA reads the slot until every number carries that
 // round.  So the data is its own flag: no fence and no second trip to L2 (a flag
 // behind a fence cost 4.5 us a round, twice this), and no CTA-wide barrier.  A
@@ -2090,7 +2090,7 @@ struct RingArgs {
   float tol;
   double nu_rel2;
   const double* xnorm2;
-  uint4* mail;     // a slot of warps x RB x rows-per-lane x 32 entries for each of the 2 K blocks
+  ulonglong2* mail;  // a slot of warps x RB x rows-per-lane x 32 entries for each of the 2 K blocks
   int* flags;
   float keep2;
   float* dnorm;    // the columns' squared norms at the end of the sweep (nullptr: not wanted)
@@ -2124,19 +2124,18 @@ __device__ __forceinline__ float x2_sum(f32x2 a) {
   return v.x + v.y;
 }
 
-// An entry of the mailbox: each 8-byte half arrives whole, so a number is there
-// when its round is.
-__device__ __forceinline__ void mail_store(uint4* p, float re, float im, unsigned stamp) {
-  asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %2};" ::"l"(p), "r"(__float_as_uint(re)), "r"(stamp),
-               "r"(__float_as_uint(im))
+// An entry of the mailbox: two elements of 8 bytes, each a number and the round
+// that it was sent in.  A vector access is one access per element, in any order,
+// so an element arrives whole and a number is there when its round is.
+__device__ __forceinline__ void mail_store(ulonglong2* p, float re, float im, unsigned stamp) {
+  const unsigned long long hi = (unsigned long long)stamp << 32;
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(hi | __float_as_uint(re)),
+               "l"(hi | __float_as_uint(im))
                : "memory");
 }
-__device__ __forceinline__ uint4 mail_load(const uint4* p) {
-  uint4 v;
-  asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p)
-               : "memory");
+__device__ __forceinline__ ulonglong2 mail_load(const ulonglong2* p) {
+  ulonglong2 v;
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
   return v;
 }
 
@@ -2203,7 +2202,7 @@ __global__ void __launch_bounds__(32 * RING_WARPS, 1) jacobi_ring32_kernel(RingA
   };
   auto slot = [&](int blk) { return A.mail + ((size_t)blk * nw + w) * (RB * 2 * RP * 32) + lane; };
   auto publish = [&](const Col (&x)[RB], int blk, unsigned stamp) {
-    uint4* m = slot(blk);
+    ulonglong2* m = slot(blk);
 #pragma unroll
     for (int j = 0; j < RB; j++)
 #pragma unroll
@@ -2214,9 +2213,9 @@ __global__ void __launch_bounds__(32 * RING_WARPS, 1) jacobi_ring32_kernel(RingA
       }
   };
   auto fetch = [&](Col (&x)[RB], int blk, unsigned stamp) {
-    const uint4* m = slot(blk);
+    const ulonglong2* m = slot(blk);
     for (int it = 0;; it++) {
-      uint4 v[RB][2 * RP];
+      ulonglong2 v[RB][2 * RP];
 #pragma unroll
       for (int j = 0; j < RB; j++)
 #pragma unroll
@@ -2225,13 +2224,13 @@ __global__ void __launch_bounds__(32 * RING_WARPS, 1) jacobi_ring32_kernel(RingA
 #pragma unroll
       for (int j = 0; j < RB; j++)
 #pragma unroll
-        for (int k = 0; k < 2 * RP; k++) here = here && v[j][k].y == stamp && v[j][k].w == stamp;
+        for (int k = 0; k < 2 * RP; k++) here = here && (unsigned)(v[j][k].x >> 32) == stamp && (unsigned)(v[j][k].y >> 32) == stamp;
 #pragma unroll
       for (int j = 0; j < RB; j++)
 #pragma unroll
         for (int k = 0; k < RP; k++) {
-          x[j].re[k] = x2_pack(__uint_as_float(v[j][2 * k].x), __uint_as_float(v[j][2 * k + 1].x));
-          x[j].im[k] = x2_pack(__uint_as_float(v[j][2 * k].z), __uint_as_float(v[j][2 * k + 1].z));
+          x[j].re[k] = x2_pack(__uint_as_float((unsigned)v[j][2 * k].x), __uint_as_float((unsigned)v[j][2 * k + 1].x));
+          x[j].im[k] = x2_pack(__uint_as_float((unsigned)v[j][2 * k].y), __uint_as_float((unsigned)v[j][2 * k + 1].y));
         }
       if (__all_sync(0xffffffffu, here)) break;
       // given up, here or elsewhere: every wait ends, the sweep runs out and the host reports it
@@ -2851,11 +2850,11 @@ int qt_jacobi_svd_ws(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, T
     if (V) QT_TRY(pscratch.get(&V1, (size_t)ldv * nn));
     QT_CHECK_CUDA(h, cudaMemsetAsync(done, 0xff, sizeof(int) * pairs * halves, h->stream));
   }
-  uint4* ring_mail = nullptr;
+  ulonglong2* ring_mail = nullptr;
   if (ring.ctas) {
     const size_t n = (size_t)2 * ring.ctas * ring.warps * RB * ring.rows * 32;
     QT_TRY(pscratch.get(&ring_mail, n));
-    QT_CHECK_CUDA(h, cudaMemsetAsync(ring_mail, 0, sizeof(uint4) * n, h->stream));  // round 0: nothing sent
+    QT_CHECK_CUDA(h, cudaMemsetAsync(ring_mail, 0, sizeof(ulonglong2) * n, h->stream));  // round 0: nothing sent
   }
   if (keep_track) {
     QT_TRY(pscratch.get(&dnorm, (size_t)nn));
