@@ -2777,8 +2777,16 @@ int qt_jacobi_svd_ws(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, T
   // one-launch cluster round, 1 for the three-kernel round.  FP64
   // storage uses the one-launch round where a pair's rows fit a cluster's
   // shared memory.
-  const int jk = h->cfg.jacobi_kernel;
-  const ring_shape ring = fp32 && jk == 0 && pairwise && !V ? shape_ring32(mm, nn) : ring_shape();
+  // A caller that allows few sweeps gets the rounds that need the fewest, at the
+  // price of their time: the Gram-based sweep kernel instead of pairwise
+  // rotations (4 or 5 sweeps of a capped sketch where those take 5 to 7); FP64
+  // pair solves of up to 12 and 3 inner sweeps instead of one (up to 24 columns 4
+  // to 6 sweeps instead of 6 or 7), and below three sweeps the three-kernel
+  // round, whose FP64 angles finish a single pair of blocks at once.  (The
+  // default limit is 80.)
+  const bool few = max_sweeps < 12;
+  const int jk = !fp32 && max_sweeps < 3 ? 1 : h->cfg.jacobi_kernel;
+  const ring_shape ring = fp32 && jk == 0 && pairwise && !V && !few ? shape_ring32(mm, nn) : ring_shape();
   const bool sweep_kernel = fp32 && jk == 0 && !ring.ctas && sweep32_fits(h, pairs);
   const bool two_launch = fp32 && (jk == 3 || (jk == 0 && !sweep_kernel && !ring.ctas));
   int xrows_c = 0, lds = 0;
@@ -2877,9 +2885,9 @@ int qt_jacobi_svd_ws(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, T
     // test decides convergence.  FP64 storage: one throughout (1, 2, 4 and 12
     // in the first two took 10.9, 11.3, 13.6 and 14.0 ms at 128 x 128).
     // QT_JACOBI_INNER0 / QT_JACOBI_INNER override the two caps.
-    static const int inner_cap = std::getenv("QT_JACOBI_INNER") ? std::atoi(std::getenv("QT_JACOBI_INNER")) : 1;
-    static const int inner_cap0 =
-        std::getenv("QT_JACOBI_INNER0") ? std::atoi(std::getenv("QT_JACOBI_INNER0")) : (fp32 ? 2 : 1);
+    static const char *inner_env = std::getenv("QT_JACOBI_INNER"), *inner_env0 = std::getenv("QT_JACOBI_INNER0");
+    const int inner_cap = inner_env ? std::atoi(inner_env) : !fp32 && few ? 3 : 1;
+    const int inner_cap0 = inner_env0 ? std::atoi(inner_env0) : fp32 ? 2 : few ? MAX_INNER : 1;
     const int max_inner = std::max(1, std::min(sweep < 2 ? inner_cap0 : inner_cap, MAX_INNER));
     // The sweep kernel goes on to the next sweep by itself where "no pair
     // rotated" is the only rule that ends the sweeps: a launch, its status
