@@ -102,7 +102,8 @@ __device__ __forceinline__ cta_rotation<float> cta_angle(float aa, float bb, flo
   // common factor 2^-e: the larger of |gr|, |gi| into [1, 2)
   const float sc = __uint_as_float((254u << 23) - (__float_as_uint(gm) & 0x7f800000u));
   const float xr = __fmul_rn(gr, sc), xi = __fmul_rn(gi, sc), xa = __fmul_rn(aa, sc), xb = __fmul_rn(bb, sc);
-  if (fmaxf(xa, xb) > 1e30f) return cta_angle64<float>(aa, bb, gr, gi, tol, nu2);
+  // (the smaller norm is above 1e-30 then, or these are no sums of two columns)
+  if (fmaxf(xa, xb) > 1e30f || fminf(xa, xb) < 0.9e-30f) return cta_angle64<float>(aa, bb, gr, gi, tol, nu2);
   const ff p1 = ff_prod(xr, xr), p2 = ff_prod(xi, xi);
   ff p = ff_sum(p1.h, p2.h);
   p = ff_fast(p.h, __fadd_rn(p.l, __fadd_rn(p1.l, p2.l)));
@@ -134,8 +135,8 @@ __device__ __forceinline__ cta_rotation<float> cta_angle(float aa, float bb, flo
   o.c = ff_round(cs, &sure);
   o.s = ff_round(sn, &sure);
   o.s = neg ? -o.s : o.s;
-  o.er = ff_round(er, &sure);
-  o.ei = ff_round(ei, &sure);
+  o.er = xr == 0.f ? xr : ff_round(er, &sure);  // (a sum of pairs loses the sign of a zero)
+  o.ei = xi == 0.f ? xi : ff_round(ei, &sure);
   o.on = true;
   // a component of the phase so small that its error term would be denormal
   sure = sure && (xr == 0.f || fabsf(xr) > 1e-15f) && (xi == 0.f || fabsf(xi) > 1e-15f);
