@@ -135,8 +135,8 @@ __device__ __forceinline__ cta_rotation<float> cta_angle(float aa, float bb, flo
   o.c = ff_round(cs, &sure);
   o.s = ff_round(sn, &sure);
   o.s = neg ? -o.s : o.s;
-  o.er = xr == 0.f ? xr : ff_round(er, &sure);  // (a sum of pairs loses the sign of a zero)
-  o.ei = xi == 0.f ? xi : ff_round(ei, &sure);
+  o.er = copysignf(ff_round(er, &sure), xr);  // (a sum of pairs loses the sign of a zero)
+  o.ei = copysignf(ff_round(ei, &sure), xi);
   o.on = true;
   // a component of the phase so small that its error term would be denormal
   sure = sure && (xr == 0.f || fabsf(xr) > 1e-15f) && (xi == 0.f || fabsf(xi) > 1e-15f);
