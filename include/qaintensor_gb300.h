@@ -49,7 +49,10 @@ typedef enum {
 typedef enum { QT_C64 = 0, QT_C128 = 1 } qt_dtype;
 
 typedef enum {
-  QT_MODE_PLAIN = 0,     /* FP64 everywhere: FP64 GEMM + exact FP64 one-sided Jacobi SVD */
+  QT_MODE_PLAIN = 0,     /* FP64 data and sums: FP64 GEMM + exact FP64 one-sided Jacobi SVD
+                            (its rotation angles are found in FP32 and the rotations
+                            brought to unit length in FP64; every sweep measures its
+                            pairs from the FP64 columns) */
   QT_MODE_CHOSEN = 1,    /* complex64: FP32-level products (tcgen05 split-TF32x3),
                             randomized range finder sized by the rank predictor,
                             FP32-storage Jacobi split with FP64 norms and tail sums;
@@ -77,11 +80,14 @@ typedef struct {
                               honoured through a certificate or the exact FP64 split */
   uint64_t seed;           /* sketch RNG seed */
   int tc_gemm;             /* chosen mode: 1 = tcgen05 split-TF32x3 products, 0 = FP32 SIMT */
-  int jacobi_kernel;       /* Jacobi round: 0 = automatic (FP32 storage: one cooperative launch per
-                              sweep, each round rebuilding its columns from the previous round's
-                              unitaries, where one CTA per pair fits on the device, else 3; FP64:
-                              one launch with cluster-resident pair rows where they fit shared
-                              memory), 1 = three kernels (Gram partials, pair solver, rotation),
+  int jacobi_kernel;       /* Jacobi round: 0 = automatic (FP32 storage: for a sketch of up to 2048
+                              rows one cooperative launch per sweep with the columns resident in
+                              registers; else one for all sweeps of a split, or per sweep of a
+                              rank pinned at chi_max, each round rebuilding its columns from the
+                              previous round's unitaries, where one CTA per pair fits on the
+                              device, else 3; FP64: one launch with cluster-resident pair rows
+                              where they fit shared memory; with max_sweeps below 12 the rounds
+                              that need the fewest sweeps), 1 = three kernels (Gram partials, pair solver, rotation),
                               2 = the one-launch cluster round, 3 = FP32 two launches per round
                               (Gram + pair solver, then rotation) */
   double cap_sketch;       /* chosen mode: sketch width of a rank pinned at the chi_max cap, as a

@@ -21,10 +21,11 @@
 //   bonds[w+1] = k
 // The tasks left to the FP64 split are listed, and a second kernel of the layer
 // takes them, a cluster of eight CTAs each or, where many are left, one CTA
-// each (batch_split64_kernel).  Tasks of one brickwork layer touch disjoint sites, so CTAs never race.  A whole program
-// (every layer) is a fixed sequence of a counter reset and kernels that the
-// host captures once in a CUDA graph.  There are no waits on
-// other CTAs: a CTA stops when the counter passes the task count.
+// each (batch_split64_kernel).  Tasks of one brickwork layer touch disjoint
+// sites, so CTAs never race.  A whole program (every layer) is a fixed sequence
+// of a counter reset and kernels that the host captures once in a CUDA graph.
+// The layer kernel has no waits on other CTAs: a CTA stops when the counter
+// passes the task count.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -239,6 +240,9 @@ __global__ void __launch_bounds__(NT) batch_layer_kernel(BatchArgs p) {
       int kc = tail_rule(s_sig, n, p.cutoff);
       int cert = QT_CERT_NONE;
       if (p.cutoff >= eta) {
+        // (Not so where frozen columns are kept: eta is about nu, and the rule
+        // drops by accumulated weight.  Their unit vectors are not orthogonal
+        // to the larger ones, and A' A'^H theta' is no projection then.)
         cert = QT_CERT_RESOLVED;
       } else if (cap < min(m, n) && kc > cap) {
         double t2 = 0;

@@ -2773,10 +2773,10 @@ int qt_jacobi_svd_ws(qt_handle* h, TS* X, int64_t mm, int64_t nn, int64_t ldx, T
   // Round implementation (cfg.jacobi_kernel): FP32 storage by default rotates
   // register-resident columns in one launch per sweep where the caller takes
   // pairwise rotations, else (and with more columns than that holds) runs the
-  // Gram-based sweep kernel, beyond its size two launches per round (Gram + pair solver, then the rotation; also 3); 2 asks for the
-  // one-launch cluster round, 1 for the three-kernel round.  FP64
-  // storage uses the one-launch round where a pair's rows fit a cluster's
-  // shared memory.
+  // Gram-based sweep kernel, beyond its size two launches per round (Gram + pair
+  // solver, then the rotation; also 3); 2 asks for the one-launch cluster
+  // round, 1 for the three-kernel round.  FP64 storage uses the one-launch
+  // round where a pair's rows fit a cluster's shared memory.
   // A caller that allows few sweeps gets the rounds that need the fewest, at the
   // price of their time: the Gram-based sweep kernel instead of pairwise
   // rotations (4 or 5 sweeps of a capped sketch where those take 5 to 7); FP64

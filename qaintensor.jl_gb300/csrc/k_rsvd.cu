@@ -307,7 +307,8 @@ constexpr double CQ_SERIES = 2e-7;
 // in the arithmetic of C.  An FP64 pass without shift mostly meets a G that is
 // the identity to rounding (the pass before it orthonormalised a block of
 // condition up to 1e4): then X = I - E/2 + 3/8 E^2, E = G - I, which needs no
-// FP64 products (E^2 is below 1e-13, and FP32 gives it to 1e-20), and the
+// FP64 products (entries of E^2 are below 64 CQ_SERIES^2 = 2.6e-12, which FP32
+// sums give to some 1e-18), and the
 // pass after it is skipped.  FP64: 90 us for the factor -- the FP64
 // instructions of one SM, 16 cycles each -- where one thread per entry and
 // three block barriers per pivot took 117; the series takes under 10.

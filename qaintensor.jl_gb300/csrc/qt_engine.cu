@@ -678,9 +678,10 @@ int fp32_scale_exponent(double norm2) {
 //   tall/square: X = theta V (V not accumulated); A' = unit columns of X for
 //     the k largest norms;
 //   wide: X = theta^H V, V (m x m) accumulated; A' = V[:, perm].
-// Either A' is orthonormal only to the Jacobi tolerance (FP32: ~1e-5); one
-// Newton-Schulz step A' <- A' (1.5 I - 0.5 A'^H A') makes it orthonormal to
-// FP32 rounding, and B' = A'^H theta is the exact projection onto it (both
+// Either A' is orthonormal only to the Jacobi tolerance (FP32: ~1e-5); a
+// Newton-Schulz step A' <- A' (1.5 I - 0.5 A'^H A'), two of them for a sketch
+// whose kept set alone converged, makes it orthonormal to FP32 rounding, and
+// B' = A'^H theta is the exact projection onto it (both
 // tensor-core GEMMs), so A' B' carries no error beyond the truncation.
 // `extra_tail` (>= 0) is a weight outside this factorisation (a sketch's
 // residual), counted as the smallest tail value of the rank rule.
